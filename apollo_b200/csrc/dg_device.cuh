@@ -71,7 +71,7 @@ struct DgDev {
   int grid_div;    // launch shape: persistent grids use SMs / grid_div (>= 1; 0 means 1)
   int tile_shape;  // mixed stage operand chunking (0 or 1), picked by the batch autotuner
   int fp64_fused;  // float64 stages: 0 the three kernels, 1 the fused stage kernel where it applies,
-                   // 2 the fused kernel where its tiles fit one resident wave (launch-bound meshes)
+                   // 2 the fused kernel where its tiles fit one resident wave
   int nghost;      // ghost element slots of a partitioned mesh (their faces' traces come from peers)
   int nbound;      // boundary faces of the local mesh
   // bounded device waits of the mixed stage kernel: polls before a wait gives
@@ -87,6 +87,7 @@ struct DgDev {
   const double *VS, *cub_r, *cub_s;
   double* srcv;
   const double *V, *Dr, *Ds, *I, *L, *gz, *gw;
+  const double* pack64;  // the fused float64 stage's operator fragments (dg_stage64.h)
   double *vol, *trace, *flux;  // scratch: [K][NP][M], [K][NF][M], [K][NF][M]
   DevState* st;
   EqParams eqp;
@@ -173,6 +174,16 @@ template <int N> struct Sizes {
 // Host launchers (dg_fp64.cu).
 // ev (optional): 4 events recorded before/between/after the three kernels
 cudaError_t launch_rhs_fp64(int eq, const DgDev& d, const StageArgs& a, cudaStream_t s, cudaEvent_t* ev = nullptr);
+// the fused float64 stage (dg_stage64.cu) on the elements of `list` (nullptr:
+// all); x and out must not overlap; the caller clears the wave-speed word
+// before a MODE_RHS launch (a MODE_STAGE launch with reset_lambda clears it for
+// the MODE_FINAL one that follows)
+cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s);
+// traces of cut faces (3 k + f) of x into dst [n][NG][M], as k_stage64 would interpolate them
+cudaError_t launch_cut_traces(int eq, const DgDev& d, const double* x, const int* blocks, int n, double* dst,
+                              cudaStream_t s);
+int stage64_wave_tiles(int eq, int N, int sms);  // tiles (of 8 elements) of one resident wave
+int device_sms();                                // SMs of the current device
 // k_lift alone on d.vol / d.flux (used by the tangent of a stage)
 cudaError_t launch_lift_fp64(int eq, const DgDev& d, const StageArgs& a, cudaStream_t s);
 cudaError_t launch_init_speed(int eq, const DgDev& d, const double* u, cudaStream_t s);

@@ -47,13 +47,14 @@ struct apollo_dg {
   int ninst = 1;
   int grid_div = 1;    // launch shape picked by the batch autotuner
   int tile_shape = 0;  // mixed stage operand chunking picked by the batch autotuner
-  int fp64_fused = 0;  // float64 stage kernels: 0 three, 1 fused, 2 fused on one-wave meshes
+  int fp64_fused = 1;  // float64 stage kernels: 0 three, 1 fused, 2 fused on one-wave meshes
   unsigned wait_limit = 0;  // apollo_dg_debug_set_waits
   int debug_stall = 0;
   // source plugins (apollo_dg_add_source): the table, VS = VVT V^T diag(w),
   // the cubature points, and the mixed stages' source buffer
   SrcTable src{};
   double *VS_d = nullptr, *cubr_d = nullptr, *cubs_d = nullptr, *srcv_d = nullptr;
+  double* pack64_d = nullptr;  // the fused float64 stage's operator fragments
   double *V_d = nullptr, *Dr_d = nullptr, *Ds_d = nullptr, *I_d = nullptr, *L_d = nullptr, *gz_d = nullptr,
          *gw_d = nullptr, *wmass_d = nullptr, *mass_d = nullptr;
   // W_d, W2_d: stage states, alternating so that a stage's output never
@@ -99,6 +100,10 @@ struct apollo_dg {
   // them), then the cut faces that touch ghost slots; a float64 stage runs the
   // first group on side_stream while the caller's exchange is in flight
   int nface_int = 0;
+  // elements without a cut face first (nel_int of them), then the others: the
+  // fused stage's launches around the exchange
+  int* elist_d = nullptr;
+  int nel_int = 0;
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_packed = nullptr, ev_interior = nullptr;
   // Euler limiter (apollo_dg_set_limiter): applied to every stage input
@@ -164,7 +169,7 @@ void free_mesh(apollo_dg* h) {
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   dfree(h->geo_d); dfree(h->faces_d); dfree(h->conn_d); dfree(h->einst_d);
   dfree(h->V_d); dfree(h->Dr_d); dfree(h->Ds_d); dfree(h->I_d); dfree(h->L_d); dfree(h->gz_d); dfree(h->gw_d);
-  dfree(h->wmass_d); dfree(h->mass_d);
+  dfree(h->wmass_d); dfree(h->mass_d); dfree(h->pack64_d);
   dfree(h->VS_d); dfree(h->cubr_d); dfree(h->cubs_d); dfree(h->srcv_d);
   dfree(h->U_d); dfree(h->W_d); dfree(h->W2_d); dfree(h->in_d); dfree(h->out_d);
   dfree(h->TU_d); dfree(h->T0_d); dfree(h->T1_d);
@@ -181,7 +186,8 @@ void free_mesh(apollo_dg* h) {
   if (h->mixed) { mixed_destroy(h->mixed); h->mixed = nullptr; }
   h->have_state = false;
   h->ninst = 1;
-  dfree(h->halo_src_d); dfree(h->halo_dst_d);
+  dfree(h->halo_src_d); dfree(h->halo_dst_d); dfree(h->elist_d);
+  h->nel_int = 0;
   if (h->ev_packed) { cudaEventDestroy(h->ev_packed); h->ev_packed = nullptr; }
   if (h->ev_interior) { cudaEventDestroy(h->ev_interior); h->ev_interior = nullptr; }
   if (h->side_stream) { cudaStreamDestroy(h->side_stream); h->side_stream = nullptr; }
@@ -212,6 +218,7 @@ DgDev make_dev(const apollo_dg* h) {
   d.faces = h->faces_d;
   d.conn = h->conn_d;
   d.V = h->V_d; d.Dr = h->Dr_d; d.Ds = h->Ds_d; d.I = h->I_d; d.L = h->L_d; d.gz = h->gz_d; d.gw = h->gw_d;
+  d.pack64 = h->pack64_d;
   d.vol = h->vol_d; d.trace = h->trace_d; d.flux = h->flux_d;
   d.st = h->st_d;
   d.einst = h->einst_d;
@@ -754,6 +761,10 @@ apollo_status set_mesh_body(apollo_dg* h, int nverts, const double* vx, const do
   CK(upload(&h->gz_d, o.gz.data(), o.gz.size()), "op upload");
   CK(upload(&h->gw_d, o.gw.data(), o.gw.size()), "op upload");
   CK(upload(&h->wmass_d, o.mass_colsum.data(), o.mass_colsum.size()), "op upload");
+  {
+    const std::vector<double> pack = build_pack64(o);
+    CK(upload(&h->pack64_d, pack.data(), pack.size()), "op upload");
+  }
   const Mat mass = inverse(o.VVT);
   CK(upload(&h->mass_d, mass.a.data(), mass.a.size()), "op upload");
   {
@@ -807,6 +818,15 @@ apollo_status set_mesh_body(apollo_dg* h, int nverts, const double* vx, const do
     for (int j = 0; j < h->n_recv; ++j) dst[j] = slot[plan.recv_face[j] / 3] * 3 + plan.recv_face[j] % 3;
     CK(upload(&h->halo_src_d, src.data(), src.size()), "halo upload");
     CK(upload(&h->halo_dst_d, dst.data(), dst.size()), "halo upload");
+    std::vector<int> order(K);
+    for (int i = 0; i < K; ++i) order[i] = i;
+    auto whole = [&](int i) {
+      for (int f = 0; f < 3; ++f)
+        if (h->conn_h[6 * i + 2 * f] >= K) return false;
+      return true;
+    };
+    h->nel_int = (int)(std::stable_partition(order.begin(), order.end(), whole) - order.begin());
+    CK(upload(&h->elist_d, order.data(), order.size()), "halo upload");
   }
   return APOLLO_OK;
 }
@@ -934,7 +954,9 @@ apollo_status apollo_dg_rhs(apollo_dg* h, double t, double dt, const double* in,
     x = h->in_d;
     o = h->out_d;
   }
-  CK(cudaMemsetAsync(&h->st_d->err, 0, sizeof(int), h->stream), "rhs");
+  // the wave-speed word and the error word behind it
+  static_assert(offsetof(DevState, err) == offsetof(DevState, lam_bits) + sizeof(unsigned long long), "one clear");
+  CK(cudaMemsetAsync(&h->st_d->lam_bits, 0, sizeof(unsigned long long) + sizeof(int), h->stream), "rhs");
   if (h->lim_on) {
     // the limited input, in the handle's input buffer (the caller's array is unchanged)
     r = enqueue_limiter(h, x, h->in_d);
@@ -948,7 +970,6 @@ apollo_status apollo_dg_rhs(apollo_dg* h, double t, double dt, const double* in,
   a.time_from_state = 0;
   a.t_arg = t;
   a.dt_arg = dt;
-  a.reset_lambda = 1;
   r = enqueue_stage(h, a, prec);
   if (r) return r;
   if (where != APOLLO_DEVICE_PTR) CK(cudaMemcpyAsync(out, h->out_d, n, cudaMemcpyDeviceToHost, h->stream), "rhs output copy");
@@ -1815,6 +1836,21 @@ apollo_status apollo_dg_dist_start(apollo_dg* h, double t, double dt, apollo_pre
   return handle_prepare_step(h, prec);
 }
 
+namespace {
+// the side stream, waiting for what the handle's stream holds now
+cudaError_t fork_side(apollo_dg* h) {
+  cudaError_t e = cudaSuccess;
+  if (!h->side_stream) {
+    e = cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_packed, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_interior, cudaEventDisableTiming);
+  }
+  if (e == cudaSuccess) e = cudaEventRecord(h->ev_packed, h->stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side_stream, h->ev_packed, 0);
+  return e;
+}
+}  // namespace
+
 apollo_status apollo_dg_stage_begin(apollo_dg* h, int stage, apollo_precision prec) {
   apollo_status r = check_ready(h);
   if (r) return r;
@@ -1828,6 +1864,16 @@ apollo_status apollo_dg_stage_begin(apollo_dg* h, int stage, apollo_precision pr
     // trace kernel for U)
     const int blk = (int)(mixed_trace_floats(h->mixed, 1) / 3 * sizeof(float));
     CK(launch_halo_blocks(a.tr_in, h->hsend, h->halo_src_d, h->n_send, blk, false, h->stream), "halo pack");
+  } else if (h->fp64_fused == 1) {
+    // the cut faces' traces, then the stage of the elements without a cut face
+    // on the side stream while the caller's exchange is in flight
+    if (h->peers.empty()) return APOLLO_OK;
+    CK(launch_cut_traces(h->eq, d, a.x, h->halo_src_d, h->n_send, (double*)h->hsend, h->stream), "halo pack");
+    if (h->nel_int > 0) {
+      CK(fork_side(h), "stage event");
+      CK(launch_stage64(h->eq, d, a, h->elist_d, h->nel_int, h->side_stream), "interior stage launch");
+      CK(cudaEventRecord(h->ev_interior, h->side_stream), "stage event");
+    }
   } else {
     a.phase = PHASE_VOLUME;
     CK(launch_rhs_fp64(h->eq, d, a, h->stream), "volume launch");
@@ -1837,13 +1883,7 @@ apollo_status apollo_dg_stage_begin(apollo_dg* h, int stage, apollo_precision pr
       // the faces between local elements need no remote trace: they run on
       // the side stream while the caller's exchange (enqueued on the handle's
       // stream after this call) is in flight; apollo_dg_stage_end joins them
-      if (!h->side_stream) {
-        CK(cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking), "side stream");
-        CK(cudaEventCreateWithFlags(&h->ev_packed, cudaEventDisableTiming), "stage event");
-        CK(cudaEventCreateWithFlags(&h->ev_interior, cudaEventDisableTiming), "stage event");
-      }
-      CK(cudaEventRecord(h->ev_packed, h->stream), "stage event");
-      CK(cudaStreamWaitEvent(h->side_stream, h->ev_packed, 0), "stage event");
+      CK(fork_side(h), "stage event");
       DgDev di = d;
       di.nfaces = h->nface_int;
       a.phase = PHASE_FACE_ONLY;
@@ -1869,7 +1909,15 @@ apollo_status apollo_dg_stage_end(apollo_dg* h, int stage, apollo_precision prec
   } else {
     const int blk = h->ops.Ng * h->M * (int)sizeof(double);
     CK(launch_halo_blocks(h->hrecv, h->trace_d, h->halo_dst_d, h->n_recv, blk, true, h->stream), "halo unpack");
-    if (!h->peers.empty() && h->nface_int > 0) {
+    if (h->fp64_fused == 1) {
+      if (h->peers.empty()) {
+        CK(launch_stage64(h->eq, d, a, nullptr, 0, h->stream), "stage launch");
+      } else {
+        // the elements with a cut face; they share no output with the others
+        CK(launch_stage64(h->eq, d, a, h->elist_d + h->nel_int, h->K - h->nel_int, h->stream), "cut stage launch");
+        if (h->nel_int > 0) CK(cudaStreamWaitEvent(h->stream, h->ev_interior, 0), "stage event");
+      }
+    } else if (!h->peers.empty() && h->nface_int > 0) {
       // the interior faces ran on the side stream since apollo_dg_stage_begin;
       // the cut faces now, then the lift over all of them
       CK(cudaStreamWaitEvent(h->stream, h->ev_interior, 0), "stage event");

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "dg_stage64.h"
 #include "dg_tables.inc"
 
 namespace apollo {
@@ -241,6 +242,88 @@ bool build_ref_ops(int N, RefOps& o) {
     }
   if (!ok) o.rot.clear();
   return true;
+}
+
+namespace {
+
+template <int N> std::vector<double> pack64_t(const RefOps& o) {
+  using P = Pack64<N>;
+  constexpr int NP = P::NP, NC = P::NC, NG = P::NG, NF = P::NF;
+  std::vector<double> out(P::SIZE, 0.0);
+  // interpolation along a face from its nodes: the same for the three faces
+  // and symmetric under reversal; the face 0 rows with their rounding averaged
+  // over the reversal, so that the two sides of a face use the same numbers
+  auto edge = [&](int g, int m) {
+    return 0.5 * (o.Interp(g, P::face_node(0, m)) + o.Interp(NG - 1 - g, P::face_node(0, N - m)));
+  };
+  const Mat W1 = matmul(o.DrW, o.Vc), W2 = matmul(o.DsW, o.Vc);  // Dr V, Ds V
+  std::vector<double> vs((size_t)NP * NC, 0.0);                  // VVT V^T diag(w)
+  for (int n = 0; n < NP; ++n)
+    for (int c = 0; c < NC; ++c) {
+      double acc = 0.0;
+      for (int j = 0; j < NP; ++j) acc += o.VVT(n, j) * o.Vc(c, j);
+      vs[(size_t)n * NC + c] = acc * o.cub_w[c];
+    }
+  for (int lane = 0; lane < 32; ++lane) {
+    const int k = lane % 4, n = lane / 4;
+    for (int fb = 0; fb < P::FB; ++fb) {
+      const int p = std::min(8 * fb + n, NF - 1);  // a column past the last point repeats it
+      for (int fc = 0; fc < 3; ++fc)
+        for (int ks = 0; ks < P::EK && P::touches(fb, fc); ++ks) {
+          const int m = 4 * ks + k;
+          out[P::E_OFF + P::e_index(fb, fc, ks) * 32 + lane] = (p / NG == fc && m <= N) ? edge(p - fc * NG, m) : 0.0;
+        }
+    }
+    for (int b = 0; b < P::NB; ++b) {
+      const int node = P::out_node(b, n);
+      if (node < 0) continue;
+      for (int j = 0; j < 2; ++j) {
+        for (int fb = 0; fb < P::FB; ++fb) {
+          const int p = 8 * fb + 2 * k + j;
+          if (p < NF) out[P::L_OFF + ((fb * P::NB + b) * 32 + lane) * 2 + j] = o.Lift(node, p);
+        }
+        for (int pb = 0; pb < P::PB; ++pb) {
+          const int c = 8 * pb + 2 * k + j;
+          if (c >= NC) continue;
+          out[P::D_OFF + (((pb * 2 + 0) * P::NB + b) * 32 + lane) * 2 + j] = o.DrW(node, c);
+          out[P::D_OFF + (((pb * 2 + 1) * P::NB + b) * 32 + lane) * 2 + j] = o.DsW(node, c);
+          out[P::S_OFF + ((pb * P::NB + b) * 32 + lane) * 2 + j] = vs[(size_t)node * NC + c];
+        }
+      }
+      for (int ks = 0; ks < P::KS; ++ks) {
+        const int from = P::node(ks, k);
+        if (from >= NP) continue;
+        out[P::W_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 0] = W1(node, from);
+        out[P::W_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 1] = W2(node, from);
+      }
+    }
+    for (int pb = 0; pb < P::PB; ++pb) {
+      const int c = std::min(8 * pb + n, NC - 1);  // as for the face points
+      for (int ks = 0; ks < P::KS; ++ks) {
+        const int from = P::node(ks, k);
+        if (from < NP) out[P::V_OFF + ((pb * ((P::KS + 1) / 2) + ks / 2) * 32 + lane) * 2 + ks % 2] = o.Vc(c, from);
+      }
+    }
+    // T: the points of one face alone, in blocks of eight
+    for (int tb = 0; tb < P::TB; ++tb)
+      for (int ks = 0; ks < P::EK; ++ks) {
+        const int g = std::min(8 * tb + n, NG - 1), m = 4 * ks + k;
+        out[P::T_OFF + (tb * P::EK + ks) * 32 + lane] = m <= N ? edge(g, m) : 0.0;
+      }
+  }
+  return out;
+}
+
+}  // namespace
+
+std::vector<double> build_pack64(const RefOps& o) {
+  switch (o.N) {
+    case 2: return pack64_t<2>(o);
+    case 3: return pack64_t<3>(o);
+    case 4: return pack64_t<4>(o);
+    case 5: return pack64_t<5>(o);
+  }
+  return {};
 }
 
 }  // namespace apollo

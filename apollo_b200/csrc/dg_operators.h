@@ -46,4 +46,7 @@ struct RefOps {
 
 bool build_ref_ops(int N, RefOps& out);
 
+// The fused float64 stage's operator fragments (layout: dg_stage64.h).
+std::vector<double> build_pack64(const RefOps& o);
+
 }  // namespace apollo

@@ -1,0 +1,73 @@
+// Layout of the fused float64 stage's operator fragments (host and device):
+// the B operands of its mma.m8n8k4 contractions in the order the lanes read
+// them, built once per mesh by build_pack64 (dg_operators.cpp) and copied to
+// shared memory by every block.
+//
+// Lane l holds B[k = l % 4][n = l / 4].  Nodes: accumulator block b covers the
+// nodes 8 b .. 8 b + 7; where more than four of them exist, column c is node
+// 8 b + c and the block is two k-steps as an A operand (step 2 b + j: nodes
+// 8 b + 2 k + j); a last block of at most four nodes puts node 8 b + c / 2 in
+// the even columns and is one k-step (node 8 b + k).  Points (cubature and
+// face) always come in blocks of eight with k-step j on the points
+// 8 b + 2 k + j.
+//   E  [entries][32]        interpolation along a face, one entry per (point block, face, k-step)
+//   L  [FB][NB][32][2 (j)]  surface lift
+//   V  [PB][ceil(KS/2)][32][2 (k-step)]   nodes -> cubature points
+//   D  [PB][2 (Dr, Ds)][NB][32][2 (j)]    weak derivatives
+//   W  [KS][NB][32][2 (Dr V, Ds V)]       their products (linear equations)
+//   S  [PB][NB][32][2 (j)]                sources
+//   T  [TB][EK][32]                       interpolation along one face alone (cut faces)
+#pragma once
+
+#include "dg_device.cuh"
+
+namespace apollo {
+
+template <int N> struct Pack64 {
+  static constexpr int NP = Sizes<N>::NP, NC = Sizes<N>::NC, NG = Sizes<N>::NG, NF = Sizes<N>::NF;
+  static constexpr int KS = (NP + 3) / 4, NB = (NP + 7) / 8, PB = (NC + 7) / 8, FB = (NF + 7) / 8, EK = (N + 4) / 4,
+                       TB = (NG + 7) / 8;
+  // whether block b holds its nodes in pairs (2 c, 2 c + 1 in one lane)
+  APOLLO_HD static constexpr bool paired(int b) { return NP - 8 * b > 4; }
+  // node of k-step `k`, k index c (NP or above: none)
+  APOLLO_HD static constexpr int node(int k, int c) {
+    return paired(k / 2) ? 8 * (k / 2) + 2 * c + k % 2 : 8 * (k / 2) + c;
+  }
+  // node of column n of accumulator block b (-1: none)
+  APOLLO_HD static constexpr int out_node(int b, int n) {
+    const int v = paired(b) ? 8 * b + n : n % 2 == 0 ? 8 * b + n / 2 : NP;
+    return v < NP ? v : -1;
+  }
+  // node m (0..N) of face f in face order: the edges of the triangular node
+  // numbering (row by row), from the face's first vertex to its second
+  APOLLO_HD static constexpr int face_node(int f, int m) {
+    return f == 0 ? m : f == 1 ? row(m) + N - m : row(N - m);
+  }
+  APOLLO_HD static constexpr int row(int j) { return j * (N + 1) - j * (j - 1) / 2; }  // first node of row j
+  // whether point block fb has points of face fc (points past the last repeat it)
+  APOLLO_HD static constexpr bool touches(int fb, int fc) {
+    const int lo = 8 * fb, hi = 8 * fb + 7 < NF ? 8 * fb + 7 : NF - 1;
+    return lo / NG <= fc && fc <= hi / NG;
+  }
+  APOLLO_HD static constexpr int e_index(int fb, int fc, int k) {
+    int i = 0;
+    for (int b = 0; b < FB; ++b)
+      for (int f = 0; f < 3; ++f)
+        if (touches(b, f)) {
+          if (b == fb && f == fc) return i + k;
+          i += EK;
+        }
+    return i;  // (FB, 0, 0): the number of entries
+  }
+  static constexpr int E_SIZE = e_index(FB, 0, 0) * 32;
+  static constexpr int L_SIZE = FB * NB * 64;
+  static constexpr int V_SIZE = PB * ((KS + 1) / 2) * 64;
+  static constexpr int D_SIZE = PB * 2 * NB * 64;
+  static constexpr int W_SIZE = KS * NB * 64;
+  static constexpr int S_SIZE = PB * NB * 64;
+  static constexpr int T_SIZE = TB * EK * 32;
+  static constexpr int E_OFF = 0, L_OFF = E_SIZE, V_OFF = L_OFF + L_SIZE, D_OFF = V_OFF + V_SIZE,
+                       W_OFF = D_OFF + D_SIZE, S_OFF = W_OFF + W_SIZE, T_OFF = S_OFF + S_SIZE, SIZE = T_OFF + T_SIZE;
+};
+
+}  // namespace apollo
