@@ -152,16 +152,7 @@ struct StageArgs {
   const float* tr_in;
   float* tr_out;
   float* tr_scratch;
-  // float64 launches of a partitioned mesh split around the trace exchange:
-  // PHASE_ALL, PHASE_VOLUME (volume term and traces) or PHASE_FACE (face
-  // fluxes and LIFT)
-  int phase;
 };
-
-// PHASE_FACE_ONLY and PHASE_LIFT split PHASE_FACE into the face kernel and
-// the lift (a partitioned stage runs its interior faces while the halo is in
-// flight, then the cut faces and the lift).
-enum { PHASE_ALL = 0, PHASE_VOLUME = 1, PHASE_FACE = 2, PHASE_FACE_ONLY = 3, PHASE_LIFT = 4 };
 
 template <int N> struct Sizes {
   static constexpr int NP = (N + 1) * (N + 2) / 2;
@@ -179,9 +170,9 @@ cudaError_t launch_rhs_fp64(int eq, const DgDev& d, const StageArgs& a, cudaStre
 // before a MODE_RHS launch (a MODE_STAGE launch with reset_lambda clears it for
 // the MODE_FINAL one that follows)
 cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s);
-// traces of cut faces (3 k + f) of x into dst [n][NG][M], as k_stage64 would interpolate them
-cudaError_t launch_cut_traces(int eq, const DgDev& d, const double* x, const int* blocks, int n, double* dst,
-                              cudaStream_t s);
+// the nodes on the cut faces (3 k + f) of x into blocks dst [n][NG M]
+cudaError_t launch_cut_nodes(int eq, const DgDev& d, const double* x, const int* blocks, int n, double* dst,
+                             cudaStream_t s);
 int stage64_wave_tiles(int eq, int N, int sms);  // tiles (of 8 elements) of one resident wave
 int device_sms();                                // SMs of the current device
 // k_lift alone on d.vol / d.flux (used by the tangent of a stage)

@@ -7,43 +7,185 @@
 
 namespace apollo {
 
+// Reciprocal and square root of numbers well inside the normal range, without
+// the range checks and branches of the general operations: the hardware's
+// approximation (PTX rcp.approx.ftz.f64, rsqrt.approx.ftz.f64; relative error
+// e of some 2^-20) corrected once by the third-order iteration that the series
+// of 1/(1-e) and (1-e)^(-1/2) give (Householder, The Numerical Treatment of a
+// Single Nonlinear Equation, 1970), which leaves e^3.  Error measured against
+// the general operations: at most one unit in the last place.
+__device__ __forceinline__ double recip_normal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double sqrt_normal(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double g = x * y, e = fma(-g, y, 1.0);
+  return fma(g, e * fma(e, 0.375, 0.5), g);
+}
+
 // Euler fluxes in float64 with one reciprocal of the density per state and
 // the flux formed along a direction directly (a n.F + b n.G in one pass): the
 // same quantities as WxEulerEqn's flux and Lax-Friedrichs flux
 // (wxeulereqn.cc:809-871, :1097-1117) to round-off, for states that need none
-// of the reference's clamps; a state that does (density below its floor or
-// not positive, pressure not positive) takes the equation's own code, which
-// applies them and raises its error flags.
+// of the reference's clamps and whose density and pressure lie between 2^-500
+// and 2^500 (checked on the high words, so that the float64 pipe does not
+// compare); any other state takes the equation's own code, which applies the
+// clamps and raises its error flags.
 template <int MF> struct EulerFast64 {
   static constexpr int IE = MF - 1;
+  static constexpr int LO = 0x20b00000, HI = 0x5f300000;  // high words of 2^-500 and 2^500
   struct Side {
-    double rho, ir, vx, vy, vz, p;
+    double rho, ir, vx, vy, vz, v2, p;
     bool clean;
   };
+  __device__ __forceinline__ static bool within(double v, int lo) {
+    return (unsigned)(__double2hiint(v) - lo) < (unsigned)(HI - lo);
+  }
   __device__ __forceinline__ static Side side(const EqParams& P, const double* q) {
-    const double g1 = P.p[0] - 1.0, minD = P.p[2];
+    const double g1 = P.p[0] - 1.0;
+    // a density whose high word is above the floor's is above the floor
+    const int lo = min(max(__double2hiint(P.p[2]) + 1, LO), HI);
     Side s;
     s.rho = q[0];
-    s.ir = 1.0 / s.rho;
+    s.ir = recip_normal(s.rho);
     s.vx = q[1] * s.ir;
     s.vy = q[2] * s.ir;
     s.vz = MF == 5 ? q[3] * s.ir : 0.0;
-    s.p = g1 * (q[IE] - 0.5 * s.rho * (s.vx * s.vx + s.vy * s.vy + s.vz * s.vz));
-    s.clean = s.rho > 0.0 && s.rho >= minD && s.p > 0.0;
+    // 1e-300 keeps the speed's square root off zero and changes no other sum
+    s.v2 = fma(s.vx, s.vx, fma(s.vy, s.vy, MF == 5 ? fma(s.vz, s.vz, 1e-300) : 1e-300));
+    s.p = g1 * fma(-0.5 * s.rho, s.v2, q[IE]);
+    s.clean = within(s.rho, lo) && within(s.p, LO);
     return s;
   }
   // the flux along (ax, ay): ax F + ay G
   __device__ __forceinline__ static void along(const Side& s, const double* q, double ax, double ay, double* R) {
     const double ua = s.vx * ax + s.vy * ay;
     R[0] = s.rho * ua;
-    R[1] = s.rho * s.vx * ua + s.p * ax;
-    R[2] = s.rho * s.vy * ua + s.p * ay;
-    if (MF == 5) R[3] = s.rho * s.vz * ua;
+    R[1] = fma(q[1], ua, s.p * ax);
+    R[2] = fma(q[2], ua, s.p * ay);
+    if (MF == 5) R[3] = q[3] * ua;
     R[IE] = (q[IE] + s.p) * ua;
+  }
+  // twice the Lax-Friedrichs flux of two clean states times w (nxw, nyw: the
+  // normal times w); returns its speed
+  __device__ __forceinline__ static double lf2(const EqParams& P, const Side& a, const Side& b, const double* qM,
+                                               const double* qP, double nxw, double nyw, double w, double* nf) {
+    double FM[MF], FP[MF];
+    along(a, qM, nxw, nyw, FM);
+    along(b, qP, nxw, nyw, FP);
+    const double cM = speed(P, a), cP = speed(P, b);
+    const double lam = cM > cP ? cM : cP, wl = w * lam;
+#pragma unroll
+    for (int c = 0; c < MF; ++c) nf[c] = fma(wl, qM[c] - qP[c], FM[c] + FP[c]);
+    return lam;
+  }
+  // twice Apollo's HLL flux of two clean states times w (wxeulereqn.cc:1121-1202:
+  // in the face's normal-tangent frame, |S_R| truncated, no z-momentum flux);
+  // false where the averaged sound speed leaves the checked range
+  __device__ __forceinline__ static bool hll2(const EqParams& P, const Side& a, const Side& b, const double* qM,
+                                              const double* qP, double nx, double ny, double w, double* nf,
+                                              double* lam) {
+    const double gamma = P.p[0];
+    const double ua = nx * a.vx + ny * a.vy, ub = nx * b.vx + ny * b.vy;
+    const double ta = nx * a.vy - ny * a.vx, tb = nx * b.vy - ny * b.vx;
+    const double ca = sqrt_normal(gamma * a.p * a.ir), cb = sqrt_normal(gamma * b.p * b.ir);
+    const double ra = sqrt_normal(a.rho), rb = sqrt_normal(b.rho), ri = recip_normal(ra + rb);
+    const double ea = qM[IE] + a.p, eb = qP[IE] + b.p;
+    const double u = (ra * ua + rb * ub) * ri, t = (ra * ta + rb * tb) * ri;
+    const double z = MF == 5 ? (ra * a.vz + rb * b.vz) * ri : 0.0;
+    const double H = (ra * (ea * a.ir) + rb * (eb * b.ir)) * ri;
+    const double c2 = (gamma - 1.0) * (H - 0.5 * (u * u + t * t + z * z));
+    if (!within(c2, LO)) return false;
+    const double c = sqrt_normal(c2);
+    const double SL = fmin(ua - ca, u - c), SR = fmax(ub + cb, u + c);
+    const double D = (2.0 * w) * recip_normal(SR - SL);
+    const double t1 = (fmin(SR, 0.0) - fmin(SL, 0.0)) * D, t2 = 2.0 * w - t1;
+    const double t3 = 0.5 * (SR * fabs(SL) - SL * abs_int(SR)) * D;
+    const double na = nx * qM[1] + ny * qM[2], nb = nx * qP[1] + ny * qP[2];
+    const double sa = nx * qM[2] - ny * qM[1], sb = nx * qP[2] - ny * qP[1];
+    nf[0] = t1 * nb + t2 * na - t3 * (qP[0] - qM[0]);
+    const double f1 = t1 * fma(nb, ub, b.p) + t2 * fma(na, ua, a.p) - t3 * (nb - na);
+    const double f2 = t1 * (sb * ub) + t2 * (sa * ua) - t3 * (sb - sa);
+    nf[1] = nx * f1 - ny * f2;
+    nf[2] = ny * f1 + nx * f2;
+    if (MF == 5) nf[3] = 0.0;
+    nf[IE] = t1 * (eb * ub) + t2 * (ea * ua) - t3 * (qP[IE] - qM[IE]);
+    const double la = sqrt_normal(a.v2) + ca, lb = sqrt_normal(b.v2) + cb;
+    *lam = la > lb ? la : lb;
+    return true;
+  }
+  // flow speed + sound speed
+  __device__ __forceinline__ static double speed(const EqParams& P, const Side& s) {
+    return sqrt_normal(s.v2) + sqrt_normal(P.p[0] * s.p * s.ir);
   }
 };
 
 template <int EQ> constexpr bool kEulerEq = EQ == EQ_EULER || EQ == EQ_EULER2D;
+
+template <int EQ> constexpr bool kLinearEq = EQ == EQ_ADVECTION || EQ == EQ_MAXWELL || EQ == EQ_MAXWELL_TM;
+
+// The linear equations' flux along (ax, ay), ax F + ay G, written out, and
+// their numerical flux as the flux of the sum of the two traces plus the
+// dissipation of their difference (wxadvectioneqn.cc:176-208,
+// wxphmaxwelleqn.cc:450-522; the upwind extensions as in dg_physics.cuh): the
+// plugins' values to round-off.
+template <int EQ> struct LinearFast64 {
+  static constexpr int M = Eq<EQ>::M;
+  __device__ __forceinline__ static void along(const EqParams& P, const double* q, double ax, double ay, double* R) {
+    if constexpr (EQ == EQ_ADVECTION) {
+      R[0] = (ax * P.p[0] + ay * P.p[1]) * q[0];
+    } else {
+      const double c2 = P.p[0] * P.p[0];
+      if constexpr (EQ == EQ_MAXWELL_TM) {
+        R[0] = c2 * (ay * q[1] - ax * q[2]);
+        R[1] = ay * q[0];
+        R[2] = -ax * q[0];
+      } else {
+        const double gm = P.p[1], chi = P.p[2], cp = chi * q[6], gp = gm * q[7];
+        R[0] = c2 * (ax * cp - ay * q[5]);
+        R[1] = c2 * (ax * q[5] + ay * cp);
+        R[2] = c2 * (ay * q[3] - ax * q[4]);
+        R[3] = ax * gp + ay * q[2];
+        R[4] = ay * gp - ax * q[2];
+        R[5] = ax * q[1] - ay * q[0];
+        R[6] = chi * (ax * q[0] + ay * q[1]);
+        R[7] = gm * c2 * (ax * q[3] + ay * q[4]);
+      }
+    }
+  }
+  // twice the numerical flux times w; returns its speed
+  __device__ __forceinline__ static double face2(const EqParams& P, double nx, double ny, double w, const double* qM,
+                                                 const double* qP, double* nf) {
+    double s[M], dq[M];
+#pragma unroll
+    for (int f = 0; f < M; ++f) {
+      s[f] = qM[f] + qP[f];
+      dq[f] = qM[f] - qP[f];
+    }
+    along(P, s, w * nx, w * ny, nf);
+    double lam;
+    if constexpr (EQ == EQ_ADVECTION) {
+      lam = dmax2(fabs(P.p[0]), fabs(P.p[1]));
+      const double diss = (int)P.p[3] == NF_UPWIND ? fabs(nx * P.p[0] + ny * P.p[1]) : lam;
+      nf[0] = fma(w * diss, dq[0], nf[0]);
+    } else {
+      lam = EQ == EQ_MAXWELL_TM ? P.p[0] : dmax3(P.p[2] * P.p[0], P.p[1] * P.p[0], P.p[0]);
+      const double wl = w * lam;
+      if (EQ == EQ_MAXWELL_TM && (int)P.p[3] == NF_UPWIND) {
+        const double bn = nx * dq[1] + ny * dq[2];
+        dq[1] -= bn * nx;
+        dq[2] -= bn * ny;
+      }
+#pragma unroll
+      for (int f = 0; f < M; ++f) nf[f] = fma(wl, dq[f], nf[f]);
+    }
+    return lam;
+  }
+};
 
 // R = rx F + ry G, S = sx F + sy G of one state
 template <int EQ>
@@ -68,33 +210,74 @@ __device__ __forceinline__ void volume_flux(const EqParams& P, const double* q, 
   }
 }
 
-// The numerical flux of one face point (qM, qP may be modified as the
-// reference modifies them); the Euler Lax-Friedrichs flux of two clean states
-// through EulerFast64
+// The same for two points: one branch for both, so that the two chains of
+// dependent operations run side by side
 template <int EQ>
-__device__ __forceinline__ double face_flux(const EqParams& P, double nx, double ny, double* qM, double* qP,
-                                            double* nf, int* err) {
+__device__ __forceinline__ void volume_flux_pair(const EqParams& P, const double (*q)[Eq<EQ>::M], double rx, double ry,
+                                                 double sx, double sy, double (*R)[Eq<EQ>::M], double (*S)[Eq<EQ>::M],
+                                                 int* err) {
+  if constexpr (kEulerEq<EQ>) {
+    using X = EulerFast64<Eq<EQ>::M>;
+    const typename X::Side a = X::side(P, q[0]), b = X::side(P, q[1]);
+    if (a.clean && b.clean) {
+      X::along(a, q[0], rx, ry, R[0]);
+      X::along(b, q[1], rx, ry, R[1]);
+      X::along(a, q[0], sx, sy, S[0]);
+      X::along(b, q[1], sx, sy, S[1]);
+      return;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) volume_flux<EQ>(P, q[j], rx, ry, sx, sy, R[j], S[j], err);
+}
+
+// Twice the numerical flux of one face point (qM, qP may be modified as the
+// reference modifies them) times w; the Euler Lax-Friedrichs flux of two clean
+// states through EulerFast64
+template <int EQ>
+__device__ __forceinline__ double face_flux2(const EqParams& P, double nx, double ny, double w, double* qM, double* qP,
+                                             double* nf, int* err) {
   constexpr int M = Eq<EQ>::M;
   if constexpr (kEulerEq<EQ>) {
     const int kind = (int)P.p[3];
     if (kind != NF_HLL && kind != NF_ROE && kind != NF_WAVE) {
       using X = EulerFast64<M>;
       const typename X::Side a = X::side(P, qM), b = X::side(P, qP);
-      if (a.clean && b.clean) {
-        double FM[M], FP[M];
-        X::along(a, qM, nx, ny, FM);
-        X::along(b, qP, nx, ny, FP);
-        const double gamma = P.p[0];
-        const double cM = sqrt(a.vx * a.vx + a.vy * a.vy + a.vz * a.vz) + sqrt(gamma * a.p * a.ir);
-        const double cP = sqrt(b.vx * b.vx + b.vy * b.vy + b.vz * b.vz) + sqrt(gamma * b.p * b.ir);
-        const double lam = cM > cP ? cM : cP;
+      if (a.clean && b.clean) return X::lf2(P, a, b, qM, qP, w * nx, w * ny, w, nf);
+    }
+  }
+  const double lam = Eq<EQ>::numflux(P, nx, ny, qM, qP, nf, err);
 #pragma unroll
-        for (int c = 0; c < M; ++c) nf[c] = 0.5 * (FM[c] + FP[c] + lam * (qM[c] - qP[c]));
-        return lam;
+  for (int c = 0; c < M; ++c) nf[c] *= 2.0 * w;
+  return lam;
+}
+
+// The same for two points of one face (HLL of clean states through EulerFast64 too)
+template <int EQ>
+__device__ __forceinline__ void face_flux2_pair(const EqParams& P, double nx, double ny, double w,
+                                                double (*qM)[Eq<EQ>::M], double (*qP)[Eq<EQ>::M],
+                                                double (*nf)[Eq<EQ>::M], double* lam, int* err) {
+  if constexpr (kEulerEq<EQ>) {
+    const int kind = (int)P.p[3];
+    if (kind != NF_ROE && kind != NF_WAVE) {
+      using X = EulerFast64<Eq<EQ>::M>;
+      const typename X::Side a0 = X::side(P, qM[0]), b0 = X::side(P, qP[0]);
+      const typename X::Side a1 = X::side(P, qM[1]), b1 = X::side(P, qP[1]);
+      if (a0.clean && b0.clean && a1.clean && b1.clean) {
+        if (kind != NF_HLL) {
+          const double nxw = w * nx, nyw = w * ny;
+          lam[0] = X::lf2(P, a0, b0, qM[0], qP[0], nxw, nyw, w, nf[0]);
+          lam[1] = X::lf2(P, a1, b1, qM[1], qP[1], nxw, nyw, w, nf[1]);
+          return;
+        }
+        if (X::hll2(P, a0, b0, qM[0], qP[0], nx, ny, w, nf[0], &lam[0]) &
+            X::hll2(P, a1, b1, qM[1], qP[1], nx, ny, w, nf[1], &lam[1]))
+          return;
       }
     }
   }
-  return Eq<EQ>::numflux(P, nx, ny, qM, qP, nf, err);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) lam[j] = face_flux2<EQ>(P, nx, ny, w, qM[j], qP[j], nf[j], err);
 }
 
 // The source plugins at one point (Apollo adds each into its output field,

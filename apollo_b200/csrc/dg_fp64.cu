@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kThreads) k_face(DgDev d, StageArgs a) {
       const double y = 0.5 * (-g.vy[0] * (r + s) + g.vy[1] * (1. + r) + g.vy[2] * (1. + s));
       apply_bc<EQ, double>(d.bcs, -fr.k2, t, x, y, nx, ny, qM, qP);
     }
-    double lam = face_flux<EQ>(d.eqp, nx, ny, qM, qP, nf, &err);
+    double lam = face_flux2<EQ>(d.eqp, nx, ny, 0.5, qM, qP, nf, &err);
     lam_acc.add(d.st, inst, fabs(lam));
     const double w = d.gw[gq] * sJ;
     store_point<M>(d.flux + ((size_t)fr.k1 * NF + fr.f1 * NG + gq) * M, nf, w);
@@ -496,27 +496,20 @@ cudaError_t launch_rhs_t(const DgDev& d, const StageArgs& a, cudaStream_t s, cud
   int per_sm = vol_res < 1 ? 1 : (vol_res > 8 ? 8 : vol_res);
   int gv = sms * per_sm;
   if (gv > vt) gv = vt;
-  if (a.phase == PHASE_ALL || a.phase == PHASE_VOLUME) {
-    if (ev) cudaEventRecord(ev[0], s);
-    k_volume<EQ, N><<<gv, kThreads, VT::BYTES, s>>>(d, a);
-    // sources enter the volume term (wxcubature2d.cc:297-325: VT (w J S))
-    if (d.src.n > 0) {
-      cudaError_t e = source_dispatch<EQ>(d, a, d.vol, 1, s);
-      if (e != cudaSuccess) return e;
-    }
-    if (ev) cudaEventRecord(ev[1], s);
+  if (ev) cudaEventRecord(ev[0], s);
+  k_volume<EQ, N><<<gv, kThreads, VT::BYTES, s>>>(d, a);
+  // sources enter the volume term (wxcubature2d.cc:297-325: VT (w J S))
+  if (d.src.n > 0) {
+    cudaError_t e = source_dispatch<EQ>(d, a, d.vol, 1, s);
+    if (e != cudaSuccess) return e;
   }
-  if (a.phase == PHASE_VOLUME) return cudaGetLastError();
-  if (a.phase != PHASE_LIFT) {
-    // the faces d.faces[0, d.nfaces): all of them, or a range of them
-    const int fthreads = d.nfaces * Sizes<N>::NG;
-    int gf = (fthreads + kThreads - 1) / kThreads;
-    if (gf > sms * 8) gf = sms * 8;
-    if (gf < 1) gf = 1;
-    if (fthreads > 0) k_face<EQ, N><<<gf, kThreads, 0, s>>>(d, a);
-    if (ev) cudaEventRecord(ev[2], s);
-  }
-  if (a.phase == PHASE_FACE_ONLY) return cudaGetLastError();
+  if (ev) cudaEventRecord(ev[1], s);
+  const int fthreads = d.nfaces * Sizes<N>::NG;
+  int gf = (fthreads + kThreads - 1) / kThreads;
+  if (gf > sms * 8) gf = sms * 8;
+  if (gf < 1) gf = 1;
+  if (fthreads > 0) k_face<EQ, N><<<gf, kThreads, 0, s>>>(d, a);
+  if (ev) cudaEventRecord(ev[2], s);
   const int lt = (d.K + LT::E - 1) / LT::E;
   int lper = lift_res < 1 ? 1 : (lift_res > 8 ? 8 : lift_res);
   int gl = sms * lper;
@@ -590,12 +583,11 @@ static int eq_fields(int eq) {
 
 int fp64_supported(int eq, int N) { return eq >= 0 && eq <= 4 && N >= 2 && N <= 5; }
 
-// The fused stage where it applies: the whole mesh on this handle (no ghost
-// elements), an output that does not overlap the input (it reads the
+// The fused stage where it applies: an output that does not overlap the input (it reads the
 // neighbours' states while other warps write theirs), and arrays that start on
 // a 16-byte boundary (its copies and vector accesses).
 static bool fused_applies(int eq, const DgDev& d, const StageArgs& a) {
-  if (d.fp64_fused == 0 || d.nghost != 0 || a.phase != PHASE_ALL) return false;
+  if (d.fp64_fused == 0) return false;
   if (d.fp64_fused == 2 && (d.K + 7) / 8 > stage64_wave_tiles(eq, d.N, num_sms())) return false;
   if (((uintptr_t)a.x | (uintptr_t)a.out | (uintptr_t)a.u0) % 16) return false;
   const size_t nbytes = (size_t)d.K * ((d.N + 1) * (d.N + 2) / 2) * eq_fields(eq) * sizeof(double);

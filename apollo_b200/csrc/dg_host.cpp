@@ -96,12 +96,9 @@ struct apollo_dg {
   int *halo_src_d = nullptr, *halo_dst_d = nullptr;
   void *hsend = nullptr, *hrecv = nullptr, *hlam = nullptr;
   size_t hsend_bytes = 0, hrecv_bytes = 0;
-  // the face list holds the faces between local elements first (nface_int of
-  // them), then the cut faces that touch ghost slots; a float64 stage runs the
-  // first group on side_stream while the caller's exchange is in flight
-  int nface_int = 0;
-  // elements without a cut face first (nel_int of them), then the others: the
-  // fused stage's launches around the exchange
+  // elements without a cut face first (nel_int of them), then the others: a
+  // float64 stage runs the first group on side_stream while the caller's
+  // exchange is in flight
   int* elist_d = nullptr;
   int nel_int = 0;
   cudaStream_t side_stream = nullptr;
@@ -191,7 +188,6 @@ void free_mesh(apollo_dg* h) {
   if (h->ev_packed) { cudaEventDestroy(h->ev_packed); h->ev_packed = nullptr; }
   if (h->ev_interior) { cudaEventDestroy(h->ev_interior); h->ev_interior = nullptr; }
   if (h->side_stream) { cudaStreamDestroy(h->side_stream); h->side_stream = nullptr; }
-  h->nface_int = 0;
   h->partitioned = false;
   h->KG = 0;
   h->peers.clear(); h->send_count.clear(); h->recv_count.clear();
@@ -738,14 +734,6 @@ apollo_status set_mesh_body(apollo_dg* h, int nverts, const double* vx, const do
   h->nbound = 0;
   for (const FaceRec& fr : h->faces_h)
     if (fr.k2 < 0) ++h->nbound;
-  // interior and boundary faces of the local elements first, the cut faces
-  // (one side a ghost slot) last; each face is computed on its own, so the
-  // order changes no result
-  std::stable_partition(h->faces_h.begin(), h->faces_h.end(),
-                        [K](const FaceRec& fr) { return fr.k1 < K && fr.k2 < K; });
-  h->nface_int = 0;
-  for (const FaceRec& fr : h->faces_h)
-    if (fr.k1 < K && fr.k2 < K) ++h->nface_int;
   // device buffers: state-sized ones for the local elements, geometry and
   // trace/flux scratch with the ghost slots
   const size_t nU = (size_t)K * Np * M, nT = (size_t)(K + G) * o.Nf * M;
@@ -1864,30 +1852,14 @@ apollo_status apollo_dg_stage_begin(apollo_dg* h, int stage, apollo_precision pr
     // trace kernel for U)
     const int blk = (int)(mixed_trace_floats(h->mixed, 1) / 3 * sizeof(float));
     CK(launch_halo_blocks(a.tr_in, h->hsend, h->halo_src_d, h->n_send, blk, false, h->stream), "halo pack");
-  } else if (h->fp64_fused == 1) {
-    // the cut faces' traces, then the stage of the elements without a cut face
-    // on the side stream while the caller's exchange is in flight
-    if (h->peers.empty()) return APOLLO_OK;
-    CK(launch_cut_traces(h->eq, d, a.x, h->halo_src_d, h->n_send, (double*)h->hsend, h->stream), "halo pack");
+  } else if (!h->peers.empty()) {
+    // the cut faces' nodes, then the stage of the elements without a cut face
+    // on the side stream while the caller's exchange is in flight (enqueued on
+    // the handle's stream after this call); apollo_dg_stage_end joins it
+    CK(launch_cut_nodes(h->eq, d, a.x, h->halo_src_d, h->n_send, (double*)h->hsend, h->stream), "halo pack");
     if (h->nel_int > 0) {
       CK(fork_side(h), "stage event");
       CK(launch_stage64(h->eq, d, a, h->elist_d, h->nel_int, h->side_stream), "interior stage launch");
-      CK(cudaEventRecord(h->ev_interior, h->side_stream), "stage event");
-    }
-  } else {
-    a.phase = PHASE_VOLUME;
-    CK(launch_rhs_fp64(h->eq, d, a, h->stream), "volume launch");
-    const int blk = h->ops.Ng * h->M * (int)sizeof(double);
-    CK(launch_halo_blocks(h->trace_d, h->hsend, h->halo_src_d, h->n_send, blk, false, h->stream), "halo pack");
-    if (!h->peers.empty() && h->nface_int > 0) {
-      // the faces between local elements need no remote trace: they run on
-      // the side stream while the caller's exchange (enqueued on the handle's
-      // stream after this call) is in flight; apollo_dg_stage_end joins them
-      CK(fork_side(h), "stage event");
-      DgDev di = d;
-      di.nfaces = h->nface_int;
-      a.phase = PHASE_FACE_ONLY;
-      CK(launch_rhs_fp64(h->eq, di, a, h->side_stream), "interior face launch");
       CK(cudaEventRecord(h->ev_interior, h->side_stream), "stage event");
     }
   }
@@ -1909,28 +1881,12 @@ apollo_status apollo_dg_stage_end(apollo_dg* h, int stage, apollo_precision prec
   } else {
     const int blk = h->ops.Ng * h->M * (int)sizeof(double);
     CK(launch_halo_blocks(h->hrecv, h->trace_d, h->halo_dst_d, h->n_recv, blk, true, h->stream), "halo unpack");
-    if (h->fp64_fused == 1) {
-      if (h->peers.empty()) {
-        CK(launch_stage64(h->eq, d, a, nullptr, 0, h->stream), "stage launch");
-      } else {
-        // the elements with a cut face; they share no output with the others
-        CK(launch_stage64(h->eq, d, a, h->elist_d + h->nel_int, h->K - h->nel_int, h->stream), "cut stage launch");
-        if (h->nel_int > 0) CK(cudaStreamWaitEvent(h->stream, h->ev_interior, 0), "stage event");
-      }
-    } else if (!h->peers.empty() && h->nface_int > 0) {
-      // the interior faces ran on the side stream since apollo_dg_stage_begin;
-      // the cut faces now, then the lift over all of them
-      CK(cudaStreamWaitEvent(h->stream, h->ev_interior, 0), "stage event");
-      DgDev dc = d;
-      dc.faces = d.faces + h->nface_int;
-      dc.nfaces = d.nfaces - h->nface_int;
-      a.phase = PHASE_FACE_ONLY;
-      CK(launch_rhs_fp64(h->eq, dc, a, h->stream), "cut face launch");
-      a.phase = PHASE_LIFT;
-      CK(launch_rhs_fp64(h->eq, d, a, h->stream), "lift launch");
+    if (h->peers.empty()) {
+      CK(launch_stage64(h->eq, d, a, nullptr, 0, h->stream), "stage launch");
     } else {
-      a.phase = PHASE_FACE;
-      CK(launch_rhs_fp64(h->eq, d, a, h->stream), "face launch");
+      // the elements with a cut face; they share no output with the others
+      CK(launch_stage64(h->eq, d, a, h->elist_d + h->nel_int, h->K - h->nel_int, h->stream), "cut stage launch");
+      if (h->nel_int > 0) CK(cudaStreamWaitEvent(h->stream, h->ev_interior, 0), "stage event");
     }
   }
   if (stage == 4 && h->hlam)

@@ -266,21 +266,20 @@ template <int N> std::vector<double> pack64_t(const RefOps& o) {
     }
   for (int lane = 0; lane < 32; ++lane) {
     const int k = lane % 4, n = lane / 4;
-    for (int fb = 0; fb < P::FB; ++fb) {
-      const int p = std::min(8 * fb + n, NF - 1);  // a column past the last point repeats it
-      for (int fc = 0; fc < 3; ++fc)
-        for (int ks = 0; ks < P::EK && P::touches(fb, fc); ++ks) {
-          const int m = 4 * ks + k;
-          out[P::E_OFF + P::e_index(fb, fc, ks) * 32 + lane] = (p / NG == fc && m <= N) ? edge(p - fc * NG, m) : 0.0;
-        }
-    }
     for (int b = 0; b < P::NB; ++b) {
       const int node = P::out_node(b, n);
       if (node < 0) continue;
       for (int j = 0; j < 2; ++j) {
         for (int fb = 0; fb < P::FB; ++fb) {
           const int p = 8 * fb + 2 * k + j;
-          if (p < NF) out[P::L_OFF + ((fb * P::NB + b) * 32 + lane) * 2 + j] = o.Lift(node, p);
+          if (p < NF) out[P::L_OFF + ((fb * P::NB + b) * 32 + lane) * 2 + j] = o.Lift(node, p) * o.gw[p % NG];
+        }
+        for (int qb = 0; qb < P::QB; ++qb) {
+          const int p = 8 * qb + 2 * k + j;
+          if (p >= P::NFN) continue;
+          double acc = 0.0;
+          for (int g = 0; g < NG; ++g) acc += o.Lift(node, p / (N + 1) * NG + g) * o.gw[g] * edge(g, p % (N + 1));
+          out[P::Q_OFF + ((qb * P::NB + b) * 32 + lane) * 2 + j] = acc;
         }
         for (int pb = 0; pb < P::PB; ++pb) {
           const int c = 8 * pb + 2 * k + j;
@@ -298,19 +297,20 @@ template <int N> std::vector<double> pack64_t(const RefOps& o) {
       }
     }
     for (int pb = 0; pb < P::PB; ++pb) {
-      const int c = std::min(8 * pb + n, NC - 1);  // as for the face points
+      const int c = std::min(8 * pb + n, NC - 1);  // a column past the last point repeats it
       for (int ks = 0; ks < P::KS; ++ks) {
         const int from = P::node(ks, k);
         if (from < NP) out[P::V_OFF + ((pb * ((P::KS + 1) / 2) + ks / 2) * 32 + lane) * 2 + ks % 2] = o.Vc(c, from);
       }
     }
-    // T: the points of one face alone, in blocks of eight
-    for (int tb = 0; tb < P::TB; ++tb)
-      for (int ks = 0; ks < P::EK; ++ks) {
-        const int g = std::min(8 * tb + n, NG - 1), m = 4 * ks + k;
-        out[P::T_OFF + (tb * P::EK + ks) * 32 + lane] = m <= N ? edge(g, m) : 0.0;
-      }
   }
+  for (int fb = 0; fb < P::FB; ++fb)
+    for (int m = 0; m <= N; ++m)
+      for (int c = 0; c < 4; ++c)
+        for (int j = 0; j < 2; ++j) {
+          const int p = std::min(8 * fb + 2 * c, NF - 2) + j;  // a pair past the last repeats it
+          out[P::E_OFF + ((fb * (N + 1) + m) * 4 + c) * 2 + j] = edge(p % NG, m);
+        }
   return out;
 }
 

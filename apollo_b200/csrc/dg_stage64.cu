@@ -19,8 +19,11 @@
 //
 // Faces.  The trace on a face depends on the N + 1 nodes on that face only,
 // so a neighbour contributes those nodes (read from its state, or from the
-// ghost slot of a cut face), and both sides' traces are short contractions
-// with the one-dimensional interpolation E [NG][N+1].  Every element evaluates
+// ghost slot of a cut face), and both sides' traces are short sums with the
+// one-dimensional interpolation E [NG][N+1].  The linear equations evaluate
+// the numerical flux at those nodes (normal, boundary state and dissipation
+// are constant along a straight face, so it too commutes with E) and lift from
+// there.  Every element evaluates
 // its own faces, as Apollo does (wxnodaldg2dmethod.cc:389-472); no face buffer
 // makes a round trip through memory.
 //
@@ -38,27 +41,31 @@ namespace apollo {
 
 namespace {
 
-template <int EQ> constexpr bool kLinearEq = EQ == EQ_ADVECTION || EQ == EQ_MAXWELL || EQ == EQ_MAXWELL_TM;
-
 // Sizes of the chain for one equation and order (doubles unless said).
 template <int EQ, int N> struct Chain {
   static constexpr int M = Eq<EQ>::M;
   static constexpr int NP = Sizes<N>::NP, NC = Sizes<N>::NC, NG = Sizes<N>::NG, NF = Sizes<N>::NF;
   static constexpr bool LIN = kLinearEq<EQ>;
   using P = Pack64<N>;
-  static constexpr int KS = P::KS, NB = P::NB, PB = P::PB, FB = P::FB, EK = P::EK;
-  static constexpr int OPS = P::E_SIZE + P::L_SIZE + (LIN ? P::W_SIZE : P::V_SIZE + P::D_SIZE);
-  static constexpr int TAB = 2 * NG;                 // gz, gw
+  static constexpr int KS = P::KS, NB = P::NB, PB = P::PB, FB = P::FB;
+  // operators in shared memory: E | L | V | D, or Q | W
+  static constexpr int OPS_OFF = LIN ? P::Q_OFF : P::E_OFF, OPS = LIN ? P::S_OFF - P::Q_OFF : P::Q_OFF;
+  static constexpr int TAB = NG;                     // gz
   static constexpr int TABI = 3 * (N + 1);           // face node table (ints)
   static constexpr int SHARED = round_up(OPS + TAB + (TABI + 1) / 2, 2);
-  // per warp: states [8][NP M], neighbour face nodes [24][N+1][M], geometry
-  // [8][16], connectivity [24] int2
-  static constexpr int X = round_up(8 * NP * M, 2), PN = round_up(24 * (N + 1) * M, 2), G = 8 * 16, C = 24;
-  static constexpr int WARP = X + PN + G + C;
+  // per warp: states [8][NP M] and geometry [8][16], double buffered where that
+  // costs no resident warp (the next tile's arrive while this one computes),
+  // neighbour face nodes [24][N+1][M], connectivity [24] int2
+  static constexpr int X = 8 * NP * M, G = 8 * 16, PN = 24 * (N + 1) * M, C = 24;
+  static constexpr int XB = M == 8 ? 1 : 2;
+  static constexpr int WARP = XB * (X + G) + PN + C;
   static constexpr size_t bytes(int warps) { return sizeof(double) * (size_t)(SHARED + warps * WARP); }
   // warps per block (one block per SM): what the registers allow
   static constexpr int fit(int w) { return bytes(w) <= 227 * 1024 ? w : fit(w - 1); }
-  static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : (N >= 5 ? 8 : 12));
+  #ifndef XW
+#define XW (N >= 5 ? 8 : 12)
+#endif
+  static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : XW);
 };
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -70,6 +77,11 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
                : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+// all but the n newest groups have arrived
+template <int n> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(n) : "memory");
+}
 
 // n consecutive doubles, 16-byte accesses when ALIGNED (both counts even)
 template <int n, bool ALIGNED>
@@ -107,93 +119,113 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   using PK = Pack64<N>;
   using P = Eq<EQ>;
   constexpr int M = T::M, NP = T::NP, NG = T::NG, NF = T::NF;
-  constexpr int KS = T::KS, NB = T::NB, PB = T::PB, FB = T::FB, EK = T::EK;
+  constexpr int KS = T::KS, NB = T::NB, PB = T::PB, FB = T::FB, NFN = PK::NFN;
   constexpr bool EVEN = (NP * M) % 2 == 0;  // every element's state starts on a 16-byte boundary
   extern __shared__ __align__(16) double smem[];
-  // operator fragments: E | L | (V | D) or W
-  double* sE = smem;
-  double* sL = sE + PK::E_SIZE;
-  double* sV = sL + PK::L_SIZE;
+  double* sOps = smem;
   double* sGz = smem + T::OPS;
-  double* sGw = sGz + NG;
-  int* sFm = (int*)(sGw + NG);
+  int* sFm = (int*)(sGz + NG);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lc = lane & 3;
-  double* sX = smem + T::SHARED + warp * T::WARP;
-  double* sP = sX + T::X;
-  double* sG = sP + T::PN;
-  int2* sC = (int2*)(sG + T::G);
-  {
-    const double* src = d.pack64;
-    constexpr int head = PK::E_SIZE + PK::L_SIZE;
-    const double* tail = src + (T::LIN ? PK::W_OFF : PK::V_OFF);
-    for (int i = 2 * tid; i < head; i += 2 * blockDim.x) cp_async16(sE + i, src + i);
-    for (int i = 2 * tid; i < T::OPS - head; i += 2 * blockDim.x) cp_async16(sV + i, tail + i);
-    for (int i = tid; i < NG; i += blockDim.x) {
-      sGz[i] = d.gz[i];
-      sGw[i] = d.gw[i];
-    }
-    for (int i = tid; i < 3 * (N + 1); i += blockDim.x) sFm[i] = PK::face_node(i / (N + 1), i % (N + 1));
-    cp_async_wait_all();
-  }
+  double* sX0 = smem + T::SHARED + warp * T::WARP;  // XB x (states, geometry)
+  double* sP = sX0 + T::XB * (T::X + T::G);
+  int2* sC = (int2*)(sP + T::PN);
+  for (int i = 2 * tid; i < T::OPS; i += 2 * blockDim.x) cp_async16(sOps + i, d.pack64 + T::OPS_OFF + i);
+  for (int i = tid; i < NG; i += blockDim.x) sGz[i] = d.gz[i];
+  for (int i = tid; i < NFN; i += blockDim.x) sFm[i] = PK::face_node(i / (N + 1), i % (N + 1));
   // the last stage of a step (and a lone right-hand side) reduces the wave
   // speeds; an earlier stage clears the word instead
   const bool want_lam = a.mode != MODE_STAGE;
   if (a.mode == MODE_STAGE && a.reset_lambda && blockIdx.x == 0)
     for (int i = tid; i < d.ninst; i += blockDim.x) d.st[i].lam_bits = 0ull;
-  __syncthreads();
   int err = 0;
   LamAcc lam_acc;
   const int n = list ? nlist : d.K;
   const int ntiles = (n + 7) / 8;
   const int stride = gridDim.x * (blockDim.x >> 5);
-  for (int tile = warp * gridDim.x + blockIdx.x; tile < ntiles; tile += stride) {
-    // rows past the end repeat the last element (their results are not stored)
-    auto elem = [&](int r) {
-      const int i = min(tile * 8 + r, n - 1);
-      return list ? list[i] : i;
-    };
-    const bool row_ok = tile * 8 + lr < n;
-    const int ke = elem(lr);
-    __syncwarp();
-    if (lane < 24) sC[lane] = *reinterpret_cast<const int2*>(d.conn + (size_t)elem(lane / 3) * 6 + 2 * (lane % 3));
-    __syncwarp();
-    // states
+  // element of row r of a tile; rows past the end repeat the last element
+  // (their results are not stored)
+  auto elem = [&](int tile, int r) {
+    const int i = min(tile * 8 + r, n - 1);
+    return list ? list[i] : i;
+  };
+  auto load_conn = [&](int tile) {
+    int2 c = make_int2(0, -1);
+    if (lane < 24) c = *reinterpret_cast<const int2*>(d.conn + (size_t)elem(tile, lane / 3) * 6 + 2 * (lane % 3));
+    return c;
+  };
+  // a tile's states and geometry (rx, ry, sx, sy, J, 1/J, nx[3], ny[3], sJ[3])
+  auto load_tile = [&](int tile, double* X) {
     if (list == nullptr && tile * 8 + 8 <= n) {
       const double* src = a.x + (size_t)tile * 8 * NP * M;
 #pragma unroll 4
-      for (int i = lane; i < 4 * NP * M; i += 32) cp_async16(sX + 2 * i, src + 2 * i);
+      for (int i = lane; i < 4 * NP * M; i += 32) cp_async16(X + 2 * i, src + 2 * i);
     } else {
       for (int i = lane; i < 8 * NP * M; i += 32) {
         const int e = i / (NP * M);
-        cp_async8(sX + i, a.x + (size_t)elem(e) * NP * M + (i - e * NP * M));
+        cp_async8(X + i, a.x + (size_t)elem(tile, e) * NP * M + (i - e * NP * M));
       }
     }
-    // geometry: rx, ry, sx, sy, J, 1/J, nx[3], ny[3], sJ[3]
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int i = lane + 32 * u, e = i >> 3, q = i & 7;
-      cp_async16(sG + 16 * e + 2 * q, reinterpret_cast<const double*>(d.geo + elem(e)) + 2 * q);
+      cp_async16(X + T::X + 16 * e + 2 * q, reinterpret_cast<const double*>(d.geo + elem(tile, e)) + 2 * q);
     }
-    // the neighbours' nodes on the shared faces, in this side's node order (a
-    // boundary or cut face stands in its own nodes; the ghost state or the
-    // remote trace replaces what they interpolate to)
-    {
-      constexpr int CH = M % 2 == 0 ? 2 : 1, CN = M / CH, PER = (N + 1) * CN;  // doubles per copy, copies per node, face
-#pragma unroll 4
-      for (int i = lane; i < 24 * PER; i += 32) {
-        const int p = i / PER, r = i - p * PER, m = r / CN, c = (r - m * CN) * CH;
-        const int2 cn = sC[p];
-        const double* src;
-        if (cn.y < 0 || cn.x >= d.K) src = a.x + ((size_t)elem(p / 3) * NP + sFm[(p % 3) * (N + 1) + m]) * M;
-        else src = a.x + ((size_t)cn.x * NP + sFm[cn.y * (N + 1) + N - m]) * M;
-        if constexpr (CH == 2) cp_async16(sP + (p * (N + 1) + m) * M + c, src + c);
-        else cp_async8(sP + (p * (N + 1) + m) * M + c, src + c);
+  };
+  int tile = warp * gridDim.x + blockIdx.x;
+  int2 conn_next = make_int2(0, -1);
+  if (tile < ntiles) {
+    conn_next = load_conn(tile);
+    if (T::XB == 2) load_tile(tile, sX0);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  for (int it = 0; tile < ntiles; tile += stride, ++it) {
+    double* sX = sX0 + (T::XB == 2 && (it & 1) ? T::X + T::G : 0);
+    const bool row_ok = tile * 8 + lr < n;
+    const int ke = elem(tile, lr);
+    __syncwarp();  // the previous tile's reads are done
+    if (T::XB == 1) load_tile(tile, sX);
+    if (lane < 24) sC[lane] = conn_next;
+    __syncwarp();
+    // the neighbours' nodes on the shared faces, in this side's node order:
+    // from the neighbour's state, or the ghost slot of a cut face (the peer's
+    // order); a boundary face stands in its own nodes, and the ghost state
+    // replaces what they give.  They arrive during the volume term.
+#pragma unroll
+    for (int fc = 0; fc < 3; ++fc) {
+      const int2 cn = sC[lr * 3 + fc];
+      const double* from = a.x + (size_t)(cn.y < 0 ? ke : cn.x) * NP * M;
+      const bool ghost = cn.x >= d.K;
+      if (ghost) from = d.trace + ((size_t)cn.x * NF + cn.y * NG) * M;
+#pragma unroll
+      for (int k = 0; k < (N + 4) / 4; ++k) {
+        const int m = 4 * k + lc;
+        if (m > N) continue;
+        const double* src = from + (ghost ? N - m : sFm[cn.y < 0 ? fc * (N + 1) + m : cn.y * (N + 1) + N - m]) * M;
+        double* dst = sP + ((lr * 3 + fc) * (N + 1) + m) * M;
+        if constexpr (M % 2 == 0) {
+#pragma unroll
+          for (int c = 0; c < M; c += 2) cp_async16(dst + c, src + c);
+        } else {
+#pragma unroll
+          for (int c = 0; c < M; ++c) cp_async8(dst + c, src + c);
+        }
       }
     }
-    cp_async_wait_all();
+    cp_async_commit();
+    if (T::XB == 2) {
+      cp_async_wait<1>();  // this tile's states (all but the neighbours' nodes)
+    } else {
+      cp_async_wait<0>();
+    }
     __syncwarp();
+    if (tile + stride < ntiles) {
+      conn_next = load_conn(tile + stride);
+      if (T::XB == 2) load_tile(tile + stride, sX0 + ((it & 1) ? 0 : T::X + T::G));
+    }
+    cp_async_commit();
     const double* xe = sX + lr * NP * M;
-    const double* ge = sG + 16 * lr;
+    const double* ge = sX + T::X + 16 * lr;
     double acc[NB][M][2];
 #pragma unroll
     for (int b = 0; b < NB; ++b)
@@ -205,14 +237,15 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     if constexpr (T::LIN) {
 #pragma unroll
       for (int k = 0; k < KS; ++k) {
-        const int node = PK::node(k, lc);
+        const int node = min(PK::node(k, lc), NP - 1);  // past the last node the operator is zero
         double q[M], R[M], S[M];
 #pragma unroll
-        for (int f = 0; f < M; ++f) q[f] = node < NP ? xe[node * M + f] : 0.0;
-        volume_flux<EQ>(d.eqp, q, rx, ry, sx, sy, R, S, &err);
+        for (int f = 0; f < M; ++f) q[f] = xe[node * M + f];
+        LinearFast64<EQ>::along(d.eqp, q, rx, ry, R);
+        LinearFast64<EQ>::along(d.eqp, q, sx, sy, S);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-          const double2 w = reinterpret_cast<const double2*>(sV)[(k * NB + b) * 32 + lane];
+          const double2 w = reinterpret_cast<const double2*>(sOps + PK::Q_SIZE)[(k * NB + b) * 32 + lane];
 #pragma unroll
           for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], R[f], w.x);
 #pragma unroll
@@ -220,13 +253,13 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
         }
       }
     } else {
-      const double* sD = sV + PK::V_SIZE;
+      const double *sV = sOps + PK::V_OFF, *sD = sOps + PK::D_OFF;
       double q[KS][M];
 #pragma unroll
       for (int k = 0; k < KS; ++k) {
-        const int node = PK::node(k, lc);
+        const int node = min(PK::node(k, lc), NP - 1);  // past the last node the operator is zero
 #pragma unroll
-        for (int f = 0; f < M; ++f) q[k][f] = node < NP ? xe[node * M + f] : 0.0;
+        for (int f = 0; f < M; ++f) q[k][f] = xe[node * M + f];
       }
 #pragma unroll 1
       for (int pb = 0; pb < PB; ++pb) {
@@ -244,14 +277,13 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
             for (int f = 0; f < M; ++f) dmma_8x8x4(v[f], q[k + 1][f], w.y);
           }
         }
-        double R[2][M], S[2][M];
+        double qc[2][M], R[2][M], S[2][M];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          double qc[M];
-#pragma unroll
-          for (int f = 0; f < M; ++f) qc[f] = v[f][j];
-          volume_flux<EQ>(d.eqp, qc, rx, ry, sx, sy, R[j], S[j], &err);
+        for (int f = 0; f < M; ++f) {
+          qc[0][f] = v[f][0];
+          qc[1][f] = v[f][1];
         }
+        volume_flux_pair<EQ>(d.eqp, qc, rx, ry, sx, sy, R, S, &err);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
           const double2 wr = reinterpret_cast<const double2*>(sD)[((pb * 2 + 0) * NB + b) * 32 + lane];
@@ -302,73 +334,92 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     }
 
     // ---- surface term
-    const double miJ = -ge[5];
-    const double* se = sE + lane;
-#pragma unroll 1
-    for (int fb = 0; fb < FB; ++fb) {
-      double vm[M][2], vp[M][2];
-#pragma unroll
-      for (int f = 0; f < M; ++f) vm[f][0] = vm[f][1] = vp[f][0] = vp[f][1] = 0.0;
-      const int f_hi = min(8 * fb + 7, NF - 1) / NG;
-#pragma unroll 1
-      for (int fc = 8 * fb / NG; fc <= f_hi; ++fc) {
-#pragma unroll
-        for (int k = 0; k < EK; ++k, se += 32) {
-          const int m = 4 * k + lc;
-          const bool in = m <= N;
-          const double w = *se;
-          const double* om = xe + sFm[fc * (N + 1) + (in ? m : 0)] * M;
-          const double* pm = sP + ((lr * 3 + fc) * (N + 1) + (in ? m : 0)) * M;
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(vm[f], in ? om[f] : 0.0, w);
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(vp[f], in ? pm[f] : 0.0, w);
-        }
-      }
-      // two face points per lane, on one face (NG is even); points past the
-      // last repeat it (their lift columns are zero)
-      const int p0 = min(fb * 8 + 2 * lc, NF - 2);
-      const int fc = p0 / NG, g0 = p0 - fc * NG;
-      const double nx = ge[6 + fc], ny = ge[9 + fc], ws = miJ * ge[12 + fc];
-      const int2 cn = sC[lr * 3 + fc];
-      double A[2][M];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        double qM[M], qP[M], nf[M];
-#pragma unroll
-        for (int f = 0; f < M; ++f) {
-          qM[f] = vm[f][j];
-          qP[f] = vp[f][j];
-        }
-        if (cn.y < 0) {
-          // Gauss point coordinates on the face (wxcubature2d.cc:118-124)
-          const ElemGeo& g = d.geo[ke];
-          const double t = a.time_from_state ? d.st[inst].t + d.st[inst].dt * a.frac : a.t_arg;
-          const double z = sGz[g0 + j];
-          const double r = fc == 0 ? z : fc == 1 ? -z : -1.0;
-          const double s = fc == 0 ? -1.0 : fc == 1 ? z : -z;
-          const double x = 0.5 * (-g.vx[0] * (r + s) + g.vx[1] * (1. + r) + g.vx[2] * (1. + s));
-          const double y = 0.5 * (-g.vy[0] * (r + s) + g.vy[1] * (1. + r) + g.vy[2] * (1. + s));
-          apply_bc<EQ, double>(d.bcs, -cn.x, t, x, y, nx, ny, qM, qP);
-        } else if (cn.x >= d.K) {
-          // a cut face: the peer's trace, in its own point order
-          const double* tp = d.trace + ((size_t)cn.x * NF + cn.y * NG + (NG - 1 - g0 - j)) * M;
-#pragma unroll
-          for (int f = 0; f < M; ++f) qP[f] = tp[f];
-        }
-        const double lam = face_flux<EQ>(d.eqp, nx, ny, qM, qP, nf, &err);
-        if (want_lam) lam_acc.add(d.st, inst, fabs(lam));
-        const double w = ws * sGw[g0 + j];
-#pragma unroll
-        for (int f = 0; f < M; ++f) A[j][f] = nf[f] * w;
-      }
+    if (T::XB == 2) cp_async_wait<1>();  // all but the next tile's states
+    __syncwarp();
+    const double miJ = -0.5 * ge[5];  // the face fluxes come out twice
+    // the ghost state of one point of boundary face fc at face coordinate z
+    auto ghost_state = [&](int tag, int fc, double z, const double* q, double* qb) {
+      const ElemGeo& g = d.geo[ke];
+      const double t = a.time_from_state ? d.st[inst].t + d.st[inst].dt * a.frac : a.t_arg;
+      // point coordinates on the face (wxcubature2d.cc:118-124)
+      const double r = fc == 0 ? z : fc == 1 ? -z : -1.0;
+      const double s = fc == 0 ? -1.0 : fc == 1 ? z : -z;
+      const double x = 0.5 * (-g.vx[0] * (r + s) + g.vx[1] * (1. + r) + g.vx[2] * (1. + s));
+      const double y = 0.5 * (-g.vy[0] * (r + s) + g.vy[1] * (1. + r) + g.vy[2] * (1. + s));
+      apply_bc<EQ, double>(d.bcs, tag, t, x, y, ge[6 + fc], ge[9 + fc], q, qb);
+    };
+    auto lift = [&](const double* ops, int block, const double (*A)[M]) {
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
-        const double2 w = reinterpret_cast<const double2*>(sL)[(fb * NB + b) * 32 + lane];
+        const double2 w = reinterpret_cast<const double2*>(ops)[(block * NB + b) * 32 + lane];
 #pragma unroll
         for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], A[0][f], w.x);
 #pragma unroll
         for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], A[1][f], w.y);
+      }
+    };
+    if constexpr (T::LIN) {
+      // the flux at the face nodes, two per lane (a node past the last repeats
+      // it; its lift column is zero).  The linear equations' boundary states
+      // read neither position nor time.
+#pragma unroll 1
+      for (int qb = 0; qb < PK::QB; ++qb) {
+        double A[2][M];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int p = min(qb * 8 + 2 * lc + j, NFN - 1), fc = p / (N + 1);
+          const double *om = xe + sFm[p] * M, *pm = sP + (lr * NFN + p) * M;
+          double qM[M], qP[M];
+#pragma unroll
+          for (int f = 0; f < M; ++f) {
+            qM[f] = om[f];
+            qP[f] = pm[f];
+          }
+          const int2 cn = sC[lr * 3 + fc];
+          if (cn.y < 0) ghost_state(-cn.x, fc, 0.0, qM, qP);
+          const double lam = LinearFast64<EQ>::face2(d.eqp, ge[6 + fc], ge[9 + fc], miJ * ge[12 + fc], qM, qP, A[j]);
+          if (want_lam) lam_acc.add(d.st, inst, lam);
+        }
+        lift(sOps, qb, A);
+      }
+    } else {
+      const double* sL = sOps + PK::L_OFF;
+#pragma unroll 1
+      for (int fb = 0; fb < FB; ++fb) {
+        // two face points per lane, on one face (NG is even); a pair past the
+        // last repeats it (its lift columns are zero)
+        const int p0 = min(fb * 8 + 2 * lc, NF - 2);
+        const int fc = p0 / NG, g0 = p0 - fc * NG;
+        // both sides' traces from the face's nodes.  On the vector units: the
+        // N + 1 terms fill only part of the tensor instruction's k-steps, and
+        // both forms run at the float64 pipe's rate.
+        double qM[2][M], qP[2][M], A[2][M], lam[2];
+        const double2* se = reinterpret_cast<const double2*>(sOps) + fb * (N + 1) * 4 + lc;
+        const double* pm = sP + (lr * 3 + fc) * (N + 1) * M;
+#pragma unroll
+        for (int m = 0; m <= N; ++m) {
+          const double2 w = se[m * 4];
+          const double* om = xe + sFm[fc * (N + 1) + m] * M;
+#pragma unroll
+          for (int f = 0; f < M; ++f) {
+            const double o = om[f], p = pm[m * M + f];
+            qM[0][f] = m == 0 ? w.x * o : fma(w.x, o, qM[0][f]);
+            qM[1][f] = m == 0 ? w.y * o : fma(w.y, o, qM[1][f]);
+            qP[0][f] = m == 0 ? w.x * p : fma(w.x, p, qP[0][f]);
+            qP[1][f] = m == 0 ? w.y * p : fma(w.y, p, qP[1][f]);
+          }
+        }
+        const int2 cn = sC[lr * 3 + fc];
+        if (cn.y < 0) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) ghost_state(-cn.x, fc, sGz[g0 + j], qM[j], qP[j]);
+        }
+        face_flux2_pair<EQ>(d.eqp, ge[6 + fc], ge[9 + fc], miJ * ge[12 + fc], qM, qP, A, lam, &err);
+        if (want_lam) {
+          lam_acc.add(d.st, inst, fabs(lam[0]));
+          lam_acc.add(d.st, inst, fabs(lam[1]));
+        }
+        lift(sL, fb, A);
       }
     }
 
@@ -433,57 +484,30 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   if (err) atomicOr(&d.st->err, err);
 }
 
-// Traces of the cut faces blocks[0, n) (face 3 k + f of the state x) into dst
-// [n][NG][M], a warp per eight faces: the contraction a neighbour's own stage
-// would form them with (its node order, its k-steps), so the ranks of a
-// partitioned mesh compute what one handle on the whole mesh computes.
+// The N + 1 nodes on each of the cut faces blocks[0, n) (face 3 k + f of the
+// state x), in face order, into the first (N + 1) M values of its block of
+// dst [n][NG M].
 template <int M, int N>
-__global__ void __launch_bounds__(128) k_cut_traces(const double* __restrict__ x, const double* __restrict__ pack,
-                                                    const int* __restrict__ blocks, int n, double* __restrict__ dst) {
+__global__ void __launch_bounds__(128) k_cut_nodes(const double* __restrict__ x, const int* __restrict__ blocks, int n,
+                                                   double* __restrict__ dst) {
   using PK = Pack64<N>;
-  constexpr int NP = PK::NP, NG = PK::NG;
-  const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
-  const int row = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 8 + lr;
-  const int id = blocks[min(row, n - 1)];
-  const double* xe = x + (size_t)(id / 3) * NP * M;
-  double q[PK::EK][M];
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (i >= n * (N + 1)) return;
+  const int j = i / (N + 1), m = i - j * (N + 1), id = blocks[j];
+  const double* src = x + ((size_t)(id / 3) * PK::NP + PK::face_node(id % 3, m)) * M;
 #pragma unroll
-  for (int k = 0; k < PK::EK; ++k) {
-    const int m = 4 * k + lc;
-#pragma unroll
-    for (int f = 0; f < M; ++f) q[k][f] = m <= N ? xe[PK::face_node(id % 3, N - m) * M + f] : 0.0;
-  }
-#pragma unroll
-  for (int tb = 0; tb < PK::TB; ++tb) {
-    double v[M][2];
-#pragma unroll
-    for (int f = 0; f < M; ++f) v[f][0] = v[f][1] = 0.0;
-#pragma unroll
-    for (int k = 0; k < PK::EK; ++k) {
-      const double w = pack[PK::T_OFF + (tb * PK::EK + k) * 32 + lane];
-#pragma unroll
-      for (int f = 0; f < M; ++f) dmma_8x8x4(v[f], q[k][f], w);
-    }
-    if (row >= n) continue;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int g = 8 * tb + 2 * lc + j;  // the neighbour's point
-      if (g >= NG) continue;
-#pragma unroll
-      for (int f = 0; f < M; ++f) dst[((size_t)row * NG + (NG - 1 - g)) * M + f] = v[f][j];
-    }
-  }
+  for (int f = 0; f < M; ++f) dst[((size_t)j * PK::NG + m) * M + f] = src[f];
 }
 
 template <int EQ>
-cudaError_t cut_traces_n(const DgDev& d, const double* x, const int* blocks, int n, double* dst, cudaStream_t s) {
+cudaError_t cut_nodes_n(const DgDev& d, const double* x, const int* blocks, int n, double* dst, cudaStream_t s) {
   constexpr int M = Eq<EQ>::M;
-  const unsigned g = (unsigned)((n + 31) / 32);
+  const unsigned g = (unsigned)((n * (d.N + 1) + 127) / 128);
   switch (d.N) {
-    case 2: k_cut_traces<M, 2><<<g, 128, 0, s>>>(x, d.pack64, blocks, n, dst); break;
-    case 3: k_cut_traces<M, 3><<<g, 128, 0, s>>>(x, d.pack64, blocks, n, dst); break;
-    case 4: k_cut_traces<M, 4><<<g, 128, 0, s>>>(x, d.pack64, blocks, n, dst); break;
-    case 5: k_cut_traces<M, 5><<<g, 128, 0, s>>>(x, d.pack64, blocks, n, dst); break;
+    case 2: k_cut_nodes<M, 2><<<g, 128, 0, s>>>(x, blocks, n, dst); break;
+    case 3: k_cut_nodes<M, 3><<<g, 128, 0, s>>>(x, blocks, n, dst); break;
+    case 4: k_cut_nodes<M, 4><<<g, 128, 0, s>>>(x, blocks, n, dst); break;
+    case 5: k_cut_nodes<M, 5><<<g, 128, 0, s>>>(x, blocks, n, dst); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -539,15 +563,15 @@ cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int
   }
 }
 
-cudaError_t launch_cut_traces(int eq, const DgDev& d, const double* x, const int* blocks, int n, double* dst,
-                              cudaStream_t s) {
+cudaError_t launch_cut_nodes(int eq, const DgDev& d, const double* x, const int* blocks, int n, double* dst,
+                             cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   switch (eq) {
-    case EQ_ADVECTION: return cut_traces_n<EQ_ADVECTION>(d, x, blocks, n, dst, s);
-    case EQ_EULER: return cut_traces_n<EQ_EULER>(d, x, blocks, n, dst, s);
-    case EQ_MAXWELL: return cut_traces_n<EQ_MAXWELL>(d, x, blocks, n, dst, s);
-    case EQ_EULER2D: return cut_traces_n<EQ_EULER2D>(d, x, blocks, n, dst, s);
-    case EQ_MAXWELL_TM: return cut_traces_n<EQ_MAXWELL_TM>(d, x, blocks, n, dst, s);
+    case EQ_ADVECTION: return cut_nodes_n<EQ_ADVECTION>(d, x, blocks, n, dst, s);
+    case EQ_EULER: return cut_nodes_n<EQ_EULER>(d, x, blocks, n, dst, s);
+    case EQ_MAXWELL: return cut_nodes_n<EQ_MAXWELL>(d, x, blocks, n, dst, s);
+    case EQ_EULER2D: return cut_nodes_n<EQ_EULER2D>(d, x, blocks, n, dst, s);
+    case EQ_MAXWELL_TM: return cut_nodes_n<EQ_MAXWELL_TM>(d, x, blocks, n, dst, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -10,13 +10,15 @@
 // the even columns and is one k-step (node 8 b + k).  Points (cubature and
 // face) always come in blocks of eight with k-step j on the points
 // 8 b + 2 k + j.
-//   E  [entries][32]        interpolation along a face, one entry per (point block, face, k-step)
-//   L  [FB][NB][32][2 (j)]  surface lift
+//   E  [FB][N+1][4][2 (j)]  interpolation along a face to the points 8 b + 2 c + j (lane column c)
+//   L  [FB][NB][32][2 (j)]  surface lift with the Gauss weights
 //   V  [PB][ceil(KS/2)][32][2 (k-step)]   nodes -> cubature points
 //   D  [PB][2 (Dr, Ds)][NB][32][2 (j)]    weak derivatives
-//   W  [KS][NB][32][2 (Dr V, Ds V)]       their products (linear equations)
+// linear equations:
+//   Q  [QB][NB][32][2 (j)]  L E: surface lift from the 3 (N + 1) face nodes
+//   W  [KS][NB][32][2 (Dr V, Ds V)]       weak derivatives from the nodes
+// all:
 //   S  [PB][NB][32][2 (j)]                sources
-//   T  [TB][EK][32]                       interpolation along one face alone (cut faces)
 #pragma once
 
 #include "dg_device.cuh"
@@ -25,8 +27,8 @@ namespace apollo {
 
 template <int N> struct Pack64 {
   static constexpr int NP = Sizes<N>::NP, NC = Sizes<N>::NC, NG = Sizes<N>::NG, NF = Sizes<N>::NF;
-  static constexpr int KS = (NP + 3) / 4, NB = (NP + 7) / 8, PB = (NC + 7) / 8, FB = (NF + 7) / 8, EK = (N + 4) / 4,
-                       TB = (NG + 7) / 8;
+  static constexpr int KS = (NP + 3) / 4, NB = (NP + 7) / 8, PB = (NC + 7) / 8, FB = (NF + 7) / 8, NFN = 3 * (N + 1),
+                       QB = (NFN + 7) / 8;
   // whether block b holds its nodes in pairs (2 c, 2 c + 1 in one lane)
   APOLLO_HD static constexpr bool paired(int b) { return NP - 8 * b > 4; }
   // node of k-step `k`, k index c (NP or above: none)
@@ -44,30 +46,15 @@ template <int N> struct Pack64 {
     return f == 0 ? m : f == 1 ? row(m) + N - m : row(N - m);
   }
   APOLLO_HD static constexpr int row(int j) { return j * (N + 1) - j * (j - 1) / 2; }  // first node of row j
-  // whether point block fb has points of face fc (points past the last repeat it)
-  APOLLO_HD static constexpr bool touches(int fb, int fc) {
-    const int lo = 8 * fb, hi = 8 * fb + 7 < NF ? 8 * fb + 7 : NF - 1;
-    return lo / NG <= fc && fc <= hi / NG;
-  }
-  APOLLO_HD static constexpr int e_index(int fb, int fc, int k) {
-    int i = 0;
-    for (int b = 0; b < FB; ++b)
-      for (int f = 0; f < 3; ++f)
-        if (touches(b, f)) {
-          if (b == fb && f == fc) return i + k;
-          i += EK;
-        }
-    return i;  // (FB, 0, 0): the number of entries
-  }
-  static constexpr int E_SIZE = e_index(FB, 0, 0) * 32;
+  static constexpr int E_SIZE = FB * (N + 1) * 8;
   static constexpr int L_SIZE = FB * NB * 64;
   static constexpr int V_SIZE = PB * ((KS + 1) / 2) * 64;
   static constexpr int D_SIZE = PB * 2 * NB * 64;
+  static constexpr int Q_SIZE = QB * NB * 64;
   static constexpr int W_SIZE = KS * NB * 64;
   static constexpr int S_SIZE = PB * NB * 64;
-  static constexpr int T_SIZE = TB * EK * 32;
   static constexpr int E_OFF = 0, L_OFF = E_SIZE, V_OFF = L_OFF + L_SIZE, D_OFF = V_OFF + V_SIZE,
-                       W_OFF = D_OFF + D_SIZE, S_OFF = W_OFF + W_SIZE, T_OFF = S_OFF + S_SIZE, SIZE = T_OFF + T_SIZE;
+                       Q_OFF = D_OFF + D_SIZE, W_OFF = Q_OFF + Q_SIZE, S_OFF = W_OFF + W_SIZE, SIZE = S_OFF + S_SIZE;
 };
 
 }  // namespace apollo

@@ -255,8 +255,8 @@ class NodalDG2d:
         self._check(self.lib.apollo_dg_set_launch_shape(self.h, grid_share, tile_shape))
 
     def set_fp64_kernels(self, fused=True):
-        """Float64 stage kernels: True (1) the fused stage kernel, False (0, the
-        default) the volume, face and LIFT kernels, 2 the fused one on meshes
+        """Float64 stage kernels: True (1, the default) the fused stage kernel,
+        False (0) the volume, face and LIFT kernels, 2 the fused one on meshes
         of about one wave of tiles."""
         self._check(self.lib.apollo_dg_set_fp64_kernels(self.h, int(fused)))
 

@@ -181,17 +181,18 @@ apollo_status apollo_dg_set_limiter(apollo_dg* h, const char* kind, const double
  * in Apollo. */
 apollo_status apollo_dg_set_launch_shape(apollo_dg* h, int grid_share, int tile_shape);
 
-/* Float64 stage kernels of this handle.  0 (the default): the volume, face
- * and LIFT kernels.  1: the fused stage kernel (the volume and surface terms
- * and the stage update of a tile of elements in one pass, each element
- * evaluating its own faces as Apollo does, DRAM traffic near the compulsory
- * bytes) wherever it applies: a whole mesh, no source plugins, and a stage
- * whose output does not overlap its input.  2: the fused kernel where the
- * mesh's tiles fit about one wave of resident blocks (small meshes, where
- * three launches cost more than the work), the three kernels elsewhere (the
- * face kernel evaluates each face once, which a per-element pass cannot).
- * The forms agree within float64 round-off, not bit for bit, so the default
- * keeps every handle (whole, partitioned, batched) on the same arithmetic. */
+/* Float64 stage kernels of this handle.  1 (the default): the fused stage
+ * kernel (the volume and surface terms and the stage update of a tile of
+ * elements in one pass, each element evaluating its own faces as Apollo does)
+ * wherever it applies: a stage whose output does not overlap its input, on
+ * arrays that start on a 16-byte boundary (the handle's own always do; a
+ * caller's of apollo_dg_rhs that do not are evaluated by the three kernels).
+ * 0: the volume, face and LIFT kernels.  2: the fused kernel where the mesh's
+ * tiles fit about one wave of resident warps, the three kernels elsewhere.
+ * Partitioned meshes with peers always run the fused kernel, so that the ranks
+ * exchange the same data whatever each of them chose.  The forms agree within
+ * float64 round-off, not bit for bit; every handle (whole, partitioned,
+ * batched) starts in the same one. */
 apollo_status apollo_dg_set_fp64_kernels(apollo_dg* h, int fused);
 
 /* The element average of a nodal field is sum_n w[n] u[n]: w[Np] receives the
