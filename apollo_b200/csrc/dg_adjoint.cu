@@ -29,6 +29,7 @@
 #include "dg_adjoint.h"
 #include "dg_dmma.cuh"
 #include "dg_dual.cuh"
+#include "dg_euler_adj.cuh"
 
 namespace apollo {
 
@@ -239,37 +240,10 @@ template <int M> struct DVec {
   double v[M];
 };
 
-// (d f*(n, a, b) / d a)^T dv and, with want_b, (d f* / d b)^T dv, by forward
-// differentiation of the equation's own numerical flux (any Numerical_Flux)
-template <int EQ, int M>
-__device__ __forceinline__ void dual_face(const EqParams& P, double nx, double ny, const DVec<M>& a,
-                                          const DVec<M>& b, const DVec<M>& dv, DVec<M>& abar, DVec<M>& bbar,
-                                          bool want_b, int* err) {
-  for (int side = 0; side < (want_b ? 2 : 1); ++side) {
-    Dual<M> A[M], B[M], nf[M];
-#pragma unroll
-    for (int f = 0; f < M; ++f) {
-      A[f] = Dual<M>(a.v[f]);
-      B[f] = Dual<M>(b.v[f]);
-      if (side == 0) A[f].d[f] = 1.0;
-      else B[f].d[f] = 1.0;
-    }
-    Eq<EQ>::numflux(P, Dual<M>(nx), Dual<M>(ny), A, B, nf, err);
-    DVec<M>& out = side == 0 ? abar : bbar;
-#pragma unroll
-    for (int j = 0; j < M; ++j) {
-      double sum = 0.0;
-#pragma unroll
-      for (int f = 0; f < M; ++f) sum += dv.v[f] * nf[f].d[j];
-      out.v[j] = sum;
-    }
-  }
-}
-
-// The same by one-component forward passes (2 M evaluations of the flux in
-// Dual<1>, the instantiation the tangent kernels already use): for the Euler
-// fluxes other than Lax-Friedrichs, whose Dual<M> code would be several times
-// larger.
+// (d f*(n, a, b) / d a)^T dv and, with want_b, (d f* / d b)^T dv by
+// one-component forward passes of Apollo's own flux, quirks included (2 M
+// evaluations in Dual<1>, the instantiation the tangent kernels already use:
+// Dual<M> code would be several times larger).
 template <int EQ, int M>
 __device__ __forceinline__ void dual1_face(const EqParams& P, double nx, double ny, const DVec<M>& a,
                                            const DVec<M>& b, const DVec<M>& dv, DVec<M>& abar, DVec<M>& bbar,
@@ -296,111 +270,7 @@ __device__ __forceinline__ void dual1_face(const EqParams& P, double nx, double 
   }
 }
 
-template <int EQ> struct AdjPhys {
-  static constexpr int M = Eq<EQ>::M;
-  // (dR/dq)^T aR + (dS/dq)^T aS,  R = rx F + ry G,  S = sx F + sy G
-  __device__ __forceinline__ static DVec<M> vol(const EqParams& P, const DVec<M>& q, double rx, double ry,
-                                                double sx, double sy, const DVec<M>& aR, const DVec<M>& aS,
-                                                int* err) {
-    Dual<M> qc[M], F[M], G[M];
-#pragma unroll
-    for (int f = 0; f < M; ++f) {
-      qc[f] = Dual<M>(q.v[f]);
-      qc[f].d[f] = 1.0;
-    }
-    Eq<EQ>::flux2(P, qc, F, G, err);
-    DVec<M> r;
-#pragma unroll
-    for (int j = 0; j < M; ++j) r.v[j] = 0.0;
-#pragma unroll
-    for (int f = 0; f < M; ++f) {
-      const double cF = rx * aR.v[f] + sx * aS.v[f], cG = ry * aR.v[f] + sy * aS.v[f];
-#pragma unroll
-      for (int j = 0; j < M; ++j) r.v[j] += cF * F[f].d[j] + cG * G[f].d[j];
-    }
-    return r;
-  }
-  // (d f*(n, a, b) / d a)^T dv and (d f* / d b)^T dv (LF_ONLY: the caller
-  // knows the flux is Lax-Friedrichs; nothing to drop here)
-  template <bool LF_ONLY = false>
-  __device__ __forceinline__ static void face(const EqParams& P, double nx, double ny, const DVec<M>& a,
-                                              const DVec<M>& b, const DVec<M>& dv, DVec<M>& abar, DVec<M>& bbar,
-                                              bool want_b, int* err) {
-    dual_face<EQ, M>(P, nx, ny, a, b, dv, abar, bbar, want_b, err);
-  }
-};
-
-template <int MF> struct EulerAdj {
-  static constexpr int IE = MF - 1;
-  // qbar += (dR/dq)^T r for the flux R along (ax, ay): reverse sweep of the
-  // flux's own graph with its clamps (rho = max(q0, minD) as a constant when
-  // clamped; p = minP as a constant when clamped),
-  // rho, v = m / rho, p = g1 (E - rho |v|^2 / 2), u = v . a,
-  // R = (rho u, rho vx u + p ax, rho vy u + p ay, [rho vz u], (E + p) u)
-  __device__ __forceinline__ static void dir(const EqParams& P, const double* q, double ax, double ay,
-                                             const double* r, double* qbar, int* err) {
-    const double g1 = P.p[0] - 1.0, minP = P.p[1], minD = P.p[2];
-    double rho = q[0];
-    if (minD == 0.0 && rho <= 0.0) *err |= ERRB_NONPHYS;
-    const bool rho_c = rho < minD;
-    if (rho_c) rho = minD;
-    const double ir = 1.0 / rho;
-    const double vx = q[1] * ir, vy = q[2] * ir, vz = MF == 5 ? q[3] * ir : 0.0, E = q[IE];
-    const double v2 = vx * vx + vy * vy + vz * vz;
-    double p = g1 * (E - 0.5 * rho * v2);
-    bool p_c = false;
-    if (p <= 0.0) {
-      if (minP == 0.0) *err |= ERRB_NONPHYS;
-      else { p = minP; p_c = true; }
-    }
-    const double u = vx * ax + vy * ay;
-    const double r3 = MF == 5 ? r[3] : 0.0;
-    const double ub = r[0] * rho + r[1] * rho * vx + r[2] * rho * vy + r3 * rho * vz + r[IE] * (E + p);
-    const double pb = p_c ? 0.0 : r[1] * ax + r[2] * ay + r[IE] * u;
-    double rhob = (r[0] + r[1] * vx + r[2] * vy + r3 * vz) * u - 0.5 * g1 * v2 * pb;
-    const double vxb = r[1] * rho * u + ub * ax - g1 * rho * vx * pb;
-    const double vyb = r[2] * rho * u + ub * ay - g1 * rho * vy * pb;
-    const double vzb = r3 * rho * u - g1 * rho * vz * pb;
-    rhob -= (vxb * vx + vyb * vy + vzb * vz) * ir;
-    if (!rho_c) qbar[0] += rhob;
-    qbar[1] += vxb * ir;
-    qbar[2] += vyb * ir;
-    if (MF == 5) qbar[3] += vzb * ir;
-    qbar[IE] += r[IE] * u + g1 * pb;
-  }
-  // Lax-Friedrichs wave speed of the primitive variables and its gradient.
-  // Where the primitive variables clamp (non-physical states) the gradient is
-  // taken as zero and NONPHYS is flagged.
-  __device__ __forceinline__ static double speed(const EqParams& P, const double* q, double* grad, int* err) {
-    const double gamma = P.p[0], g1 = gamma - 1.0, minP = P.p[1], minD = P.p[2];
-    const double q3 = MF == 5 ? q[3] : 0.0;
-    if (!(q[0] > 0.0)) {
-      *err |= ERRB_NONPHYS;
-#pragma unroll
-      for (int j = 0; j < MF; ++j) grad[j] = 0.0;
-      return sqrt(gamma * minP / minD);
-    }
-    const double rho = q[0], ir = 1.0 / rho;
-    const double u = q[1] / rho, v = q[2] / rho, w = q3 / rho;
-    double p = g1 * (q[IE] - 0.5 * (q[1] * q[1] + q[2] * q[2] + q3 * q3) / q[0]);
-    const double sp = sqrt(u * u + v * v + w * w);
-    if (p <= 0.0) {
-      *err |= ERRB_NONPHYS;
-#pragma unroll
-      for (int j = 0; j < MF; ++j) grad[j] = 0.0;
-      return sp + sqrt(gamma * minP / rho);
-    }
-    const double cs = sqrt(gamma * p / rho);
-    const double ks = sp > 0.0 ? ir / sp : 0.0;  // d|v|/dm = v / (|v| rho)
-    const double kc = 0.5 * gamma / (cs * rho);   // dcs/dp = kc, dcs/drho = -kc p / rho
-    grad[0] = -sp * ir + kc * (0.5 * g1 * (u * u + v * v + w * w) - p * ir);
-    grad[1] = u * ks - kc * g1 * u;
-    grad[2] = v * ks - kc * g1 * v;
-    if (MF == 5) grad[3] = w * ks - kc * g1 * w;
-    grad[IE] = kc * g1;
-    return sp + cs;
-  }
-};
+template <int EQ> struct AdjPhys;
 
 template <int MF> struct EulerAdjPhys {
   static constexpr int M = MF;
@@ -414,41 +284,10 @@ template <int MF> struct EulerAdjPhys {
     EulerAdj<MF>::dir(P, q.v, sx, sy, aS.v, r.v, err);
     return r;
   }
-  // f* = 1/2 [Fn(a) + Fn(b) + lambda (a - b)], lambda = max(c(a), c(b)):
-  // abar = 1/2 [ (dFn(a)/da)^T dv + lambda dv + (dv . (a - b)) grad c(a) [a wins] ]
-  // bbar = 1/2 [ (dFn(b)/db)^T dv - lambda dv + (dv . (a - b)) grad c(b) [b wins] ]
-  template <bool LF_ONLY = false>
   __device__ __forceinline__ static void face(const EqParams& P, double nx, double ny, const DVec<M>& a,
                                               const DVec<M>& b, const DVec<M>& dv, DVec<M>& abar, DVec<M>& bbar,
                                               bool want_b, int* err) {
-    if constexpr (!LF_ONLY) {
-      if ((int)P.p[3] != NF_LF) {
-        // HLL, Roe, Wave: the derivative of Apollo's own flux, quirks included
-        dual1_face<MF == 5 ? EQ_EULER : EQ_EULER2D, M>(P, nx, ny, a, b, dv, abar, bbar, want_b, err);
-        return;
-      }
-    }
-    double ga[M], gb[M];
-    const double ca = EulerAdj<MF>::speed(P, a.v, ga, err), cb = EulerAdj<MF>::speed(P, b.v, gb, err);
-    const bool a_wins = ca > cb;  // the branch the forward flux takes
-    const double lam = a_wins ? ca : cb;
-    double jump = 0.0;
-#pragma unroll
-    for (int f = 0; f < M; ++f) jump += dv.v[f] * (a.v[f] - b.v[f]);
-    double fa[M];
-#pragma unroll
-    for (int j = 0; j < M; ++j) fa[j] = 0.0;
-    EulerAdj<MF>::dir(P, a.v, nx, ny, dv.v, fa, err);
-#pragma unroll
-    for (int j = 0; j < M; ++j) abar.v[j] = 0.5 * (fa[j] + lam * dv.v[j] + (a_wins ? jump * ga[j] : 0.0));
-    if (want_b) {
-      double fb[M];
-#pragma unroll
-      for (int j = 0; j < M; ++j) fb[j] = 0.0;
-      EulerAdj<MF>::dir(P, b.v, nx, ny, dv.v, fb, err);
-#pragma unroll
-      for (int j = 0; j < M; ++j) bbar.v[j] = 0.5 * (fb[j] - lam * dv.v[j] + (a_wins ? 0.0 : jump * gb[j]));
-    }
+    dual1_face<MF == 5 ? EQ_EULER : EQ_EULER2D, M>(P, nx, ny, a, b, dv, abar, bbar, want_b, err);
   }
 };
 template <> struct AdjPhys<EQ_EULER> : EulerAdjPhys<5> {};
@@ -532,11 +371,7 @@ __global__ void __launch_bounds__(kDThreads) k_adj_pre(DgDev d, const double* __
   }
 }
 
-// GEN: the general face code (boundary faces, and the Euler fluxes other
-// than Lax-Friedrichs); without it, the kernel for meshes with no boundary
-// face and a Lax-Friedrichs (or linear) flux, whose smaller code keeps more
-// of its state in registers.
-template <int EQ, int N, bool GEN>
+template <int EQ, int N>
 __global__ void __launch_bounds__(kDThreads, 2) k_adj_main(DgDev d, AdjArgs a) {
   using P = Eq<EQ>;
   constexpr int M = P::M;
@@ -604,7 +439,7 @@ __global__ void __launch_bounds__(kDThreads, 2) k_adj_main(DgDev d, AdjArgs a) {
       for (int j = 0; j < M; ++j) sQC[c * LDB + e * M + j] = gbar.v[j];
     }
     // faces: w_g (s_own - s_partner) d f*(n_own, a, b) / d a at every Gauss point
-    const bool two_sided = GEN && flux_two_sided<EQ>(d.eqp);
+    const bool two_sided = flux_two_sided<EQ>(d.eqp);
     for (int idx = tid; idx < ne * NF; idx += kDThreads) {
       const int e = idx / NF, fg = idx - e * NF, fc = fg / NG, gq = fg - fc * NG;
       const int k = k0 + e;
@@ -639,18 +474,14 @@ __global__ void __launch_bounds__(kDThreads, 2) k_adj_main(DgDev d, AdjArgs a) {
           for (int j = 0; j < M; ++j) abar.v[j] += bbar.v[j];
         } else {
 #pragma unroll
-        for (int f = 0; f < M; ++f) {
-          qa.v[f] = d.trace[own + f];
-          qb.v[f] = d.trace[par + f];
-          dvec.v[f] = w * (a.sbar[own + f] - a.sbar[par + f]);
+          for (int f = 0; f < M; ++f) {
+            qa.v[f] = d.trace[own + f];
+            qb.v[f] = d.trace[par + f];
+            dvec.v[f] = w * (a.sbar[own + f] - a.sbar[par + f]);
+          }
+          DVec<M> unused;
+          AdjPhys<EQ>::face(d.eqp, g.nx[fc], g.ny[fc], qa, qb, dvec, abar, unused, false, &err);
         }
-        DVec<M> unused;
-        AdjPhys<EQ>::template face<!GEN>(d.eqp, g.nx[fc], g.ny[fc], qa, qb, dvec, abar, unused, false, &err);
-        }
-      } else if constexpr (!GEN) {
-        // (the host launches this form only for meshes without boundary faces)
-#pragma unroll
-        for (int j = 0; j < M; ++j) abar.v[j] = 0.0;
       } else {
         // boundary: ghost state b = A a + c (every supported boundary hook is
         // affine in the trace); abar = (df*/da)^T dv + A^T (df*/db)^T dv
@@ -767,18 +598,10 @@ cudaError_t adjoint_t(const DgDev& d, const AdjArgs& a, cudaStream_t s) {
   static int rpre = 1, rmain = 1;
   cudaError_t e = set_smem(k_adj_pre<EQ, N>, T::PRE_BYTES, cpre, rpre);
   if (e != cudaSuccess) return e;
-  static unsigned clean = 0;
-  static int rlean = 1;
-  e = set_smem(k_adj_main<EQ, N, true>, T::MAIN_BYTES, cmain, rmain);
-  if (e != cudaSuccess) return e;
-  e = set_smem(k_adj_main<EQ, N, false>, T::MAIN_BYTES, clean, rlean);
+  e = set_smem(k_adj_main<EQ, N>, T::MAIN_BYTES, cmain, rmain);
   if (e != cudaSuccess) return e;
   k_adj_pre<EQ, N><<<tile_grid(d.K, T::E, rpre), kDThreads, T::PRE_BYTES, s>>>(d, a.x, a.wbar, a.sbar);
-  const bool lf = !(EQ == EQ_EULER || EQ == EQ_EULER2D) || (int)d.eqp.p[3] == NF_LF;
-  if (d.nbound == 0 && lf)
-    k_adj_main<EQ, N, false><<<tile_grid(d.K, T::E, rlean), kDThreads, T::MAIN_BYTES, s>>>(d, a);
-  else
-    k_adj_main<EQ, N, true><<<tile_grid(d.K, T::E, rmain), kDThreads, T::MAIN_BYTES, s>>>(d, a);
+  k_adj_main<EQ, N><<<tile_grid(d.K, T::E, rmain), kDThreads, T::MAIN_BYTES, s>>>(d, a);
   return cudaGetLastError();
 }
 
@@ -806,26 +629,21 @@ cudaError_t adjoint_n(const DgDev& d, const AdjArgs& a, cudaStream_t s) {
 
 }  // namespace
 
+// Apollo's fluxes other than Lax-Friedrichs go through the kernels above,
+// everything else through the fragment chain (dg_deriv64.cu)
+static bool general_flux(int eq, const DgDev& d) {
+  const int kind = (int)d.eqp.p[3];
+  return (eq == EQ_EULER || eq == EQ_EULER2D) && (kind == NF_HLL || kind == NF_ROE || kind == NF_WAVE);
+}
+
 cudaError_t launch_tangent_stage(int eq, const DgDev& d, const TanArgs& a, cudaStream_t s) {
-  switch (eq) {
-    case EQ_ADVECTION: return tangent_n<EQ_ADVECTION>(d, a, s);
-    case EQ_EULER: return tangent_n<EQ_EULER>(d, a, s);
-    case EQ_MAXWELL: return tangent_n<EQ_MAXWELL>(d, a, s);
-    case EQ_EULER2D: return tangent_n<EQ_EULER2D>(d, a, s);
-    case EQ_MAXWELL_TM: return tangent_n<EQ_MAXWELL_TM>(d, a, s);
-    default: return cudaErrorInvalidValue;
-  }
+  if (!general_flux(eq, d)) return launch_tangent64(eq, d, a, s);
+  return eq == EQ_EULER ? tangent_n<EQ_EULER>(d, a, s) : tangent_n<EQ_EULER2D>(d, a, s);
 }
 
 cudaError_t launch_adjoint_stage(int eq, const DgDev& d, const AdjArgs& a, cudaStream_t s) {
-  switch (eq) {
-    case EQ_ADVECTION: return adjoint_n<EQ_ADVECTION>(d, a, s);
-    case EQ_EULER: return adjoint_n<EQ_EULER>(d, a, s);
-    case EQ_MAXWELL: return adjoint_n<EQ_MAXWELL>(d, a, s);
-    case EQ_EULER2D: return adjoint_n<EQ_EULER2D>(d, a, s);
-    case EQ_MAXWELL_TM: return adjoint_n<EQ_MAXWELL_TM>(d, a, s);
-    default: return cudaErrorInvalidValue;
-  }
+  if (!general_flux(eq, d)) return launch_adjoint64(eq, d, a, s);
+  return eq == EQ_EULER ? adjoint_n<EQ_EULER>(d, a, s) : adjoint_n<EQ_EULER2D>(d, a, s);
 }
 
 }  // namespace apollo

@@ -7,9 +7,12 @@
 
 namespace apollo {
 
+// Both need arrays on 16-byte boundaries, and outputs that overlap no input but
+// z and du0 (they read the neighbours of x, dx and wbar).
+//
 // Tangent of a stage: dout = tangent of the stage result along dx (and du0
-// for MODE_FINAL), at the state x.  d.trace receives the traces of x;
-// dtrace, dvol, dflux are scratch ([K][NF][M], [K][NP][M], [K][NF][M]).
+// for MODE_FINAL), at the state x.  d.trace is scratch, as are dtrace, dvol,
+// dflux ([K][NF][M], [K][NP][M], [K][NF][M]).
 struct TanArgs {
   const double* x;
   const double* dx;
@@ -23,9 +26,8 @@ struct TanArgs {
 };
 
 // Adjoint of a stage: out = alpha * wbar + beta * L'(x)^T wbar + gamma * z
-// (z may be null).  d.trace receives the traces of x; sbar is scratch
-// [K][NF][M].  out may alias z (each element is read before it is written);
-// it may not alias x or wbar.
+// (z may be null).  d.trace and sbar [K][NF][M] are scratch.  out may alias z
+// (each element is read before it is written).
 struct AdjArgs {
   const double* x;
   const double* wbar;
@@ -38,5 +40,9 @@ struct AdjArgs {
 
 cudaError_t launch_tangent_stage(int eq, const DgDev& d, const TanArgs& a, cudaStream_t s);
 cudaError_t launch_adjoint_stage(int eq, const DgDev& d, const AdjArgs& a, cudaStream_t s);
+
+// Their fragment-chain form (dg_deriv64.cu): Lax-Friedrichs and linear fluxes
+cudaError_t launch_tangent64(int eq, const DgDev& d, const TanArgs& a, cudaStream_t s);
+cudaError_t launch_adjoint64(int eq, const DgDev& d, const AdjArgs& a, cudaStream_t s);
 
 }  // namespace apollo

@@ -27,6 +27,13 @@ __device__ __forceinline__ double sqrt_normal(double x) {
   return fma(g, e * fma(e, 0.375, 0.5), g);
 }
 
+__device__ __forceinline__ double rsqrt_normal(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+
 // Euler fluxes in float64 with one reciprocal of the density per state and
 // the flux formed along a direction directly (a n.F + b n.G in one pass): the
 // same quantities as WxEulerEqn's flux and Lax-Friedrichs flux
@@ -118,6 +125,133 @@ template <int MF> struct EulerFast64 {
     *lam = la > lb ? la : lb;
     return true;
   }
+  // qb = (d (aR . R + aS . S) / d q)^T of the fluxes R along (rx, ry), S along
+  // (sx, sy): with cF = rx aR + sx aS, cG = ry aR + sy aS the reverse sweep of
+  // cF . F + cG . G, F = (m1, m1 vx + p, m1 vy, (E + p) vx) and so on
+  __device__ __forceinline__ static void vol_t(const EqParams& P, const Side& s, const double* q, double rx, double ry,
+                                               double sx, double sy, const double* aR, const double* aS, double* qb) {
+    const double g1 = P.p[0] - 1.0;
+    double cF[MF], cG[MF];
+#pragma unroll
+    for (int f = 0; f < MF; ++f) {
+      cF[f] = rx * aR[f] + sx * aS[f];
+      cG[f] = ry * aR[f] + sy * aS[f];
+    }
+    const double Hp = q[IE] + s.p;
+    const double eb = cF[IE] * s.vx + cG[IE] * s.vy, pb = g1 * (cF[1] + cG[2] + eb);
+    const double xb = cF[1] * q[1] + cG[1] * q[2] + cF[IE] * Hp, yb = cF[2] * q[1] + cG[2] * q[2] + cG[IE] * Hp;
+    double zb = 0.0;
+    if (MF == 5) zb = cF[3] * q[1] + cG[3] * q[2];
+    qb[0] = fma(0.5 * pb, s.v2, -(xb * s.vx + yb * s.vy + zb * s.vz) * s.ir);
+    qb[1] = cF[0] + cF[1] * s.vx + cF[2] * s.vy + (MF == 5 ? cF[3] * s.vz : 0.0) + xb * s.ir - pb * s.vx;
+    qb[2] = cG[0] + cG[1] * s.vx + cG[2] * s.vy + (MF == 5 ? cG[3] * s.vz : 0.0) + yb * s.ir - pb * s.vy;
+    if (MF == 5) qb[3] = zb * s.ir - pb * s.vz;
+    qb[IE] = eb + pb;
+  }
+  // qb = (d (n . F) / d q)^T r
+  __device__ __forceinline__ static void along_t(const EqParams& P, const Side& s, const double* q, double nx,
+                                                 double ny, const double* r, double* qb) {
+    const double g1 = P.p[0] - 1.0, un = s.vx * nx + s.vy * ny;
+    const double ub = (r[1] * q[1] + r[2] * q[2] + (MF == 5 ? r[3] * q[3] : 0.0) + r[IE] * (q[IE] + s.p)) * s.ir;
+    const double pb = g1 * (r[1] * nx + r[2] * ny + r[IE] * un), t = r[0] + ub;
+    qb[0] = fma(0.5 * pb, s.v2, -ub * un);
+    qb[1] = r[1] * un + t * nx - pb * s.vx;
+    qb[2] = r[2] * un + t * ny - pb * s.vy;
+    if (MF == 5) qb[3] = r[3] * un - pb * s.vz;
+    qb[IE] = r[IE] * un + pb;
+  }
+  // flow speed + sound speed, and with the reciprocals of both the gradient
+  struct Speed {
+    double c, cs, rv, rc;  // sum, sound speed, 1 / flow speed, 1 / sound speed
+  };
+  __device__ __forceinline__ static Speed speeds(const EqParams& P, const Side& s) {
+    Speed r;
+    const double c2 = P.p[0] * s.p * s.ir;
+    r.rv = rsqrt_normal(s.v2);
+    r.rc = rsqrt_normal(c2);
+    r.cs = c2 * r.rc;
+    r.c = s.v2 * r.rv + r.cs;
+    return r;
+  }
+  // g += w grad c
+  __device__ __forceinline__ static void add_speed_grad(const EqParams& P, const Side& s, const Speed& v, double w,
+                                                        double* g) {
+    const double g1 = P.p[0] - 1.0;
+    const double kc = 0.5 * P.p[0] * s.ir * v.rc * g1, k = w * (v.rv * s.ir - kc);
+    g[0] += w * (0.5 * kc * s.v2 - (s.v2 * v.rv + 0.5 * v.cs) * s.ir);
+    g[1] += k * s.vx;
+    g[2] += k * s.vy;
+    if (MF == 5) g[3] += k * s.vz;
+    g[IE] += w * kc;
+  }
+  // (d f*/d a)^T dv and, with want_b, (d f*/d b)^T dv of twice the
+  // Lax-Friedrichs flux f* = Fn(a) + Fn(b) + max(c(a), c(b)) (a - b)
+  __device__ __forceinline__ static void lf2_t(const EqParams& P, const Side& a, const Side& b, const double* qM,
+                                               const double* qP, double nx, double ny, const double* dv, bool want_b,
+                                               double* ab, double* bb) {
+    const Speed ca = speeds(P, a), cb = speeds(P, b);
+    const bool a_wins = ca.c > cb.c;  // the branch the forward flux takes
+    const double lam = a_wins ? ca.c : cb.c;
+    double jump = 0.0;
+#pragma unroll
+    for (int f = 0; f < MF; ++f) jump += dv[f] * (qM[f] - qP[f]);
+    along_t(P, a, qM, nx, ny, dv, ab);
+#pragma unroll
+    for (int f = 0; f < MF; ++f) ab[f] += lam * dv[f];
+    if (a_wins) add_speed_grad(P, a, ca, jump, ab);
+    if (want_b) {
+      along_t(P, b, qP, nx, ny, dv, bb);
+#pragma unroll
+      for (int f = 0; f < MF; ++f) bb[f] -= lam * dv[f];
+      if (!a_wins) add_speed_grad(P, b, cb, jump, bb);
+    }
+  }
+  // derivatives along dq: of velocity and pressure, of the flux along (ax, ay),
+  // of the speed
+  struct Rate {
+    double vx, vy, vz, p;
+  };
+  __device__ __forceinline__ static Rate rate(const EqParams& P, const Side& s, const double* dq) {
+    const double g1 = P.p[0] - 1.0;
+    Rate r;
+    r.vx = (dq[1] - s.vx * dq[0]) * s.ir;
+    r.vy = (dq[2] - s.vy * dq[0]) * s.ir;
+    r.vz = MF == 5 ? (dq[3] - s.vz * dq[0]) * s.ir : 0.0;
+    double m = s.vx * dq[1] + s.vy * dq[2];
+    if (MF == 5) m += s.vz * dq[3];
+    r.p = g1 * (dq[IE] - m + 0.5 * s.v2 * dq[0]);
+    return r;
+  }
+  __device__ __forceinline__ static void along_d(const Side& s, const Rate& r, const double* q, const double* dq,
+                                                 double ax, double ay, double* R) {
+    const double un = s.vx * ax + s.vy * ay, du = r.vx * ax + r.vy * ay;
+    R[0] = dq[0] * un + s.rho * du;
+    R[1] = dq[1] * un + q[1] * du + r.p * ax;
+    R[2] = dq[2] * un + q[2] * du + r.p * ay;
+    if (MF == 5) R[3] = dq[3] * un + q[3] * du;
+    R[IE] = (dq[IE] + r.p) * un + (q[IE] + s.p) * du;
+  }
+  __device__ __forceinline__ static double speed_d(const EqParams& P, const Side& s, const Rate& r, const Speed& v,
+                                                   double drho) {
+    const double dv2 = s.vx * r.vx + s.vy * r.vy + (MF == 5 ? s.vz * r.vz : 0.0);
+    // cs^2 = gamma p / rho
+    return dv2 * v.rv + 0.5 * (P.p[0] * r.p * v.rc - v.cs * drho) * s.ir;
+  }
+  // derivative of twice the Lax-Friedrichs flux, times w
+  __device__ __forceinline__ static void lf2_d(const EqParams& P, const Side& a, const Side& b, const double* qM,
+                                               const double* qP, const double* dM, const double* dP, double nxw,
+                                               double nyw, double w, double* nf) {
+    const Rate ra = rate(P, a, dM), rb = rate(P, b, dP);
+    const Speed ca = speeds(P, a), cb = speeds(P, b);
+    const bool a_wins = ca.c > cb.c;
+    const double lam = w * (a_wins ? ca.c : cb.c);
+    const double dlam = w * (a_wins ? speed_d(P, a, ra, ca, dM[0]) : speed_d(P, b, rb, cb, dP[0]));
+    double FM[MF], FP[MF];
+    along_d(a, ra, qM, dM, nxw, nyw, FM);
+    along_d(b, rb, qP, dP, nxw, nyw, FP);
+#pragma unroll
+    for (int c = 0; c < MF; ++c) nf[c] = fma(dlam, qM[c] - qP[c], fma(lam, dM[c] - dP[c], FM[c] + FP[c]));
+  }
   // flow speed + sound speed
   __device__ __forceinline__ static double speed(const EqParams& P, const Side& s) {
     return sqrt_normal(s.v2) + sqrt_normal(P.p[0] * s.p * s.ir);
@@ -154,6 +288,47 @@ template <int EQ> struct LinearFast64 {
         R[5] = ax * q[1] - ay * q[0];
         R[6] = chi * (ax * q[0] + ay * q[1]);
         R[7] = gm * c2 * (ax * q[3] + ay * q[4]);
+      }
+    }
+  }
+  // qb = (d along / d q)^T r
+  __device__ __forceinline__ static void along_t(const EqParams& P, const double* r, double ax, double ay,
+                                                 double* qb) {
+    if constexpr (EQ == EQ_ADVECTION) {
+      qb[0] = (ax * P.p[0] + ay * P.p[1]) * r[0];
+    } else {
+      const double c2 = P.p[0] * P.p[0];
+      if constexpr (EQ == EQ_MAXWELL_TM) {
+        qb[0] = ay * r[1] - ax * r[2];
+        qb[1] = c2 * ay * r[0];
+        qb[2] = -c2 * ax * r[0];
+      } else {
+        const double gm = P.p[1], chi = P.p[2], c6 = chi * r[6], c7 = gm * c2 * r[7];
+        qb[0] = ax * c6 - ay * r[5];
+        qb[1] = ax * r[5] + ay * c6;
+        qb[2] = ay * r[3] - ax * r[4];
+        qb[3] = c2 * ay * r[2] + ax * c7;
+        qb[4] = ay * c7 - c2 * ax * r[2];
+        qb[5] = c2 * (ax * r[1] - ay * r[0]);
+        qb[6] = chi * c2 * (ax * r[0] + ay * r[1]);
+        qb[7] = gm * (ax * r[3] + ay * r[4]);
+      }
+    }
+  }
+  // dissipation of a jump, as face2 applies it (symmetric)
+  __device__ __forceinline__ static void dissipate(const EqParams& P, double nx, double ny, const double* dq,
+                                                   double* out) {
+    if constexpr (EQ == EQ_ADVECTION) {
+      const double lam = dmax2(fabs(P.p[0]), fabs(P.p[1]));
+      out[0] = ((int)P.p[3] == NF_UPWIND ? fabs(nx * P.p[0] + ny * P.p[1]) : lam) * dq[0];
+    } else {
+      const double lam = EQ == EQ_MAXWELL_TM ? P.p[0] : dmax3(P.p[2] * P.p[0], P.p[1] * P.p[0], P.p[0]);
+#pragma unroll
+      for (int f = 0; f < M; ++f) out[f] = lam * dq[f];
+      if (EQ == EQ_MAXWELL_TM && (int)P.p[3] == NF_UPWIND) {
+        const double bn = lam * (nx * dq[1] + ny * dq[2]);
+        out[1] -= bn * nx;
+        out[2] -= bn * ny;
       }
     }
   }

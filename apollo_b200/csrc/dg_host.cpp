@@ -1207,6 +1207,15 @@ apollo_status copy_in(apollo_dg* h, double* dst, const double* src, int where) {
   return APOLLO_OK;
 }
 
+// Whether a caller's device array can stand for one of the handle's: on a
+// 16-byte boundary and, for an output, clear of the inputs a and b.
+bool direct(const double* p) { return (uintptr_t)p % 16 == 0; }
+bool direct_out(const apollo_dg* h, const double* out, const double* a, const double* b) {
+  const size_t n = state_doubles(h);
+  auto apart = [n, out](const double* q) { return out + n <= q || q + n <= out; };
+  return direct(out) && apart(a) && apart(b);
+}
+
 apollo_status copy_out(apollo_dg* h, double* dst, const double* src, int where) {
   const size_t n = state_doubles(h) * sizeof(double);
   CK(cudaMemcpyAsync(dst, src, n, where == APOLLO_DEVICE_PTR ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
@@ -1648,11 +1657,12 @@ apollo_status apollo_dg_tangent(apollo_dg* h, int nsteps, double t0, double dt, 
   for (int n = 0; n < nsteps; ++n) {
     const double tn = t0 + n * dt;
     for (int s = 0; s < 5; ++s) {
-      // the tangent stage reads the stage's input state before the value stage replaces it
-      double* wb[2] = {h->W_d, h->W2_d};
+      // the tangent stage reads the stage's input state before the value stage replaces it;
+      // both alternate buffers (a stage reads its neighbours' inputs)
+      double *wb[2] = {h->W_d, h->W2_d}, *tb[2] = {h->tW_d, h->A_d[0]};
       const double* x = s == 0 ? h->U_d : wb[(s - 1) & 1];
-      const double* dx = s == 0 ? h->tU_d : h->tW_d;
-      double* dout = s < 4 ? h->tW_d : h->tU_d;
+      const double* dx = s == 0 ? h->tU_d : tb[(s - 1) & 1];
+      double* dout = s < 4 ? tb[s & 1] : h->tU_d;
       r = tangent_stage(h, s, s < 4 ? MODE_STAGE : MODE_FINAL, x, dx, s < 4 ? nullptr : h->tU_d, dout, tn, dt);
       if (!r) r = fixed_stage(h, s, x, h->U_d, s < 4 ? wb[s & 1] : h->U_d, tn, dt);
       if (r) return r;
@@ -1674,18 +1684,22 @@ apollo_status apollo_dg_rhs_jvp(apollo_dg* h, double t, const double* x, const d
   if (r) return r;
   const double *xd = x, *vd = v;
   double* od = out;
-  if (where != APOLLO_DEVICE_PTR) {
+  const bool dev = where == APOLLO_DEVICE_PTR;
+  if (!dev || !direct(x)) {
     r = copy_in(h, h->in_d, x, where);
-    if (!r) r = copy_in(h, h->tU_d, v, where);
     if (r) return r;
     xd = h->in_d;
-    vd = h->tU_d;
-    od = h->out_d;
   }
+  if (!dev || !direct(v)) {
+    r = copy_in(h, h->tU_d, v, where);
+    if (r) return r;
+    vd = h->tU_d;
+  }
+  if (!dev || !direct_out(h, out, x, v)) od = h->out_d;
   r = tangent_stage(h, 0, MODE_RHS, xd, vd, nullptr, od, t, 0.0);
   if (r) return r;
-  if (where != APOLLO_DEVICE_PTR) {
-    r = copy_out(h, out, h->out_d, where);
+  if (od != out) {
+    r = copy_out(h, out, od, where);
     if (r) return r;
   }
   return finish(h);
@@ -1704,18 +1718,22 @@ apollo_status apollo_dg_rhs_vjp(apollo_dg* h, double t, const double* x, const d
   if (r) return r;
   const double *xd = x, *wd = w;
   double* od = out;
-  if (where != APOLLO_DEVICE_PTR) {
+  const bool dev = where == APOLLO_DEVICE_PTR;
+  if (!dev || !direct(x)) {
     r = copy_in(h, h->in_d, x, where);
-    if (!r) r = copy_in(h, h->A_d[0], w, where);
     if (r) return r;
     xd = h->in_d;
-    wd = h->A_d[0];
-    od = h->out_d;
   }
+  if (!dev || !direct(w)) {
+    r = copy_in(h, h->A_d[0], w, where);
+    if (r) return r;
+    wd = h->A_d[0];
+  }
+  if (!dev || !direct_out(h, out, x, w)) od = h->out_d;
   r = adjoint_stage(h, xd, wd, nullptr, od, 0.0, 1.0, 0.0, t);
   if (r) return r;
-  if (where != APOLLO_DEVICE_PTR) {
-    r = copy_out(h, out, h->out_d, where);
+  if (od != out) {
+    r = copy_out(h, out, od, where);
     if (r) return r;
   }
   return finish(h);

@@ -287,6 +287,23 @@ template <int N> std::vector<double> pack64_t(const RefOps& o) {
           out[P::D_OFF + (((pb * 2 + 0) * P::NB + b) * 32 + lane) * 2 + j] = o.DrW(node, c);
           out[P::D_OFF + (((pb * 2 + 1) * P::NB + b) * 32 + lane) * 2 + j] = o.DsW(node, c);
           out[P::S_OFF + ((pb * P::NB + b) * 32 + lane) * 2 + j] = vs[(size_t)node * NC + c];
+          out[P::VT_OFF + ((pb * P::NB + b) * 32 + lane) * 2 + j] = o.Vc(c, node);
+        }
+        // the adjoint's face contributions reach the nodes of the face only
+        for (int fb = 0; fb < P::FB; ++fb) {
+          const int p = 8 * fb + 2 * k + j;
+          for (int m = 0; m <= N && p < NF; ++m)
+            if (P::face_node(p / NG, m) == node)
+              out[P::ET_OFF + ((fb * P::NB + b) * 32 + lane) * 2 + j] = o.gw[p % NG] * edge(p % NG, m);
+        }
+        for (int qb = 0; qb < P::QB; ++qb) {
+          const int p = 8 * qb + 2 * k + j;
+          for (int m = 0; m <= N && p < P::NFN; ++m)
+            if (P::face_node(p / (N + 1), m) == node) {
+              double acc = 0.0;
+              for (int g = 0; g < NG; ++g) acc += edge(g, m) * o.gw[g] * edge(g, p % (N + 1));
+              out[P::Z_OFF + ((qb * P::NB + b) * 32 + lane) * 2 + j] = acc;
+            }
         }
       }
       for (int ks = 0; ks < P::KS; ++ks) {
@@ -294,13 +311,20 @@ template <int N> std::vector<double> pack64_t(const RefOps& o) {
         if (from >= NP) continue;
         out[P::W_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 0] = W1(node, from);
         out[P::W_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 1] = W2(node, from);
+        out[P::WT_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 0] = W1(from, node);
+        out[P::WT_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 1] = W2(from, node);
+        out[P::Y_OFF + (ks * P::NB + b) * 32 + lane] = o.VVT(node, from);
       }
     }
     for (int pb = 0; pb < P::PB; ++pb) {
       const int c = std::min(8 * pb + n, NC - 1);  // a column past the last point repeats it
       for (int ks = 0; ks < P::KS; ++ks) {
         const int from = P::node(ks, k);
-        if (from < NP) out[P::V_OFF + ((pb * ((P::KS + 1) / 2) + ks / 2) * 32 + lane) * 2 + ks % 2] = o.Vc(c, from);
+        if (from >= NP) continue;
+        out[P::V_OFF + ((pb * ((P::KS + 1) / 2) + ks / 2) * 32 + lane) * 2 + ks % 2] = o.Vc(c, from);
+        if (8 * pb + n >= NC) continue;
+        out[P::DT_OFF + ((pb * P::KS + ks) * 32 + lane) * 2 + 0] = o.DrW(from, c);
+        out[P::DT_OFF + ((pb * P::KS + ks) * 32 + lane) * 2 + 1] = o.DsW(from, c);
       }
     }
   }

@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dg_chain64.cuh"
 #include "dg_device.cuh"
 #include "dg_dmma.cuh"
 #include "dg_flux64.cuh"
@@ -68,47 +69,6 @@ template <int EQ, int N> struct Chain {
   static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : XW);
 };
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// all but the n newest groups have arrived
-template <int n> __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(n) : "memory");
-}
-
-// n consecutive doubles, 16-byte accesses when ALIGNED (both counts even)
-template <int n, bool ALIGNED>
-__device__ __forceinline__ void load_run(const double* __restrict__ p, double* v) {
-  if constexpr (ALIGNED && n % 2 == 0) {
-#pragma unroll
-    for (int i = 0; i < n; i += 2) {
-      const double2 t = *reinterpret_cast<const double2*>(p + i);
-      v[i] = t.x;
-      v[i + 1] = t.y;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < n; ++i) v[i] = p[i];
-  }
-}
-template <int n, bool ALIGNED>
-__device__ __forceinline__ void store_run(double* __restrict__ p, const double* v) {
-  if constexpr (ALIGNED && n % 2 == 0) {
-#pragma unroll
-    for (int i = 0; i < n; i += 2) *reinterpret_cast<double2*>(p + i) = make_double2(v[i], v[i + 1]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < n; ++i) p[i] = v[i];
-  }
-}
-
 // One SSPRK stage (or right-hand side).  Reads the neighbours of x: x and out
 // must not overlap.  `list` (nlist entries) names the elements of this launch;
 // nullptr: all of them.
@@ -120,7 +80,6 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   using P = Eq<EQ>;
   constexpr int M = T::M, NP = T::NP, NG = T::NG, NF = T::NF;
   constexpr int KS = T::KS, NB = T::NB, PB = T::PB, FB = T::FB, NFN = PK::NFN;
-  constexpr bool EVEN = (NP * M) % 2 == 0;  // every element's state starts on a 16-byte boundary
   extern __shared__ __align__(16) double smem[];
   double* sOps = smem;
   double* sGz = smem + T::OPS;
@@ -155,10 +114,8 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   };
   // a tile's states and geometry (rx, ry, sx, sy, J, 1/J, nx[3], ny[3], sJ[3])
   auto load_tile = [&](int tile, double* X) {
-    if (list == nullptr && tile * 8 + 8 <= n) {
-      const double* src = a.x + (size_t)tile * 8 * NP * M;
-#pragma unroll 4
-      for (int i = lane; i < 4 * NP * M; i += 32) cp_async16(X + 2 * i, src + 2 * i);
+    if (list == nullptr) {
+      copy_tile<NP * M>(X, a.x, tile, n, lane);
     } else {
       for (int i = lane; i < 8 * NP * M; i += 32) {
         const int e = i / (NP * M);
@@ -202,14 +159,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
         const int m = 4 * k + lc;
         if (m > N) continue;
         const double* src = from + (ghost ? N - m : sFm[cn.y < 0 ? fc * (N + 1) + m : cn.y * (N + 1) + N - m]) * M;
-        double* dst = sP + ((lr * 3 + fc) * (N + 1) + m) * M;
-        if constexpr (M % 2 == 0) {
-#pragma unroll
-          for (int c = 0; c < M; c += 2) cp_async16(dst + c, src + c);
-        } else {
-#pragma unroll
-          for (int c = 0; c < M; ++c) cp_async8(dst + c, src + c);
-        }
+        cp_async_node<M>(sP + ((lr * 3 + fc) * (N + 1) + m) * M, src);
       }
     }
     cp_async_commit();
@@ -425,58 +375,38 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
 
     // ---- stage update, in the lanes that hold the nodes
     const double dt = a.time_from_state ? d.st[inst].dt : a.dt_arg;
-    const double c_stage = dt / 4.0;  // dt/(s-1), s = 5
-    const double c_al = 4.0 / 5.0, c_be = dt / 5.0, c_ga = 1.0 / 5.0;
+    const double c_r = a.mode == MODE_STAGE ? dt / 4.0 : dt / 5.0;  // dt/(s-1) and dt/s, s = 5
     if (row_ok) {
+      double* out = a.out + (size_t)ke * NP * M;
+      const double* u0 = a.u0 + (size_t)ke * NP * M;
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
-        constexpr int PAIR = 2 * M;
-        if (PK::paired(b)) {
-          // nodes n0, n0 + 1: 2 M consecutive values
-          const int n0 = b * 8 + 2 * lc;
-          if (n0 >= NP) continue;
-          const bool both = n0 + 1 < NP;
-          double r[PAIR], o[PAIR], xv[PAIR], uv[PAIR];
+        double o[M][2];
 #pragma unroll
-          for (int f = 0; f < M; ++f) {
-            r[f] = acc[b][f][0];
-            r[M + f] = acc[b][f][1];
-          }
+        for (int f = 0; f < M; ++f)
 #pragma unroll
-          for (int f = 0; f < PAIR; ++f) {
-            const bool use = f < M || both;
-            if (use && r[f] != r[f]) err |= ERRB_NAN;
-            xv[f] = use ? xe[n0 * M + f] : 0.0;
-            uv[f] = 0.0;
+          for (int j = 0; j < 2; ++j) {
+            o[f][j] = acc[b][f][j];
+            if (o[f][j] != o[f][j]) err |= ERRB_NAN;
           }
-          const size_t off = ((size_t)ke * NP + n0) * M;
-          if (a.mode == MODE_FINAL) {
-            if (both) load_run<PAIR, EVEN>(a.u0 + off, uv);
-            else load_run<M, EVEN>(a.u0 + off, uv);
-          }
+        if (a.mode != MODE_RHS) {
+          double x[M][2];
+          load_block<M, PK>(xe, b, lc, x);
+          if (a.mode == MODE_STAGE) {
 #pragma unroll
-          for (int f = 0; f < PAIR; ++f) {
-            if (a.mode == MODE_RHS) o[f] = r[f];
-            else if (a.mode == MODE_STAGE) o[f] = xv[f] + c_stage * r[f];
-            else o[f] = c_al * xv[f] + c_be * r[f] + c_ga * uv[f];
-          }
-          if (both) store_run<PAIR, EVEN>(a.out + off, o);
-          else store_run<M, EVEN>(a.out + off, o);
-        } else {
-          const int n0 = b * 8 + lc;
-          if (n0 >= NP) continue;
-          const size_t off = ((size_t)ke * NP + n0) * M;
+            for (int f = 0; f < M; ++f)
 #pragma unroll
-          for (int f = 0; f < M; ++f) {
-            const double r = acc[b][f][0], xv = xe[n0 * M + f];
-            if (r != r) err |= ERRB_NAN;
-            double o;
-            if (a.mode == MODE_RHS) o = r;
-            else if (a.mode == MODE_STAGE) o = xv + c_stage * r;
-            else o = c_al * xv + c_be * r + c_ga * a.u0[off + f];
-            a.out[off + f] = o;
+              for (int j = 0; j < 2; ++j) o[f][j] = x[f][j] + c_r * o[f][j];
+          } else {
+            double u[M][2];
+            load_block<M, PK>(u0, b, lc, u);
+#pragma unroll
+            for (int f = 0; f < M; ++f)
+#pragma unroll
+              for (int j = 0; j < 2; ++j) o[f][j] = (4.0 / 5.0) * x[f][j] + c_r * o[f][j] + (1.0 / 5.0) * u[f][j];
           }
         }
+        store_block<M, PK>(out, b, lc, o);
       }
     }
   }

@@ -19,6 +19,13 @@
 //   W  [KS][NB][32][2 (Dr V, Ds V)]       weak derivatives from the nodes
 // all:
 //   S  [PB][NB][32][2 (j)]                sources
+// adjoint (dg_deriv64.cu), the transposes:
+//   DT [PB][KS][32][2 (Dr, Ds)]           nodes -> cubature points
+//   VT [PB][NB][32][2 (j)]                cubature points -> nodes
+//   ET [FB][NB][32][2 (j)]                face points -> nodes with the Gauss weights
+//   Y  [KS][NB][32]                       V V^T (the lift is V V^T I^T)
+//   WT [KS][NB][32][2]                    of Dr V and Ds V (linear equations)
+//   Z  [QB][NB][32][2 (j)]                E^T diag(w) E per face, face nodes -> nodes (linear equations)
 #pragma once
 
 #include "dg_device.cuh"
@@ -54,7 +61,11 @@ template <int N> struct Pack64 {
   static constexpr int W_SIZE = KS * NB * 64;
   static constexpr int S_SIZE = PB * NB * 64;
   static constexpr int E_OFF = 0, L_OFF = E_SIZE, V_OFF = L_OFF + L_SIZE, D_OFF = V_OFF + V_SIZE,
-                       Q_OFF = D_OFF + D_SIZE, W_OFF = Q_OFF + Q_SIZE, S_OFF = W_OFF + W_SIZE, SIZE = S_OFF + S_SIZE;
+                       Q_OFF = D_OFF + D_SIZE, W_OFF = Q_OFF + Q_SIZE, S_OFF = W_OFF + W_SIZE;
+  static constexpr int DT_SIZE = PB * KS * 64, VT_SIZE = PB * NB * 64, ET_SIZE = FB * NB * 64, Y_SIZE = KS * NB * 32;
+  static constexpr int DT_OFF = S_OFF + S_SIZE, VT_OFF = DT_OFF + DT_SIZE, ET_OFF = VT_OFF + VT_SIZE,
+                       Y_OFF = ET_OFF + ET_SIZE, WT_OFF = Y_OFF + Y_SIZE, Z_OFF = WT_OFF + W_SIZE,
+                       SIZE = Z_OFF + Q_SIZE;
 };
 
 }  // namespace apollo

@@ -108,3 +108,63 @@ def test_overlapping_and_misaligned_arrays(kind):
         _, got = s.step(0.1, 0.01, x, out)
         assert rel_l2(out.cpu().numpy(), ref) <= 1e-12, name
         assert got == pytest.approx(sugg, rel=1e-14), name
+
+
+@pytest.mark.parametrize("K", [7, 25])
+@pytest.mark.parametrize("N", [2, 3, 4, 5])
+@pytest.mark.parametrize("kind,flux", [(k, CASES[k][2]) for k in CASES] + [("eulerEqn2d", "LF")])
+def test_derivatives_on_partial_tiles(kind, flux, N, K):
+    """The tangent against central differences of the right-hand side (step
+    1e-5 of the state: truncation 1e-10 of the third derivative, rounding 1e-16
+    / 1e-5 of the terms, so 1e-7 relative), the adjoint as its transpose."""
+    p, bc, _, _ = CASES[kind]
+    s = NodalDG2d(N, 0.5, kind, p, _mesh(K, seed=N + 3), bcs=(bc,), numerical_flux=flux)
+    rng = np.random.default_rng(K + N)
+    x, v, w = _state(kind, s.shape, rng), rng.standard_normal(s.shape), rng.standard_normal(s.shape)
+    if kind.startswith("euler") and flux != "LF":
+        x[..., 1:-1] *= 1.01  # off the integers of the truncated HLL bound
+    jv, jtw = s.rhs_jvp(0.2, x, v), s.rhs_vjp(0.2, x, w)
+    h = 1e-5
+    fd = (s.step(0.2, 0.0, x + h * v)[0] - s.step(0.2, 0.0, x - h * v)[0]) / (2 * h)
+    if flux != "HLL":
+        assert rel_l2(jv, fd) <= 1e-7
+    scale = np.linalg.norm(jv) * np.linalg.norm(w)
+    assert abs(np.vdot(jv, w) - np.vdot(v, jtw)) <= 1e-12 * scale
+
+
+def test_derivatives_with_overlapping_and_misaligned_arrays():
+    """Such arrays go through the handle's own buffers: the same bits."""
+    torch = pytest.importorskip("torch")
+    p, bc, _, _ = CASES["eulerEqn2d"]
+    s = NodalDG2d(3, 0.5, "eulerEqn2d", p, _mesh(25, seed=2), bcs=(bc,))
+    rng = np.random.default_rng(1)
+    x, v = _state("eulerEqn2d", s.shape, rng), rng.standard_normal(s.shape)
+    n, sh = x.size, s.shape
+    xd, vd = torch.from_numpy(x).cuda(), torch.from_numpy(v).cuda()
+    jv, jtv = s.rhs_jvp(0.0, xd, vd).cpu(), s.rhs_vjp(0.0, xd, vd).cpu()
+    buf = torch.zeros(3 * n + 6, dtype=torch.float64, device="cuda")
+    x1, v1, o1 = buf[1:1 + n].view(sh), buf[n + 1:2 * n + 1].view(sh), buf[2 * n + 3:3 * n + 3].view(sh)
+    x1.copy_(xd)
+    v1.copy_(vd)
+    s.rhs_jvp(0.0, x1, v1, o1)
+    assert torch.equal(o1.cpu(), jv)
+    s.rhs_vjp(0.0, x1, v1, o1)
+    assert torch.equal(o1.cpu(), jtv)
+    x2, v2 = xd.clone(), vd.clone()
+    s.rhs_jvp(0.0, x2, v2, v2)
+    assert torch.equal(v2.cpu(), jv)
+
+
+@pytest.mark.parametrize("kind", ["maxwellTM", "eulerEqn2d"])
+def test_tangent_trajectory_is_the_transpose_of_the_adjoint(kind):
+    """Two steps each way on a partial tile: the tangent's stage buffers."""
+    p, bc, _, _ = CASES[kind]
+    s = NodalDG2d(3, 0.5, kind, p, _mesh(25, seed=4), bcs=(bc,), numerical_flux="LF")
+    rng = np.random.default_rng(7)
+    x, v, w = _state(kind, s.shape, rng), rng.standard_normal(s.shape), rng.standard_normal(s.shape)
+    s.set_state(x)
+    du = s.tangent(2, 0.0, 1e-3, v)
+    s.set_state(x)
+    s.forward_fixed(2, 0.0, 1e-3, 1)
+    g = s.backward(w)
+    assert abs(np.vdot(du, w) - np.vdot(v, g)) <= 1e-12 * np.linalg.norm(du) * np.linalg.norm(w)
