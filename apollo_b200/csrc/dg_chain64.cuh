@@ -36,27 +36,46 @@ template <int n> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(n) : "memory");
 }
 
-// The eight elements 8 tile .. 8 tile + 7 of an array [n][per] into dst
-// [8][per], rows past the end repeating the last element; src starts on a
-// 16-byte boundary (eight elements of doubles then always do).
-template <int per>
+// Row strides (doubles) of a tile in shared memory, padded so that the lanes of
+// one access phase (two rows of four lanes for 16 bytes, four rows for 8) fall
+// on different banks: a whole element's nodes (per = NP M; an odd count is
+// copied without padding, 16 bytes at a time), a row's face nodes (3 (N+1) M),
+// and its geometry.
+constexpr int elem_stride(int per, int m) {
+  if (per % 2) return per;
+  if (m % 2 == 0) return per % 4 == 2 ? per : per + 2;
+  return per + (12 - per % 8) % 8;
+}
+constexpr int face_stride(int per, int m) { return m % 2 == 0 ? (per % 4 == 2 ? per : per + 2) : per | 1; }
+constexpr int kGeoStride = 18;
+
+// The eight elements 8 tile .. 8 tile + 7 of an array [n][per] into dst, one
+// every `stride` doubles, rows past the end repeating the last element; src
+// starts on a 16-byte boundary (eight elements of doubles then always do).
+template <int per, int stride>
 __device__ __forceinline__ void copy_tile(double* dst, const double* __restrict__ src, int tile, int n, int lane) {
   if (tile * 8 + 8 <= n) {
     const double* s = src + (size_t)tile * 8 * per;
+    if constexpr (per == stride) {
 #pragma unroll 4
-    for (int i = lane; i < 4 * per; i += 32) cp_async16(dst + 2 * i, s + 2 * i);
+      for (int i = lane; i < 4 * per; i += 32) cp_async16(dst + 2 * i, s + 2 * i);
+    } else {
+#pragma unroll 4
+      for (int i = lane; i < 4 * per; i += 32) cp_async16(dst + 2 * i + i / (per / 2) * (stride - per), s + 2 * i);
+    }
   } else {
     for (int i = lane; i < 8 * per; i += 32) {
       const int e = i / per;
-      cp_async8(dst + i, src + (size_t)min(tile * 8 + e, n - 1) * per + (i - e * per));
+      cp_async8(dst + e * stride + (i - e * per), src + (size_t)min(tile * 8 + e, n - 1) * per + (i - e * per));
     }
   }
 }
 
-// n consecutive doubles, 16-byte accesses when ALIGNED (both counts even)
-template <int n, bool ALIGNED>
+// n consecutive doubles, 16-byte accesses when n is even (a node of an even
+// number of fields starts on such a boundary)
+template <int n>
 __device__ __forceinline__ void load_run(const double* __restrict__ p, double* v) {
-  if constexpr (ALIGNED && n % 2 == 0) {
+  if constexpr (n % 2 == 0) {
 #pragma unroll
     for (int i = 0; i < n; i += 2) {
       const double2 t = *reinterpret_cast<const double2*>(p + i);
@@ -68,9 +87,9 @@ __device__ __forceinline__ void load_run(const double* __restrict__ p, double* v
     for (int i = 0; i < n; ++i) v[i] = p[i];
   }
 }
-template <int n, bool ALIGNED>
+template <int n>
 __device__ __forceinline__ void store_run(double* __restrict__ p, const double* v) {
-  if constexpr (ALIGNED && n % 2 == 0) {
+  if constexpr (n % 2 == 0) {
 #pragma unroll
     for (int i = 0; i < n; i += 2) *reinterpret_cast<double2*>(p + i) = make_double2(v[i], v[i + 1]);
   } else {
@@ -79,44 +98,30 @@ __device__ __forceinline__ void store_run(double* __restrict__ p, const double* 
   }
 }
 
-// A lane's node values of accumulator block b of one element, v[field][0, 1]
-// (PK: the order's Pack64, which says how the block holds its nodes).
+// A lane's node values of accumulator block b of one element, v[field][j] at
+// node 8 b + 4 j + lc (PK: the order's Pack64).
 template <int M, class PK>
 __device__ __forceinline__ void load_block(const double* __restrict__ e, int b, int lc, double (*v)[2]) {
-  constexpr bool EVEN = (PK::NP * M) % 2 == 0;
-  double t[2 * M];
 #pragma unroll
-  for (int f = 0; f < 2 * M; ++f) t[f] = 0.0;
-  if (PK::paired(b)) {
-    const int n0 = 8 * b + 2 * lc;
-    if (n0 + 1 < PK::NP) load_run<2 * M, EVEN>(e + n0 * M, t);
-    else if (n0 < PK::NP) load_run<M, EVEN>(e + n0 * M, t);
-  } else {
-    const int n0 = 8 * b + lc;
-    if (n0 < PK::NP) load_run<M, false>(e + n0 * M, t);
-  }
+  for (int j = 0; j < 2; ++j) {
+    const int n = 8 * b + 4 * j + lc;
+    double t[M];
 #pragma unroll
-  for (int f = 0; f < M; ++f) {
-    v[f][0] = t[f];
-    v[f][1] = t[M + f];
+    for (int f = 0; f < M; ++f) t[f] = 0.0;
+    if (n < PK::NP) load_run<M>(e + n * M, t);
+#pragma unroll
+    for (int f = 0; f < M; ++f) v[f][j] = t[f];
   }
 }
 template <int M, class PK>
 __device__ __forceinline__ void store_block(double* __restrict__ e, int b, int lc, const double (*v)[2]) {
-  constexpr bool EVEN = (PK::NP * M) % 2 == 0;
-  double t[2 * M];
 #pragma unroll
-  for (int f = 0; f < M; ++f) {
-    t[f] = v[f][0];
-    t[M + f] = v[f][1];
-  }
-  if (PK::paired(b)) {
-    const int n0 = 8 * b + 2 * lc;
-    if (n0 + 1 < PK::NP) store_run<2 * M, EVEN>(e + n0 * M, t);
-    else if (n0 < PK::NP) store_run<M, EVEN>(e + n0 * M, t);
-  } else {
-    const int n0 = 8 * b + lc;
-    if (n0 < PK::NP) store_run<M, false>(e + n0 * M, t);
+  for (int j = 0; j < 2; ++j) {
+    const int n = 8 * b + 4 * j + lc;
+    double t[M];
+#pragma unroll
+    for (int f = 0; f < M; ++f) t[f] = v[f][j];
+    if (n < PK::NP) store_run<M>(e + n * M, t);
   }
 }
 

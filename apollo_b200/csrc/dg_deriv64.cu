@@ -41,7 +41,8 @@ template <int EQ, int N> struct Deriv {
   static constexpr int ADJ_OPS = LIN ? P::W_SIZE + P::Q_SIZE : P::E_SIZE + P::V_SIZE + P::DT_SIZE + P::VT_SIZE + P::ET_SIZE;
   static constexpr int TAN_OPS = LIN ? P::S_OFF - P::Q_OFF : P::Q_OFF;
   static constexpr int TABS = NG + (3 * (N + 1) + 1) / 2;
-  static constexpr int X = 8 * NP * M, PN = 24 * (N + 1) * M, G = 8 * 16, C = 24;
+  static constexpr int ES = elem_stride(NP * M, M), FS = face_stride(3 * (N + 1) * M, M);
+  static constexpr int X = 8 * ES, PN = 8 * FS, G = 8 * kGeoStride, C = 24;
   static constexpr int WARP = (LIN ? 1 : 2) * (X + PN) + G + C;
   static constexpr size_t bytes(int ops, int warps) {
     return sizeof(double) * (size_t)(round_up(ops + TABS, 2) + warps * WARP);
@@ -92,8 +93,8 @@ __global__ void __launch_bounds__(128) k_adj_y(DgDev d, const double* __restrict
 }
 
 // The face nodes of array x that the tile's elements see across their faces,
-// in this side's order, into dst [24][N+1][M] (a boundary face: its own).
-template <int N, int M>
+// in this side's order, into dst [8][FS] (a boundary face: its own).
+template <int N, int M, int FS>
 __device__ __forceinline__ void copy_face_nodes(double* dst, const double* __restrict__ x, const int2* sC,
                                                 const int* sFm, int ke, int lr, int lc) {
   using PK = Pack64<N>;
@@ -105,7 +106,7 @@ __device__ __forceinline__ void copy_face_nodes(double* dst, const double* __res
     for (int k = 0; k < (N + 4) / 4; ++k) {
       const int m = 4 * k + lc;
       if (m > N) continue;
-      cp_async_node<M>(dst + ((lr * 3 + fc) * (N + 1) + m) * M,
+      cp_async_node<M>(dst + lr * FS + (fc * (N + 1) + m) * M,
                        from + sFm[cn.y < 0 ? fc * (N + 1) + m : cn.y * (N + 1) + N - m] * M);
     }
   }
@@ -144,16 +145,16 @@ template <int EQ, int N> struct Warp {
     __syncwarp();  // the previous tile's reads are done
     if (lane < 24)
       sC[lane] = *reinterpret_cast<const int2*>(d.conn + (size_t)min(tile * 8 + lane / 3, d.K - 1) * 6 + 2 * (lane % 3));
-    copy_tile<NP * M>(sB, b, tile, d.K, lane);
-    if (!T::LIN) copy_tile<NP * M>(sA, a, tile, d.K, lane);
+    copy_tile<NP * M, T::ES>(sB, b, tile, d.K, lane);
+    if (!T::LIN) copy_tile<NP * M, T::ES>(sA, a, tile, d.K, lane);
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int i = lane + 32 * u, e = i >> 3, q = i & 7;
-      cp_async16(sG + 16 * e + 2 * q, reinterpret_cast<const double*>(d.geo + min(tile * 8 + e, d.K - 1)) + 2 * q);
+      cp_async16(sG + kGeoStride * e + 2 * q, reinterpret_cast<const double*>(d.geo + min(tile * 8 + e, d.K - 1)) + 2 * q);
     }
     __syncwarp();
-    copy_face_nodes<N, M>(sPB, b, sC, sFm, ke, lr, lc);
-    if (!T::LIN) copy_face_nodes<N, M>(sPA, a, sC, sFm, ke, lr, lc);
+    copy_face_nodes<N, M, T::FS>(sPB, b, sC, sFm, ke, lr, lc);
+    if (!T::LIN) copy_face_nodes<N, M, T::FS>(sPA, a, sC, sFm, ke, lr, lc);
     cp_async_wait_all();
     __syncwarp();
   }
@@ -161,7 +162,7 @@ template <int EQ, int N> struct Warp {
   __device__ __forceinline__ void hook(const DgDev& d, int ke, int tag, int fc, double z, double t, const double* q,
                                        double* qb) const {
     const ElemGeo& g = d.geo[ke];
-    const double* ge = sG + 16 * lr;
+    const double* ge = sG + kGeoStride * lr;
     const double r = fc == 0 ? z : fc == 1 ? -z : -1.0;
     const double s = fc == 0 ? -1.0 : fc == 1 ? z : -z;
     const double x = 0.5 * (-g.vx[0] * (r + s) + g.vx[1] * (1. + r) + g.vx[2] * (1. + s));
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
 #pragma unroll
     for (int b = 0; b < NB; ++b) load_block<M, PK>(a.wbar + (size_t)ke * NP * M, b, lc, wv[b]);
     W.load(d, tile, a.x, y);
-    const double *ge = W.sG + 16 * lr, *xe = W.sA + lr * NP * M, *ye = W.sB + lr * NP * M;
+    const double *ge = W.sG + kGeoStride * lr, *xe = W.sA + lr * T::ES, *ye = W.sB + lr * T::ES;
     const double rx = ge[0], ry = ge[1], sx = ge[2], sy = ge[3];
     double acc[NB][M][2];
 #pragma unroll
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int p = min(qb * 8 + 2 * lc + j, PK::NFN - 1), fc = p / (N + 1);
-          const double *om = ye + W.sFm[p] * M, *pm = W.sPB + (lr * PK::NFN + p) * M;
+          const double *om = ye + W.sFm[p] * M, *pm = W.sPB + lr * T::FS + p * M;
           const double nx = ge[6 + fc], ny = ge[9 + fc], hs = 0.5 * ge[12 + fc];
           const int2 cn = W.sC[lr * 3 + fc];
           double dv[M], t[M];
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
         const bool wall = cn.y < 0;
         double qM[2][M], qP[2][M], dv[2][M], A[2][M];
         const double2* se = reinterpret_cast<const double2*>(sE) + fb * (N + 1) * 4 + lc;
-        const int face = (lr * 3 + fc) * (N + 1) * M;
+        const int face = lr * T::FS + fc * (N + 1) * M;
         const double hs = 0.5 * ge[12 + fc], nx = ge[6 + fc], ny = ge[9 + fc];
 #pragma unroll
         for (int m = 0; m <= N; ++m) {
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
   for (int tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; tile < ntiles; tile += gridDim.x * (blockDim.x >> 5)) {
     const int ke = min(tile * 8 + lr, d.K - 1);
     W.load(d, tile, a.x, a.dx);
-    const double *ge = W.sG + 16 * lr, *xe = W.sA + lr * NP * M, *de = W.sB + lr * NP * M;
+    const double *ge = W.sG + kGeoStride * lr, *xe = W.sA + lr * T::ES, *de = W.sB + lr * T::ES;
     const double rx = ge[0], ry = ge[1], sx = ge[2], sy = ge[3], miJ = -0.5 * ge[5];
     double acc[NB][M][2];
 #pragma unroll
@@ -471,7 +472,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int p = min(qb * 8 + 2 * lc + j, PK::NFN - 1), fc = p / (N + 1);
-          const double *om = de + W.sFm[p] * M, *pm = W.sPB + (lr * PK::NFN + p) * M;
+          const double *om = de + W.sFm[p] * M, *pm = W.sPB + lr * T::FS + p * M;
           double qM[M], qP[M];
 #pragma unroll
           for (int f = 0; f < M; ++f) {
@@ -525,7 +526,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
         const int2 cn = W.sC[lr * 3 + fc];
         double qM[2][M], qP[2][M], dM[2][M], dP[2][M], A[2][M];
         const double2* se = reinterpret_cast<const double2*>(sE) + fb * (N + 1) * 4 + lc;
-        const int face = (lr * 3 + fc) * (N + 1) * M;
+        const int face = lr * T::FS + fc * (N + 1) * M;
         const double w = miJ * ge[12 + fc], nx = ge[6 + fc], ny = ge[9 + fc];
 #pragma unroll
         for (int m = 0; m <= N; ++m) {

@@ -407,52 +407,52 @@ __device__ __forceinline__ void volume_flux_pair(const EqParams& P, const double
 }
 
 // Twice the numerical flux of one face point (qM, qP may be modified as the
-// reference modifies them) times w; the Euler Lax-Friedrichs flux of two clean
-// states through EulerFast64
-template <int EQ>
+// reference modifies them) times w.  GF: any numerical flux; otherwise the
+// Euler flux is Lax-Friedrichs.
+template <int EQ, bool GF>
 __device__ __forceinline__ double face_flux2(const EqParams& P, double nx, double ny, double w, double* qM, double* qP,
                                              double* nf, int* err) {
   constexpr int M = Eq<EQ>::M;
-  if constexpr (kEulerEq<EQ>) {
-    const int kind = (int)P.p[3];
-    if (kind != NF_HLL && kind != NF_ROE && kind != NF_WAVE) {
-      using X = EulerFast64<M>;
-      const typename X::Side a = X::side(P, qM), b = X::side(P, qP);
-      if (a.clean && b.clean) return X::lf2(P, a, b, qM, qP, w * nx, w * ny, w, nf);
-    }
+  double lam;
+  if constexpr (kEulerEq<EQ> && !GF) {
+    using X = EulerFast64<M>;
+    const typename X::Side a = X::side(P, qM), b = X::side(P, qP);
+    if (a.clean && b.clean) return X::lf2(P, a, b, qM, qP, w * nx, w * ny, w, nf);
+    lam = Eq<EQ>::lf(P, nx, ny, qM, qP, nf, err);
+  } else {
+    lam = Eq<EQ>::numflux(P, nx, ny, qM, qP, nf, err);
   }
-  const double lam = Eq<EQ>::numflux(P, nx, ny, qM, qP, nf, err);
 #pragma unroll
   for (int c = 0; c < M; ++c) nf[c] *= 2.0 * w;
   return lam;
 }
 
-// The same for two points of one face (HLL of clean states through EulerFast64 too)
-template <int EQ>
+// The same for two points of one face: one branch for both
+template <int EQ, bool GF>
 __device__ __forceinline__ void face_flux2_pair(const EqParams& P, double nx, double ny, double w,
                                                 double (*qM)[Eq<EQ>::M], double (*qP)[Eq<EQ>::M],
                                                 double (*nf)[Eq<EQ>::M], double* lam, int* err) {
   if constexpr (kEulerEq<EQ>) {
-    const int kind = (int)P.p[3];
-    if (kind != NF_ROE && kind != NF_WAVE) {
-      using X = EulerFast64<Eq<EQ>::M>;
-      const typename X::Side a0 = X::side(P, qM[0]), b0 = X::side(P, qP[0]);
-      const typename X::Side a1 = X::side(P, qM[1]), b1 = X::side(P, qP[1]);
-      if (a0.clean && b0.clean && a1.clean && b1.clean) {
-        if (kind != NF_HLL) {
-          const double nxw = w * nx, nyw = w * ny;
-          lam[0] = X::lf2(P, a0, b0, qM[0], qP[0], nxw, nyw, w, nf[0]);
-          lam[1] = X::lf2(P, a1, b1, qM[1], qP[1], nxw, nyw, w, nf[1]);
-          return;
-        }
-        if (X::hll2(P, a0, b0, qM[0], qP[0], nx, ny, w, nf[0], &lam[0]) &
-            X::hll2(P, a1, b1, qM[1], qP[1], nx, ny, w, nf[1], &lam[1]))
-          return;
+    using X = EulerFast64<Eq<EQ>::M>;
+    const typename X::Side a0 = X::side(P, qM[0]), b0 = X::side(P, qP[0]);
+    const typename X::Side a1 = X::side(P, qM[1]), b1 = X::side(P, qP[1]);
+    const bool clean = a0.clean && b0.clean && a1.clean && b1.clean;
+    if constexpr (!GF) {
+      if (clean) {
+        const double nxw = w * nx, nyw = w * ny;
+        lam[0] = X::lf2(P, a0, b0, qM[0], qP[0], nxw, nyw, w, nf[0]);
+        lam[1] = X::lf2(P, a1, b1, qM[1], qP[1], nxw, nyw, w, nf[1]);
+        return;
       }
+    } else {
+      if (clean && (int)P.p[3] == NF_HLL &&
+          (X::hll2(P, a0, b0, qM[0], qP[0], nx, ny, w, nf[0], &lam[0]) &
+           X::hll2(P, a1, b1, qM[1], qP[1], nx, ny, w, nf[1], &lam[1])))
+        return;
     }
   }
 #pragma unroll
-  for (int j = 0; j < 2; ++j) lam[j] = face_flux2<EQ>(P, nx, ny, w, qM[j], qP[j], nf[j], err);
+  for (int j = 0; j < 2; ++j) lam[j] = face_flux2<EQ, GF>(P, nx, ny, w, qM[j], qP[j], nf[j], err);
 }
 
 // The source plugins at one point (Apollo adds each into its output field,

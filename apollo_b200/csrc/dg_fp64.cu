@@ -221,7 +221,10 @@ __global__ void __launch_bounds__(kThreads) k_face(DgDev d, StageArgs a) {
       const double y = 0.5 * (-g.vy[0] * (r + s) + g.vy[1] * (1. + r) + g.vy[2] * (1. + s));
       apply_bc<EQ, double>(d.bcs, -fr.k2, t, x, y, nx, ny, qM, qP);
     }
-    double lam = face_flux2<EQ>(d.eqp, nx, ny, 0.5, qM, qP, nf, &err);
+    const int kind = (int)d.eqp.p[3];
+    const double lam = kind == NF_HLL || kind == NF_ROE || kind == NF_WAVE
+                           ? face_flux2<EQ, true>(d.eqp, nx, ny, 0.5, qM, qP, nf, &err)
+                           : face_flux2<EQ, false>(d.eqp, nx, ny, 0.5, qM, qP, nf, &err);
     lam_acc.add(d.st, inst, fabs(lam));
     const double w = d.gw[gq] * sJ;
     store_point<M>(d.flux + ((size_t)fr.k1 * NF + fr.f1 * NG + gq) * M, nf, w);

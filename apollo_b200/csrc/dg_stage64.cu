@@ -54,10 +54,11 @@ template <int EQ, int N> struct Chain {
   static constexpr int TAB = NG;                     // gz
   static constexpr int TABI = 3 * (N + 1);           // face node table (ints)
   static constexpr int SHARED = round_up(OPS + TAB + (TABI + 1) / 2, 2);
-  // per warp: states [8][NP M] and geometry [8][16], double buffered where that
+  // per warp: states [8][ES] and geometry [8][18], double buffered where that
   // costs no resident warp (the next tile's arrive while this one computes),
-  // neighbour face nodes [24][N+1][M], connectivity [24] int2
-  static constexpr int X = 8 * NP * M, G = 8 * 16, PN = 24 * (N + 1) * M, C = 24;
+  // neighbour face nodes [8][FS] (a row's three faces of N + 1 nodes), connectivity [24] int2
+  static constexpr int ES = elem_stride(NP * M, M), FS = face_stride(3 * (N + 1) * M, M);
+  static constexpr int X = 8 * ES, G = 8 * kGeoStride, PN = 8 * FS, C = 24;
   static constexpr int XB = M == 8 ? 1 : 2;
   static constexpr int WARP = XB * (X + G) + PN + C;
   static constexpr size_t bytes(int warps) { return sizeof(double) * (size_t)(SHARED + warps * WARP); }
@@ -71,8 +72,9 @@ template <int EQ, int N> struct Chain {
 
 // One SSPRK stage (or right-hand side).  Reads the neighbours of x: x and out
 // must not overlap.  `list` (nlist entries) names the elements of this launch;
-// nullptr: all of them.
-template <int EQ, int N>
+// nullptr: all of them.  GF: the Euler flux is HLL, Roe or Wave (a kernel of its
+// own, so that their code does not take registers from the others).
+template <int EQ, int N, bool GF>
 __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     k_stage64(DgDev d, StageArgs a, const int* __restrict__ list, int nlist) {
   using T = Chain<EQ, N>;
@@ -115,17 +117,17 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   // a tile's states and geometry (rx, ry, sx, sy, J, 1/J, nx[3], ny[3], sJ[3])
   auto load_tile = [&](int tile, double* X) {
     if (list == nullptr) {
-      copy_tile<NP * M>(X, a.x, tile, n, lane);
+      copy_tile<NP * M, T::ES>(X, a.x, tile, n, lane);
     } else {
       for (int i = lane; i < 8 * NP * M; i += 32) {
         const int e = i / (NP * M);
-        cp_async8(X + i, a.x + (size_t)elem(tile, e) * NP * M + (i - e * NP * M));
+        cp_async8(X + e * T::ES + (i - e * NP * M), a.x + (size_t)elem(tile, e) * NP * M + (i - e * NP * M));
       }
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int i = lane + 32 * u, e = i >> 3, q = i & 7;
-      cp_async16(X + T::X + 16 * e + 2 * q, reinterpret_cast<const double*>(d.geo + elem(tile, e)) + 2 * q);
+      cp_async16(X + T::X + kGeoStride * e + 2 * q, reinterpret_cast<const double*>(d.geo + elem(tile, e)) + 2 * q);
     }
   };
   int tile = warp * gridDim.x + blockIdx.x;
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
         const int m = 4 * k + lc;
         if (m > N) continue;
         const double* src = from + (ghost ? N - m : sFm[cn.y < 0 ? fc * (N + 1) + m : cn.y * (N + 1) + N - m]) * M;
-        cp_async_node<M>(sP + ((lr * 3 + fc) * (N + 1) + m) * M, src);
+        cp_async_node<M>(sP + lr * T::FS + (fc * (N + 1) + m) * M, src);
       }
     }
     cp_async_commit();
@@ -174,8 +176,8 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
       if (T::XB == 2) load_tile(tile + stride, sX0 + ((it & 1) ? 0 : T::X + T::G));
     }
     cp_async_commit();
-    const double* xe = sX + lr * NP * M;
-    const double* ge = sX + T::X + 16 * lr;
+    const double* xe = sX + lr * T::ES;
+    const double* ge = sX + T::X + kGeoStride * lr;
     double acc[NB][M][2];
 #pragma unroll
     for (int b = 0; b < NB; ++b)
@@ -318,7 +320,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int p = min(qb * 8 + 2 * lc + j, NFN - 1), fc = p / (N + 1);
-          const double *om = xe + sFm[p] * M, *pm = sP + (lr * NFN + p) * M;
+          const double *om = xe + sFm[p] * M, *pm = sP + lr * T::FS + p * M;
           double qM[M], qP[M];
 #pragma unroll
           for (int f = 0; f < M; ++f) {
@@ -345,7 +347,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
         // both forms run at the float64 pipe's rate.
         double qM[2][M], qP[2][M], A[2][M], lam[2];
         const double2* se = reinterpret_cast<const double2*>(sOps) + fb * (N + 1) * 4 + lc;
-        const double* pm = sP + (lr * 3 + fc) * (N + 1) * M;
+        const double* pm = sP + lr * T::FS + fc * (N + 1) * M;
 #pragma unroll
         for (int m = 0; m <= N; ++m) {
           const double2 w = se[m * 4];
@@ -364,7 +366,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
 #pragma unroll
           for (int j = 0; j < 2; ++j) ghost_state(-cn.x, fc, sGz[g0 + j], qM[j], qP[j]);
         }
-        face_flux2_pair<EQ>(d.eqp, ge[6 + fc], ge[9 + fc], miJ * ge[12 + fc], qM, qP, A, lam, &err);
+        face_flux2_pair<EQ, GF>(d.eqp, ge[6 + fc], ge[9 + fc], miJ * ge[12 + fc], qM, qP, A, lam, &err);
         if (want_lam) {
           lam_acc.add(d.st, inst, fabs(lam[0]));
           lam_acc.add(d.st, inst, fabs(lam[1]));
@@ -443,14 +445,14 @@ cudaError_t cut_nodes_n(const DgDev& d, const double* x, const int* blocks, int 
   return cudaGetLastError();
 }
 
-template <int EQ, int N>
+template <int EQ, int N, bool GF>
 cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s) {
   using T = Chain<EQ, N>;
   static unsigned configured = 0;  // bit per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(configured & (1u << (dev & 31)))) {
-    cudaError_t e = cudaFuncSetAttribute(k_stage64<EQ, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_stage64<EQ, N, GF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)T::bytes(T::WMAX));
     if (e != cudaSuccess) return e;
     configured |= 1u << (dev & 31);
@@ -465,17 +467,17 @@ cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nl
   const int tiles = (n + 7) / 8, grid = tiles < sms ? tiles : sms;
   int warps = (tiles + grid - 1) / grid;
   if (warps > T::WMAX) warps = T::WMAX;
-  k_stage64<EQ, N><<<grid, 32 * warps, T::bytes(warps), s>>>(d, a, list, nlist);
+  k_stage64<EQ, N, GF><<<grid, 32 * warps, T::bytes(warps), s>>>(d, a, list, nlist);
   return cudaGetLastError();
 }
 
-template <int EQ>
+template <int EQ, bool GF>
 cudaError_t dispatch_n(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s) {
   switch (d.N) {
-    case 2: return launch_t<EQ, 2>(d, a, list, nlist, s);
-    case 3: return launch_t<EQ, 3>(d, a, list, nlist, s);
-    case 4: return launch_t<EQ, 4>(d, a, list, nlist, s);
-    case 5: return launch_t<EQ, 5>(d, a, list, nlist, s);
+    case 2: return launch_t<EQ, 2, GF>(d, a, list, nlist, s);
+    case 3: return launch_t<EQ, 3, GF>(d, a, list, nlist, s);
+    case 4: return launch_t<EQ, 4, GF>(d, a, list, nlist, s);
+    case 5: return launch_t<EQ, 5, GF>(d, a, list, nlist, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -483,12 +485,17 @@ cudaError_t dispatch_n(const DgDev& d, const StageArgs& a, const int* list, int 
 }  // namespace
 
 cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s) {
+  const int kind = (int)d.eqp.p[3];
+  const bool gf = kind == NF_HLL || kind == NF_ROE || kind == NF_WAVE;  // Euler kinds only
   switch (eq) {
-    case EQ_ADVECTION: return dispatch_n<EQ_ADVECTION>(d, a, list, nlist, s);
-    case EQ_EULER: return dispatch_n<EQ_EULER>(d, a, list, nlist, s);
-    case EQ_MAXWELL: return dispatch_n<EQ_MAXWELL>(d, a, list, nlist, s);
-    case EQ_EULER2D: return dispatch_n<EQ_EULER2D>(d, a, list, nlist, s);
-    case EQ_MAXWELL_TM: return dispatch_n<EQ_MAXWELL_TM>(d, a, list, nlist, s);
+    case EQ_ADVECTION: return dispatch_n<EQ_ADVECTION, false>(d, a, list, nlist, s);
+    case EQ_EULER:
+      return gf ? dispatch_n<EQ_EULER, true>(d, a, list, nlist, s) : dispatch_n<EQ_EULER, false>(d, a, list, nlist, s);
+    case EQ_MAXWELL: return dispatch_n<EQ_MAXWELL, false>(d, a, list, nlist, s);
+    case EQ_EULER2D:
+      return gf ? dispatch_n<EQ_EULER2D, true>(d, a, list, nlist, s)
+                : dispatch_n<EQ_EULER2D, false>(d, a, list, nlist, s);
+    case EQ_MAXWELL_TM: return dispatch_n<EQ_MAXWELL_TM, false>(d, a, list, nlist, s);
     default: return cudaErrorInvalidValue;
   }
 }

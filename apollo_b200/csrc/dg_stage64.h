@@ -3,13 +3,12 @@
 // them, built once per mesh by build_pack64 (dg_operators.cpp) and copied to
 // shared memory by every block.
 //
-// Lane l holds B[k = l % 4][n = l / 4].  Nodes: accumulator block b covers the
-// nodes 8 b .. 8 b + 7; where more than four of them exist, column c is node
-// 8 b + c and the block is two k-steps as an A operand (step 2 b + j: nodes
-// 8 b + 2 k + j); a last block of at most four nodes puts node 8 b + c / 2 in
-// the even columns and is one k-step (node 8 b + k).  Points (cubature and
-// face) always come in blocks of eight with k-step j on the points
-// 8 b + 2 k + j.
+// Lane l holds B[k = l % 4][n = l / 4].  Nodes: k-step s holds the nodes
+// 4 s + k; accumulator block b has node 8 b + 4 (n % 2) + n / 2 in column n, so
+// a lane's two columns are its nodes of the k-steps 2 b and 2 b + 1 (four
+// neighbouring lanes then hold four consecutive nodes: their shared-memory and
+// global accesses are consecutive).  Points (cubature and face) come in blocks
+// of eight with k-step j on the points 8 b + 2 k + j.
 //   E  [FB][N+1][4][2 (j)]  interpolation along a face to the points 8 b + 2 c + j (lane column c)
 //   L  [FB][NB][32][2 (j)]  surface lift with the Gauss weights
 //   V  [PB][ceil(KS/2)][32][2 (k-step)]   nodes -> cubature points
@@ -36,15 +35,11 @@ template <int N> struct Pack64 {
   static constexpr int NP = Sizes<N>::NP, NC = Sizes<N>::NC, NG = Sizes<N>::NG, NF = Sizes<N>::NF;
   static constexpr int KS = (NP + 3) / 4, NB = (NP + 7) / 8, PB = (NC + 7) / 8, FB = (NF + 7) / 8, NFN = 3 * (N + 1),
                        QB = (NFN + 7) / 8;
-  // whether block b holds its nodes in pairs (2 c, 2 c + 1 in one lane)
-  APOLLO_HD static constexpr bool paired(int b) { return NP - 8 * b > 4; }
   // node of k-step `k`, k index c (NP or above: none)
-  APOLLO_HD static constexpr int node(int k, int c) {
-    return paired(k / 2) ? 8 * (k / 2) + 2 * c + k % 2 : 8 * (k / 2) + c;
-  }
+  APOLLO_HD static constexpr int node(int k, int c) { return 4 * k + c; }
   // node of column n of accumulator block b (-1: none)
   APOLLO_HD static constexpr int out_node(int b, int n) {
-    const int v = paired(b) ? 8 * b + n : n % 2 == 0 ? 8 * b + n / 2 : NP;
+    const int v = 8 * b + 4 * (n % 2) + n / 2;
     return v < NP ? v : -1;
   }
   // node m (0..N) of face f in face order: the edges of the triangular node
