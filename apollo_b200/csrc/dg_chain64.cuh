@@ -71,6 +71,38 @@ __device__ __forceinline__ void copy_tile(double* dst, const double* __restrict_
   }
 }
 
+// Where a (row, face) pair's nodes come from: element (or ghost slot) x, y =
+// its face | 4: in reverse order | 8: a ghost slot of face-node blocks.
+__device__ __forceinline__ int2 face_source(int2 conn, int own, int face, int K) {
+  if (conn.y < 0) return make_int2(own, face);  // boundary: its own nodes stand in
+  return make_int2(conn.x, conn.y | 4 | (conn.x >= K ? 8 : 0));
+}
+// Bulk copies from shared to global memory (16-byte boundaries and sizes): the
+// writes of a tile's rows as the lanes that issue them see fit; read_done
+// before the shared memory is reused, all_done before the block ends.
+__device__ __forceinline__ void bulk_store(double* dst, const double* src, int bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst),
+               "r"((unsigned)__cvta_generic_to_shared(src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_read_done() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+__device__ __forceinline__ void bulk_all_done() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+// a full tile [8][stride] of elements of `per` doubles to global memory
+template <int per, int stride>
+__device__ __forceinline__ void bulk_store_tile(double* dst, const double* src, int lane) {
+  fence_async_proxy();
+  __syncwarp();
+  if constexpr (per % 2 == 0) {
+    if (lane < 8) bulk_store(dst + lane * per, src + lane * stride, per * 8);
+  } else {
+    static_assert(per == stride, "rows of an odd count are not padded");
+    if (lane == 0) bulk_store(dst, src, 8 * per * 8);
+  }
+  bulk_commit();
+}
+
 // n consecutive doubles, 16-byte accesses when n is even (a node of an even
 // number of fields starts on such a boundary)
 template <int n>

@@ -56,18 +56,20 @@ template <int EQ, int N> struct Chain {
   static constexpr int SHARED = round_up(OPS + TAB + (TABI + 1) / 2, 2);
   // per warp: states [8][ES] and geometry [8][18], double buffered where that
   // costs no resident warp (the next tile's arrive while this one computes),
-  // neighbour face nodes [8][FS] (a row's three faces of N + 1 nodes), connectivity [24] int2
+  // neighbour face nodes [8][FS] (a row's three faces of N + 1 nodes), connectivity
+  // [24] int2 and where the face nodes come from [24] int2
   static constexpr int ES = elem_stride(NP * M, M), FS = face_stride(3 * (N + 1) * M, M);
-  static constexpr int X = 8 * ES, G = 8 * kGeoStride, PN = 8 * FS, C = 24;
+  static constexpr int X = 8 * ES, G = 8 * kGeoStride, PN = 8 * FS, C = 48;
   static constexpr int XB = M == 8 ? 1 : 2;
+  // results leave by bulk copies where a row is long enough to pay for one:
+  // K = 130,050: Euler N = 4 (480 bytes a row) 209 -> 204 us, Maxwell TM N = 5
+  // (one copy of 4,032) 105 -> 95; Euler N = 2 (192 bytes) 89 -> 93
+  static constexpr bool BULK = NP * M >= 30;
   static constexpr int WARP = XB * (X + G) + PN + C;
   static constexpr size_t bytes(int warps) { return sizeof(double) * (size_t)(SHARED + warps * WARP); }
   // warps per block (one block per SM): what the registers allow
   static constexpr int fit(int w) { return bytes(w) <= 227 * 1024 ? w : fit(w - 1); }
-  #ifndef XW
-#define XW (N >= 5 ? 8 : 12)
-#endif
-  static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : XW);
+    static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : (N >= 5 ? 8 : 12));
 };
 
 // One SSPRK stage (or right-hand side).  Reads the neighbours of x: x and out
@@ -89,7 +91,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lc = lane & 3;
   double* sX0 = smem + T::SHARED + warp * T::WARP;  // XB x (states, geometry)
   double* sP = sX0 + T::XB * (T::X + T::G);
-  int2* sC = (int2*)(sP + T::PN);
+  int2 *sC = (int2*)(sP + T::PN), *sS = sC + 24;
   for (int i = 2 * tid; i < T::OPS; i += 2 * blockDim.x) cp_async16(sOps + i, d.pack64 + T::OPS_OFF + i);
   for (int i = tid; i < NG; i += blockDim.x) sGz[i] = d.gz[i];
   for (int i = tid; i < NFN; i += blockDim.x) sFm[i] = PK::face_node(i / (N + 1), i % (N + 1));
@@ -142,9 +144,13 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     double* sX = sX0 + (T::XB == 2 && (it & 1) ? T::X + T::G : 0);
     const bool row_ok = tile * 8 + lr < n;
     const int ke = elem(tile, lr);
+    if (T::XB == 1) bulk_read_done();
     __syncwarp();  // the previous tile's reads are done
     if (T::XB == 1) load_tile(tile, sX);
-    if (lane < 24) sC[lane] = conn_next;
+    if (lane < 24) {
+      sC[lane] = conn_next;
+      sS[lane] = face_source(conn_next, elem(tile, lane / 3), lane % 3, d.K);
+    }
     __syncwarp();
     // the neighbours' nodes on the shared faces, in this side's node order:
     // from the neighbour's state, or the ghost slot of a cut face (the peer's
@@ -152,16 +158,15 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     // replaces what they give.  They arrive during the volume term.
 #pragma unroll
     for (int fc = 0; fc < 3; ++fc) {
-      const int2 cn = sC[lr * 3 + fc];
-      const double* from = a.x + (size_t)(cn.y < 0 ? ke : cn.x) * NP * M;
-      const bool ghost = cn.x >= d.K;
-      if (ghost) from = d.trace + ((size_t)cn.x * NF + cn.y * NG) * M;
+      const int2 s = sS[lr * 3 + fc];
+      const int f = s.y & 3;
+      const double* from = (s.y & 8) ? d.trace + ((size_t)s.x * NF + f * NG) * M : a.x + (size_t)s.x * NP * M;
 #pragma unroll
       for (int k = 0; k < (N + 4) / 4; ++k) {
         const int m = 4 * k + lc;
         if (m > N) continue;
-        const double* src = from + (ghost ? N - m : sFm[cn.y < 0 ? fc * (N + 1) + m : cn.y * (N + 1) + N - m]) * M;
-        cp_async_node<M>(sP + lr * T::FS + (fc * (N + 1) + m) * M, src);
+        const int mm = s.y & 4 ? N - m : m;
+        cp_async_node<M>(sP + lr * T::FS + (fc * (N + 1) + m) * M, from + ((s.y & 8) ? mm : sFm[f * (N + 1) + mm]) * M);
       }
     }
     cp_async_commit();
@@ -170,13 +175,14 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     } else {
       cp_async_wait<0>();
     }
+    if (T::XB == 2) bulk_read_done();  // the other buffer's results are on their way
     __syncwarp();
     if (tile + stride < ntiles) {
       conn_next = load_conn(tile + stride);
       if (T::XB == 2) load_tile(tile + stride, sX0 + ((it & 1) ? 0 : T::X + T::G));
     }
     cp_async_commit();
-    const double* xe = sX + lr * T::ES;
+    double* xe = sX + lr * T::ES;
     const double* ge = sX + T::X + kGeoStride * lr;
     double acc[NB][M][2];
 #pragma unroll
@@ -378,9 +384,15 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     // ---- stage update, in the lanes that hold the nodes
     const double dt = a.time_from_state ? d.st[inst].dt : a.dt_arg;
     const double c_r = a.mode == MODE_STAGE ? dt / 4.0 : dt / 5.0;  // dt/(s-1) and dt/s, s = 5
+    // a full tile's results replace its states in shared memory and leave by
+    // bulk copies; rows of a partial tile or of a list, and short rows, are
+    // stored from here
+    const bool whole = T::BULK && list == nullptr && tile * 8 + 8 <= n;
+    if (whole) __syncwarp();  // the states have been read
     if (row_ok) {
       double* out = a.out + (size_t)ke * NP * M;
       const double* u0 = a.u0 + (size_t)ke * NP * M;
+      int top = 0;  // the largest exponent and leading fraction: above infinity's, a NaN
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         double o[M][2];
@@ -389,7 +401,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             o[f][j] = acc[b][f][j];
-            if (o[f][j] != o[f][j]) err |= ERRB_NAN;
+            top = max(top, __double2hiint(o[f][j]) & 0x7fffffff);
           }
         if (a.mode != MODE_RHS) {
           double x[M][2];
@@ -408,10 +420,14 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
               for (int j = 0; j < 2; ++j) o[f][j] = (4.0 / 5.0) * x[f][j] + c_r * o[f][j] + (1.0 / 5.0) * u[f][j];
           }
         }
-        store_block<M, PK>(out, b, lc, o);
+        if (whole) store_block<M, PK>(xe, b, lc, o);
+        else store_block<M, PK>(out, b, lc, o);
       }
+      if (top > 0x7ff00000) err |= ERRB_NAN;
     }
+    if (whole) bulk_store_tile<NP * M, T::ES>(a.out + (size_t)tile * 8 * NP * M, sX, lane);
   }
+  bulk_all_done();
   if (want_lam) lam_acc.flush_warp(d.st);
   if (err) atomicOr(&d.st->err, err);
 }
