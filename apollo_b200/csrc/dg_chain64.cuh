@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "dg_device.cuh"
+#include "dg_dmma.cuh"
 
 namespace apollo {
 
@@ -156,5 +157,81 @@ __device__ __forceinline__ void store_block(double* __restrict__ e, int b, int l
     if (n < PK::NP) store_run<M>(e + n * M, t);
   }
 }
+
+// A lane's node accumulators of one element: a[b][f][j] at node 8 b + 4 j + lc,
+// and this lane's share of the TL nodes past the last block.
+template <int M, class PK> struct Nodes {
+  double a[PK::NB][M][2];
+  double t[PK::TL > 0 ? PK::TL : 1][M];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int b = 0; b < PK::NB; ++b)
+#pragma unroll
+      for (int f = 0; f < M; ++f) a[b][f][0] = a[b][f][1] = 0.0;
+#pragma unroll
+    for (int n = 0; n < PK::TL; ++n)
+#pragma unroll
+      for (int f = 0; f < M; ++f) t[n][f] = 0.0;
+  }
+  // += the contraction of two A operands with a "nodes" entry in memory (the
+  // fields of a mask, the same in the whole warp; the others' operands are zero)
+  __device__ __forceinline__ void add(const double* entry, int lane, const double* A0, const double* A1,
+                                      unsigned fields = ~0u) {
+#pragma unroll
+    for (int b = 0; b < PK::NB; ++b) {
+      const double2 w = reinterpret_cast<const double2*>(entry)[b * 32 + lane];
+#pragma unroll
+      for (int f = 0; f < M; ++f)
+        if (fields >> f & 1) dmma_8x8x4(a[b][f], A0[f], w.x);
+#pragma unroll
+      for (int f = 0; f < M; ++f)
+        if (fields >> f & 1) dmma_8x8x4(a[b][f], A1[f], w.y);
+    }
+#pragma unroll
+    for (int n = 0; n < PK::TL; ++n) {
+      const double2 w = reinterpret_cast<const double2*>(entry + PK::NB * 64)[n * 4 + (lane & 3)];
+#pragma unroll
+      for (int f = 0; f < M; ++f) t[n][f] = fma(A1[f], w.y, fma(A0[f], w.x, t[n][f]));
+    }
+  }
+  // += with the first of the pair only
+  __device__ __forceinline__ void add1(const double* entry, int lane, const double* A0) {
+#pragma unroll
+    for (int b = 0; b < PK::NB; ++b) {
+      const double w = entry[(b * 32 + lane) * 2];
+#pragma unroll
+      for (int f = 0; f < M; ++f) dmma_8x8x4(a[b][f], A0[f], w);
+    }
+#pragma unroll
+    for (int n = 0; n < PK::TL; ++n) {
+      const double w = entry[PK::NB * 64 + (n * 4 + (lane & 3)) * 2];
+#pragma unroll
+      for (int f = 0; f < M; ++f) t[n][f] = fma(A0[f], w, t[n][f]);
+    }
+  }
+  // the four lanes' shares together (all lanes of the warp)
+  __device__ __forceinline__ void finish() {
+#pragma unroll
+    for (int n = 0; n < PK::TL; ++n)
+#pragma unroll
+      for (int f = 0; f < M; ++f) {
+        t[n][f] += __shfl_xor_sync(0xffffffffu, t[n][f], 1);
+        t[n][f] += __shfl_xor_sync(0xffffffffu, t[n][f], 2);
+      }
+  }
+  // block b of NBT as load_block has it
+  __device__ __forceinline__ void get(int b, int lc, double (*v)[2]) const {
+#pragma unroll
+    for (int f = 0; f < M; ++f) {
+      if (b < PK::NB) {
+        v[f][0] = a[b < PK::NB ? b : 0][f][0];
+        v[f][1] = a[b < PK::NB ? b : 0][f][1];
+      } else {
+        v[f][0] = PK::TL == 2 && lc == 1 ? t[PK::TL == 2 ? 1 : 0][f] : t[0][f];
+        v[f][1] = 0.0;
+      }
+    }
+  }
+};
 
 }  // namespace apollo

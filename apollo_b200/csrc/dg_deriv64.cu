@@ -56,39 +56,34 @@ template <int EQ, int N> struct Deriv {
 template <int M, int N>
 __global__ void __launch_bounds__(128) k_adj_y(DgDev d, const double* __restrict__ w, double* __restrict__ y) {
   using PK = Pack64<N>;
-  constexpr int NP = PK::NP, NB = PK::NB, KS = PK::KS;
+  constexpr int NP = PK::NP;
   const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
   const int row = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 8 + lr;
   const int k = min(row, d.K - 1);
   const double* we = w + (size_t)k * NP * M;
   const double s = -d.geo[k].invJ;
-  double acc[NB][M][2];
+  Nodes<M, PK> acc;
+  acc.zero();
 #pragma unroll
-  for (int b = 0; b < NB; ++b)
-#pragma unroll
-    for (int f = 0; f < M; ++f) acc[b][f][0] = acc[b][f][1] = 0.0;
-#pragma unroll
-  for (int ks = 0; ks < KS; ++ks) {
+  for (int ks = 0; ks < PK::KS; ++ks) {
     const int node = min(PK::node(ks, lc), NP - 1);  // past the last node the operator is zero
     double q[M];
 #pragma unroll
     for (int f = 0; f < M; ++f) q[f] = we[node * M + f];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      const double op = __ldg(d.pack64 + PK::Y_OFF + (ks * NB + b) * 32 + lane);
-#pragma unroll
-      for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], q[f], op);
-    }
+    acc.add1(d.pack64 + PK::Y_OFF + ks * PK::NS, lane, q);
   }
+  acc.finish();
   if (row >= d.K) return;
 #pragma unroll
-  for (int b = 0; b < NB; ++b) {
+  for (int b = 0; b < PK::NBT; ++b) {
+    double v[M][2];
+    acc.get(b, lc, v);
 #pragma unroll
     for (int f = 0; f < M; ++f) {
-      acc[b][f][0] *= s;
-      acc[b][f][1] *= s;
+      v[f][0] *= s;
+      v[f][1] *= s;
     }
-    store_block<M, PK>(y + (size_t)k * NP * M, b, lc, acc[b]);
+    store_block<M, PK>(y + (size_t)k * NP * M, b, lc, v);
   }
 }
 
@@ -117,7 +112,7 @@ __device__ __forceinline__ void copy_face_nodes(double* dst, const double* __res
 template <int EQ, int N> struct Warp {
   using T = Deriv<EQ, N>;
   using PK = Pack64<N>;
-  static constexpr int M = T::M, NP = T::NP, NB = PK::NB;
+  static constexpr int M = T::M, NP = T::NP;
   int lane, lr, lc;
   double *sGz, *sA, *sB, *sPA, *sPB, *sG;
   int* sFm;
@@ -180,18 +175,6 @@ template <int EQ, int N> struct Warp {
 #pragma unroll
     for (int f = 0; f < M; ++f) out[f] -= base[f];
   }
-  // acc += the contraction of a block's two points per lane with ops [block][NB][32][2]
-  __device__ __forceinline__ void contract(double (*acc)[M][2], const double* ops, int block,
-                                           const double (*A)[M]) const {
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      const double2 w = reinterpret_cast<const double2*>(ops)[(block * NB + b) * 32 + lane];
-#pragma unroll
-      for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], A[0][f], w.x);
-#pragma unroll
-      for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], A[1][f], w.y);
-    }
-  }
   // V q at block pb's two points of this lane
   __device__ __forceinline__ void to_points(const double* sV, int pb, const double* e, double (*q)[M]) const {
     double v[M][2];
@@ -220,7 +203,7 @@ template <int EQ, int N>
 __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(DgDev d, AdjArgs a, const double* __restrict__ y) {
   using T = Deriv<EQ, N>;
   using PK = Pack64<N>;
-  constexpr int M = T::M, NP = T::NP, NG = T::NG, NF = T::NF, KS = PK::KS, NB = PK::NB;
+  constexpr int M = T::M, NP = T::NP, NG = T::NG, NF = T::NF, KS = PK::KS;
   extern __shared__ __align__(16) double smem[];
   // operators: WT | Z, or E | V | DT | VT | ET
   double *sE = smem, *sV = sE + PK::E_SIZE, *sDT = sV + PK::V_SIZE, *sVT = sDT + PK::DT_SIZE, *sET = sVT + PK::VT_SIZE;
@@ -247,17 +230,14 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
   const int ntiles = (d.K + 7) / 8;
   for (int tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; tile < ntiles; tile += gridDim.x * (blockDim.x >> 5)) {
     const int ke = min(tile * 8 + lr, d.K - 1);
-    double wv[NB][M][2];
+    double wv[PK::NBT][M][2];
 #pragma unroll
-    for (int b = 0; b < NB; ++b) load_block<M, PK>(a.wbar + (size_t)ke * NP * M, b, lc, wv[b]);
+    for (int b = 0; b < PK::NBT; ++b) load_block<M, PK>(a.wbar + (size_t)ke * NP * M, b, lc, wv[b]);
     W.load(d, tile, a.x, y);
     const double *ge = W.sG + kGeoStride * lr, *xe = W.sA + lr * T::ES, *ye = W.sB + lr * T::ES;
     const double rx = ge[0], ry = ge[1], sx = ge[2], sy = ge[3];
-    double acc[NB][M][2];
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-      for (int f = 0; f < M; ++f) acc[b][f][0] = acc[b][f][1] = 0.0;
+    Nodes<M, PK> acc;
+    acc.zero();
     if constexpr (T::LIN) {
 #pragma unroll
       for (int k = 0; k < KS; ++k) {
@@ -266,14 +246,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
         for (int f = 0; f < M; ++f) w[f] = wv[k / 2][f][k % 2];
         LinearFast64<EQ>::along_t(d.eqp, w, rx, ry, u);
         LinearFast64<EQ>::along_t(d.eqp, w, sx, sy, z);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          const double2 op = reinterpret_cast<const double2*>(sWT)[(k * NB + b) * 32 + lane];
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], u[f], op.x);
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], z[f], op.y);
-        }
+        acc.add(sWT + k * PK::NS, lane, u, z);
       }
       // at the face nodes: sJ (y_own - y_partner) through the flux Jacobian
 #pragma unroll 1
@@ -301,7 +274,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
 #pragma unroll
           for (int f = 0; f < M; ++f) A[j][f] += t[f];
         }
-        W.contract(acc, sZ, qb, A);
+        acc.add(sZ + (qb) * PK::NS, lane, A[0], A[1]);
       }
     } else {
       using X = EulerFast64<M>;
@@ -340,7 +313,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
             EulerAdj<M>::dir(d.eqp, q[j], sx, sy, aS[j], g[j], &err);
           }
         }
-        W.contract(acc, sVT, pb, g);
+        acc.add(sVT + (pb) * PK::NS, lane, g[0], g[1]);
       }
 #pragma unroll 1
       for (int fb = 0; fb < PK::FB; ++fb) {
@@ -392,19 +365,21 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
             for (int f = 0; f < M; ++f) A[j][f] += ab[f];
           }
         }
-        W.contract(acc, sET, fb, A);
+        acc.add(sET + (fb) * PK::NS, lane, A[0], A[1]);
       }
     }
+    acc.finish();
     if (tile * 8 + lr < d.K) {
       const size_t off = (size_t)ke * NP * M;
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
+      for (int b = 0; b < PK::NBT; ++b) {
         double o[M][2];
+        acc.get(b, lc, o);
 #pragma unroll
         for (int f = 0; f < M; ++f)
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            o[f][j] = a.beta * acc[b][f][j];
+            o[f][j] *= a.beta;
             if (a.alpha != 0.0) o[f][j] += a.alpha * wv[b][f][j];
           }
         if (a.z) {
@@ -426,7 +401,7 @@ template <int EQ, int N>
 __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(DgDev d, TanArgs a) {
   using T = Deriv<EQ, N>;
   using PK = Pack64<N>;
-  constexpr int M = T::M, NP = T::NP, NG = T::NG, NF = T::NF, KS = PK::KS, NB = PK::NB;
+  constexpr int M = T::M, NP = T::NP, NG = T::NG, NF = T::NF, KS = PK::KS;
   extern __shared__ __align__(16) double smem[];
   for (int i = 2 * threadIdx.x; i < T::TAN_OPS; i += 2 * blockDim.x)
     cp_async16(smem + i, d.pack64 + (T::LIN ? PK::Q_OFF : PK::E_OFF) + i);
@@ -442,11 +417,8 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
     W.load(d, tile, a.x, a.dx);
     const double *ge = W.sG + kGeoStride * lr, *xe = W.sA + lr * T::ES, *de = W.sB + lr * T::ES;
     const double rx = ge[0], ry = ge[1], sx = ge[2], sy = ge[3], miJ = -0.5 * ge[5];
-    double acc[NB][M][2];
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-      for (int f = 0; f < M; ++f) acc[b][f][0] = acc[b][f][1] = 0.0;
+    Nodes<M, PK> acc;
+    acc.zero();
     if constexpr (T::LIN) {
       const double *sQ = smem, *sW = smem + PK::Q_SIZE;
 #pragma unroll
@@ -457,14 +429,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
         for (int f = 0; f < M; ++f) q[f] = de[node * M + f];
         LinearFast64<EQ>::along(d.eqp, q, rx, ry, R);
         LinearFast64<EQ>::along(d.eqp, q, sx, sy, S);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          const double2 op = reinterpret_cast<const double2*>(sW)[(k * NB + b) * 32 + lane];
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], R[f], op.x);
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], S[f], op.y);
-        }
+        acc.add(sW + k * PK::NS, lane, R, S);
       }
 #pragma unroll 1
       for (int qb = 0; qb < PK::QB; ++qb) {
@@ -483,7 +448,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
           if (cn.y < 0) W.hook_linear(d, ke, -cn.x, fc, 0.0, a.t, qM, qP);
           LinearFast64<EQ>::face2(d.eqp, ge[6 + fc], ge[9 + fc], miJ * ge[12 + fc], qM, qP, A[j]);
         }
-        W.contract(acc, sQ, qb, A);
+        acc.add(sQ + (qb) * PK::NS, lane, A[0], A[1]);
       }
     } else {
       using X = EulerFast64<M>;
@@ -517,8 +482,8 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
             }
           }
         }
-        W.contract(acc, sD, pb * 2, R);
-        W.contract(acc, sD, pb * 2 + 1, S);
+        acc.add(sD + (pb * 2) * PK::NS, lane, R[0], R[1]);
+        acc.add(sD + (pb * 2 + 1) * PK::NS, lane, S[0], S[1]);
       }
 #pragma unroll 1
       for (int fb = 0; fb < PK::FB; ++fb) {
@@ -573,15 +538,18 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
             for (int f = 0; f < M; ++f) A[j][f] = 2.0 * w * nf[f].d[0];
           }
         }
-        W.contract(acc, sL, fb, A);
+        acc.add(sL + (fb) * PK::NS, lane, A[0], A[1]);
       }
     }
     // the stage update's tangent
+    acc.finish();
     if (tile * 8 + lr < d.K) {
       const size_t off = (size_t)ke * NP * M;
       const double c_r = a.mode == MODE_STAGE ? a.dt / 4.0 : a.dt / 5.0;
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
+      for (int b = 0; b < PK::NBT; ++b) {
+        double o[M][2];
+        acc.get(b, lc, o);
         if (a.mode != MODE_RHS) {
           double x[M][2];
           load_block<M, PK>(de, b, lc, x);
@@ -589,18 +557,17 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
 #pragma unroll
             for (int f = 0; f < M; ++f)
 #pragma unroll
-              for (int j = 0; j < 2; ++j) acc[b][f][j] = x[f][j] + c_r * acc[b][f][j];
+              for (int j = 0; j < 2; ++j) o[f][j] = x[f][j] + c_r * o[f][j];
           } else {
             double u[M][2];
             load_block<M, PK>(a.du0 + off, b, lc, u);
 #pragma unroll
             for (int f = 0; f < M; ++f)
 #pragma unroll
-              for (int j = 0; j < 2; ++j)
-                acc[b][f][j] = (4.0 / 5.0) * x[f][j] + c_r * acc[b][f][j] + (1.0 / 5.0) * u[f][j];
+              for (int j = 0; j < 2; ++j) o[f][j] = (4.0 / 5.0) * x[f][j] + c_r * o[f][j] + (1.0 / 5.0) * u[f][j];
           }
         }
-        store_block<M, PK>(a.dout + off, b, lc, acc[b]);
+        store_block<M, PK>(a.dout + off, b, lc, o);
       }
     }
   }

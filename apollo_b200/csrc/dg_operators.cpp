@@ -264,62 +264,56 @@ template <int N> std::vector<double> pack64_t(const RefOps& o) {
       for (int j = 0; j < NP; ++j) acc += o.VVT(n, j) * o.Vc(c, j);
       vs[(size_t)n * NC + c] = acc * o.cub_w[c];
     }
-  for (int lane = 0; lane < 32; ++lane) {
-    const int k = lane % 4, n = lane / 4;
-    for (int b = 0; b < P::NB; ++b) {
-      const int node = P::out_node(b, n);
-      if (node < 0) continue;
+  for (int node = 0; node < NP; ++node)
+    for (int k = 0; k < 4; ++k) {
+      auto at = [&](int off, int entry, int op) -> double& { return out[off + entry * P::NS + P::place(node, k, op)]; };
       for (int j = 0; j < 2; ++j) {
         for (int fb = 0; fb < P::FB; ++fb) {
           const int p = 8 * fb + 2 * k + j;
-          if (p < NF) out[P::L_OFF + ((fb * P::NB + b) * 32 + lane) * 2 + j] = o.Lift(node, p) * o.gw[p % NG];
+          if (p >= NF) continue;
+          at(P::L_OFF, fb, j) = o.Lift(node, p) * o.gw[p % NG];
+          // the adjoint's face contributions reach the nodes of the face only
+          for (int m = 0; m <= N; ++m)
+            if (P::face_node(p / NG, m) == node) at(P::ET_OFF, fb, j) = o.gw[p % NG] * edge(p % NG, m);
         }
         for (int qb = 0; qb < P::QB; ++qb) {
           const int p = 8 * qb + 2 * k + j;
           if (p >= P::NFN) continue;
-          double acc = 0.0;
-          for (int g = 0; g < NG; ++g) acc += o.Lift(node, p / (N + 1) * NG + g) * o.gw[g] * edge(g, p % (N + 1));
-          out[P::Q_OFF + ((qb * P::NB + b) * 32 + lane) * 2 + j] = acc;
+          const int face = p / (N + 1), m0 = p % (N + 1);
+          double q = 0.0;
+          for (int g = 0; g < NG; ++g) q += o.Lift(node, face * NG + g) * o.gw[g] * edge(g, m0);
+          at(P::Q_OFF, qb, j) = q;
+          for (int m = 0; m <= N; ++m)
+            if (P::face_node(face, m) == node) {
+              double z = 0.0;
+              for (int g = 0; g < NG; ++g) z += edge(g, m) * o.gw[g] * edge(g, m0);
+              at(P::Z_OFF, qb, j) = z;
+            }
         }
         for (int pb = 0; pb < P::PB; ++pb) {
           const int c = 8 * pb + 2 * k + j;
           if (c >= NC) continue;
-          out[P::D_OFF + (((pb * 2 + 0) * P::NB + b) * 32 + lane) * 2 + j] = o.DrW(node, c);
-          out[P::D_OFF + (((pb * 2 + 1) * P::NB + b) * 32 + lane) * 2 + j] = o.DsW(node, c);
-          out[P::S_OFF + ((pb * P::NB + b) * 32 + lane) * 2 + j] = vs[(size_t)node * NC + c];
-          out[P::VT_OFF + ((pb * P::NB + b) * 32 + lane) * 2 + j] = o.Vc(c, node);
-        }
-        // the adjoint's face contributions reach the nodes of the face only
-        for (int fb = 0; fb < P::FB; ++fb) {
-          const int p = 8 * fb + 2 * k + j;
-          for (int m = 0; m <= N && p < NF; ++m)
-            if (P::face_node(p / NG, m) == node)
-              out[P::ET_OFF + ((fb * P::NB + b) * 32 + lane) * 2 + j] = o.gw[p % NG] * edge(p % NG, m);
-        }
-        for (int qb = 0; qb < P::QB; ++qb) {
-          const int p = 8 * qb + 2 * k + j;
-          for (int m = 0; m <= N && p < P::NFN; ++m)
-            if (P::face_node(p / (N + 1), m) == node) {
-              double acc = 0.0;
-              for (int g = 0; g < NG; ++g) acc += edge(g, m) * o.gw[g] * edge(g, p % (N + 1));
-              out[P::Z_OFF + ((qb * P::NB + b) * 32 + lane) * 2 + j] = acc;
-            }
+          at(P::D_OFF, 2 * pb, j) = o.DrW(node, c);
+          at(P::D_OFF, 2 * pb + 1, j) = o.DsW(node, c);
+          at(P::S_OFF, pb, j) = vs[(size_t)node * NC + c];
+          at(P::VT_OFF, pb, j) = o.Vc(c, node);
         }
       }
       for (int ks = 0; ks < P::KS; ++ks) {
         const int from = P::node(ks, k);
         if (from >= NP) continue;
-        out[P::W_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 0] = W1(node, from);
-        out[P::W_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 1] = W2(node, from);
-        out[P::WT_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 0] = W1(from, node);
-        out[P::WT_OFF + ((ks * P::NB + b) * 32 + lane) * 2 + 1] = W2(from, node);
-        out[P::Y_OFF + (ks * P::NB + b) * 32 + lane] = o.VVT(node, from);
+        at(P::W_OFF, ks, 0) = W1(node, from);
+        at(P::W_OFF, ks, 1) = W2(node, from);
+        at(P::WT_OFF, ks, 0) = W1(from, node);
+        at(P::WT_OFF, ks, 1) = W2(from, node);
+        at(P::Y_OFF, ks, 0) = o.VVT(node, from);
       }
     }
+  for (int lane = 0; lane < 32; ++lane)
     for (int pb = 0; pb < P::PB; ++pb) {
-      const int c = std::min(8 * pb + n, NC - 1);  // a column past the last point repeats it
+      const int n = lane / 4, c = std::min(8 * pb + n, NC - 1);  // a column past the last point repeats it
       for (int ks = 0; ks < P::KS; ++ks) {
-        const int from = P::node(ks, k);
+        const int from = P::node(ks, lane % 4);
         if (from >= NP) continue;
         out[P::V_OFF + ((pb * ((P::KS + 1) / 2) + ks / 2) * 32 + lane) * 2 + ks % 2] = o.Vc(c, from);
         if (8 * pb + n >= NC) continue;
@@ -327,7 +321,6 @@ template <int N> std::vector<double> pack64_t(const RefOps& o) {
         out[P::DT_OFF + ((pb * P::KS + ks) * 32 + lane) * 2 + 1] = o.DsW(from, c);
       }
     }
-  }
   for (int fb = 0; fb < P::FB; ++fb)
     for (int m = 0; m <= N; ++m)
       for (int c = 0; c < 4; ++c)

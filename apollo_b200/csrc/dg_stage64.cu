@@ -48,7 +48,6 @@ template <int EQ, int N> struct Chain {
   static constexpr int NP = Sizes<N>::NP, NC = Sizes<N>::NC, NG = Sizes<N>::NG, NF = Sizes<N>::NF;
   static constexpr bool LIN = kLinearEq<EQ>;
   using P = Pack64<N>;
-  static constexpr int KS = P::KS, NB = P::NB, PB = P::PB, FB = P::FB;
   // operators in shared memory: E | L | V | D, or Q | W
   static constexpr int OPS_OFF = LIN ? P::Q_OFF : P::E_OFF, OPS = LIN ? P::S_OFF - P::Q_OFF : P::Q_OFF;
   static constexpr int TAB = NG;                     // gz
@@ -83,7 +82,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   using PK = Pack64<N>;
   using P = Eq<EQ>;
   constexpr int M = T::M, NP = T::NP, NG = T::NG, NF = T::NF;
-  constexpr int KS = T::KS, NB = T::NB, PB = T::PB, FB = T::FB, NFN = PK::NFN;
+  constexpr int KS = PK::KS, PB = PK::PB, FB = PK::FB, NFN = PK::NFN;
   extern __shared__ __align__(16) double smem[];
   double* sOps = smem;
   double* sGz = smem + T::OPS;
@@ -184,11 +183,8 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     cp_async_commit();
     double* xe = sX + lr * T::ES;
     const double* ge = sX + T::X + kGeoStride * lr;
-    double acc[NB][M][2];
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-      for (int f = 0; f < M; ++f) acc[b][f][0] = acc[b][f][1] = 0.0;
+    Nodes<M, PK> acc;
+    acc.zero();
 
     // ---- volume term
     const double rx = ge[0], ry = ge[1], sx = ge[2], sy = ge[3];
@@ -201,14 +197,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
         for (int f = 0; f < M; ++f) q[f] = xe[node * M + f];
         LinearFast64<EQ>::along(d.eqp, q, rx, ry, R);
         LinearFast64<EQ>::along(d.eqp, q, sx, sy, S);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          const double2 w = reinterpret_cast<const double2*>(sOps + PK::Q_SIZE)[(k * NB + b) * 32 + lane];
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], R[f], w.x);
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], S[f], w.y);
-        }
+        acc.add(sOps + PK::Q_SIZE + k * PK::NS, lane, R, S);
       }
     } else {
       const double *sV = sOps + PK::V_OFF, *sD = sOps + PK::D_OFF;
@@ -242,19 +231,8 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
           qc[1][f] = v[f][1];
         }
         volume_flux_pair<EQ>(d.eqp, qc, rx, ry, sx, sy, R, S, &err);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          const double2 wr = reinterpret_cast<const double2*>(sD)[((pb * 2 + 0) * NB + b) * 32 + lane];
-          const double2 ws = reinterpret_cast<const double2*>(sD)[((pb * 2 + 1) * NB + b) * 32 + lane];
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], R[0][f], wr.x);
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], R[1][f], wr.y);
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], S[0][f], ws.x);
-#pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], S[1][f], ws.y);
-        }
+        acc.add(sD + (2 * pb) * PK::NS, lane, R[0], R[1]);
+        acc.add(sD + (2 * pb + 1) * PK::NS, lane, S[0], S[1]);
       }
     }
     const int inst = inst_of(d, ke);
@@ -278,16 +256,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
           for (int f = 0; f < M; ++f) s[j][f] = 0.0;
           source_terms<M>(d.src, t, x, y, s[j]);
         }
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          const double2 w = __ldg(reinterpret_cast<const double2*>(d.pack64 + PK::S_OFF) + (pb * NB + b) * 32 + lane);
-#pragma unroll
-          for (int f = 0; f < M; ++f)
-            if (fields & (1u << f)) {
-              dmma_8x8x4(acc[b][f], s[0][f], w.x);
-              dmma_8x8x4(acc[b][f], s[1][f], w.y);
-            }
-        }
+        acc.add(d.pack64 + PK::S_OFF + pb * PK::NS, lane, s[0], s[1], fields);
       }
     }
 
@@ -305,16 +274,6 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
       const double x = 0.5 * (-g.vx[0] * (r + s) + g.vx[1] * (1. + r) + g.vx[2] * (1. + s));
       const double y = 0.5 * (-g.vy[0] * (r + s) + g.vy[1] * (1. + r) + g.vy[2] * (1. + s));
       apply_bc<EQ, double>(d.bcs, tag, t, x, y, ge[6 + fc], ge[9 + fc], q, qb);
-    };
-    auto lift = [&](const double* ops, int block, const double (*A)[M]) {
-#pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        const double2 w = reinterpret_cast<const double2*>(ops)[(block * NB + b) * 32 + lane];
-#pragma unroll
-        for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], A[0][f], w.x);
-#pragma unroll
-        for (int f = 0; f < M; ++f) dmma_8x8x4(acc[b][f], A[1][f], w.y);
-      }
     };
     if constexpr (T::LIN) {
       // the flux at the face nodes, two per lane (a node past the last repeats
@@ -338,7 +297,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
           const double lam = LinearFast64<EQ>::face2(d.eqp, ge[6 + fc], ge[9 + fc], miJ * ge[12 + fc], qM, qP, A[j]);
           if (want_lam) lam_acc.add(d.st, inst, lam);
         }
-        lift(sOps, qb, A);
+        acc.add(sOps + qb * PK::NS, lane, A[0], A[1]);
       }
     } else {
       const double* sL = sOps + PK::L_OFF;
@@ -377,7 +336,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
           lam_acc.add(d.st, inst, fabs(lam[0]));
           lam_acc.add(d.st, inst, fabs(lam[1]));
         }
-        lift(sL, fb, A);
+        acc.add(sL + fb * PK::NS, lane, A[0], A[1]);
       }
     }
 
@@ -387,6 +346,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
     // a full tile's results replace its states in shared memory and leave by
     // bulk copies; rows of a partial tile or of a list, and short rows, are
     // stored from here
+    acc.finish();
     const bool whole = T::BULK && list == nullptr && tile * 8 + 8 <= n;
     if (whole) __syncwarp();  // the states have been read
     if (row_ok) {
@@ -394,15 +354,14 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
       const double* u0 = a.u0 + (size_t)ke * NP * M;
       int top = 0;  // the largest exponent and leading fraction: above infinity's, a NaN
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
+      for (int b = 0; b < PK::NBT; ++b) {
         double o[M][2];
+        acc.get(b, lc, o);
 #pragma unroll
-        for (int f = 0; f < M; ++f)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            o[f][j] = acc[b][f][j];
-            top = max(top, __double2hiint(o[f][j]) & 0x7fffffff);
-          }
+        for (int f = 0; f < M; ++f) {
+          top = max(top, __double2hiint(o[f][0]) & 0x7fffffff);
+          top = max(top, __double2hiint(o[f][1]) & 0x7fffffff);
+        }
         if (a.mode != MODE_RHS) {
           double x[M][2];
           load_block<M, PK>(xe, b, lc, x);
