@@ -37,6 +37,27 @@ template <int n> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(n) : "memory");
 }
 
+// Overlap with the kernel before in the stream (programmatic dependent launch):
+// a kernel launched with `overlap` may start while that one still runs, does
+// what depends on none of its results (operators, connectivity), and waits for
+// its completion here; allow_next lets the kernel after start in the same way.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+template <class... P, class... A>
+cudaError_t launch_kernel(void (*k)(P...), int grid, int threads, size_t smem, cudaStream_t s, bool overlap, A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&c, k, args...);
+}
+
 // Row strides (doubles) of a tile in shared memory, padded so that the lanes of
 // one access phase (two rows of four lanes for 16 bytes, four rows for 8) fall
 // on different banks: a whole element's nodes (per = NP M; an odd count is
@@ -56,13 +77,19 @@ constexpr int kGeoStride = 18;
 template <int per, int stride>
 __device__ __forceinline__ void copy_tile(double* dst, const double* __restrict__ src, int tile, int n, int lane) {
   if (tile * 8 + 8 <= n) {
-    const double* s = src + (size_t)tile * 8 * per;
-    if constexpr (per == stride) {
-#pragma unroll 4
-      for (int i = lane; i < 4 * per; i += 32) cp_async16(dst + 2 * i, s + 2 * i);
-    } else {
-#pragma unroll 4
-      for (int i = lane; i < 4 * per; i += 32) cp_async16(dst + 2 * i + i / (per / 2) * (stride - per), s + 2 * i);
+    const double* s = src + (size_t)tile * 8 * per + 2 * lane;
+    double* t = dst + 2 * lane;
+    if constexpr (per % 2) {  // not padded: 4 per pieces of 16 bytes in a row
+#pragma unroll
+      for (int u = 0; u < (4 * per + 31) / 32; ++u)
+        if (u < 4 * per / 32 || 32 * u + lane < 4 * per) cp_async16(t + 64 * u, s + 64 * u);
+    } else {  // row by row, so that every address is the lane's plus a constant
+#pragma unroll
+      for (int u = 0; u < (per / 2 + 31) / 32; ++u)
+        if (u < per / 64 || 32 * u + lane < per / 2) {
+#pragma unroll
+          for (int r = 0; r < 8; ++r) cp_async16(t + r * stride + 64 * u, s + r * per + 64 * u);
+        }
     }
   } else {
     for (int i = lane; i < 8 * per; i += 32) {
@@ -128,6 +155,20 @@ __device__ __forceinline__ void store_run(double* __restrict__ p, const double* 
   } else {
 #pragma unroll
     for (int i = 0; i < n; ++i) p[i] = v[i];
+  }
+}
+
+// n consecutive doubles of shared memory, read here and not kept in registers
+// from an earlier read
+template <int n> __device__ __forceinline__ void shared_run(const double* p, double* v) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  if constexpr (n % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < n; i += 2)
+      asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];\n" : "=d"(v[i]), "=d"(v[i + 1]) : "r"(a + 8 * i));
+  } else {
+#pragma unroll
+    for (int i = 0; i < n; ++i) asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v[i]) : "r"(a + 8 * i));
   }
 }
 

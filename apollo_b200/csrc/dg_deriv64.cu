@@ -60,6 +60,8 @@ __global__ void __launch_bounds__(128) k_adj_y(DgDev d, const double* __restrict
   const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
   const int row = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 8 + lr;
   const int k = min(row, d.K - 1);
+  allow_next();
+  wait_previous();
   const double* we = w + (size_t)k * NP * M;
   const double s = -d.geo[k].invJ;
   Nodes<M, PK> acc;
@@ -179,13 +181,14 @@ template <int EQ, int N> struct Warp {
   __device__ __forceinline__ void to_points(const double* sV, int pb, const double* e, double (*q)[M]) const {
     double v[M][2];
 #pragma unroll
-    for (int f = 0; f < M; ++f) v[f][0] = v[f][1] = 0.0;
-#pragma unroll
     for (int k = 0; k < PK::KS; k += 2) {
       const double2 w = reinterpret_cast<const double2*>(sV)[(pb * ((PK::KS + 1) / 2) + k / 2) * 32 + lane];
       const int n0 = min(PK::node(k, lc), NP - 1), n1 = min(PK::node(k + 1, lc), NP - 1);
 #pragma unroll
-      for (int f = 0; f < M; ++f) dmma_8x8x4(v[f], e[n0 * M + f], w.x);
+      for (int f = 0; f < M; ++f) {
+        if (k == 0) dmma_8x8x4_first(v[f], e[n0 * M + f], w.x);
+        else dmma_8x8x4(v[f], e[n0 * M + f], w.x);
+      }
       if (k + 1 < PK::KS) {
 #pragma unroll
         for (int f = 0; f < M; ++f) dmma_8x8x4(v[f], e[n1 * M + f], w.y);
@@ -223,8 +226,10 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
   }
   Warp<EQ, N> W;
   W.init(d, smem, T::ADJ_OPS);
+  allow_next();
   cp_async_wait_all();
   __syncthreads();
+  wait_previous();
   const int lane = W.lane, lr = W.lr, lc = W.lc;
   int err = 0;  // the float64 forward reports non-physical states
   const int ntiles = (d.K + 7) / 8;
@@ -283,14 +288,18 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
         double q[2][M], r[M][2], s[M][2], g[2][M];
         W.to_points(sV, pb, xe, q);
 #pragma unroll
-        for (int f = 0; f < M; ++f) r[f][0] = r[f][1] = s[f][0] = s[f][1] = 0.0;
-#pragma unroll
         for (int k = 0; k < KS; ++k) {
           const double2 op = reinterpret_cast<const double2*>(sDT)[(pb * KS + k) * 32 + lane];
 #pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(r[f], wv[k / 2][f][k % 2], op.x);
+          for (int f = 0; f < M; ++f) {
+            if (k == 0) dmma_8x8x4_first(r[f], wv[0][f][0], op.x);
+            else dmma_8x8x4(r[f], wv[k / 2][f][k % 2], op.x);
+          }
 #pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(s[f], wv[k / 2][f][k % 2], op.y);
+          for (int f = 0; f < M; ++f) {
+            if (k == 0) dmma_8x8x4_first(s[f], wv[0][f][0], op.y);
+            else dmma_8x8x4(s[f], wv[k / 2][f][k % 2], op.y);
+          }
         }
         double aR[2][M], aS[2][M];
 #pragma unroll
@@ -407,8 +416,10 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
     cp_async16(smem + i, d.pack64 + (T::LIN ? PK::Q_OFF : PK::E_OFF) + i);
   Warp<EQ, N> W;
   W.init(d, smem, T::TAN_OPS);
+  allow_next();
   cp_async_wait_all();
   __syncthreads();
+  wait_previous();
   const int lane = W.lane, lr = W.lr, lc = W.lc;
   int err = 0;  // the float64 forward reports non-physical states
   const int ntiles = (d.K + 7) / 8;
@@ -598,11 +609,11 @@ cudaError_t adjoint_t(const DgDev& d, const AdjArgs& a, cudaStream_t s) {
   static unsigned configured = 0;
   cudaError_t e = allow_smem(k_adjoint64<EQ, N>, T::bytes(T::ADJ_OPS, T::ADJ_WARPS), configured);
   if (e != cudaSuccess) return e;
-  k_adj_y<T::M, N><<<(d.K + 31) / 32, 128, 0, s>>>(d, a.wbar, a.sbar);
+  e = launch_kernel(k_adj_y<T::M, N>, (d.K + 31) / 32, 128, 0, s, false, d, a.wbar, a.sbar);
+  if (e != cudaSuccess) return e;
   int grid, warps;
   shape(d.K, T::ADJ_WARPS, &grid, &warps);
-  k_adjoint64<EQ, N><<<grid, 32 * warps, T::bytes(T::ADJ_OPS, warps), s>>>(d, a, a.sbar);
-  return cudaGetLastError();
+  return launch_kernel(k_adjoint64<EQ, N>, grid, 32 * warps, T::bytes(T::ADJ_OPS, warps), s, true, d, a, a.sbar);
 }
 
 template <int EQ, int N>
@@ -613,8 +624,7 @@ cudaError_t tangent_t(const DgDev& d, const TanArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   int grid, warps;
   shape(d.K, T::TAN_WARPS, &grid, &warps);
-  k_tangent64<EQ, N><<<grid, 32 * warps, T::bytes(T::TAN_OPS, warps), s>>>(d, a);
-  return cudaGetLastError();
+  return launch_kernel(k_tangent64<EQ, N>, grid, 32 * warps, T::bytes(T::TAN_OPS, warps), s, false, d, a);
 }
 
 template <int EQ>

@@ -146,6 +146,8 @@ struct StageArgs {
   double t_arg;
   double dt_arg;        // dt used when time_from_state == 0
   int reset_lambda;     // volume kernel zeroes st->lam_bits first
+  int overlap;          // fused float64 stage: the kernel before in the stream is one of the same step, and this
+                        // one may start while it runs (it waits for it before it reads any of its results)
   // mixed precision only: fp32 face traces [K][3][NG M, padded] of x (tr_in) and of
   // the stage result (tr_out, nullptr: not needed); for MODE_RHS the launcher
   // first computes the traces of x into tr_scratch and reads them from there
@@ -178,7 +180,8 @@ int device_sms();                                // SMs of the current device
 // k_lift alone on d.vol / d.flux (used by the tangent of a stage)
 cudaError_t launch_lift_fp64(int eq, const DgDev& d, const StageArgs& a, cudaStream_t s);
 cudaError_t launch_init_speed(int eq, const DgDev& d, const double* u, cudaStream_t s);
-cudaError_t launch_finalize(const DgDev& d, cudaStream_t s);
+// overlap: as StageArgs::overlap
+cudaError_t launch_finalize(const DgDev& d, cudaStream_t s, bool overlap = false);
 // st[i].lam_bits = 0 for every instance
 cudaError_t launch_reset_lambda(const DgDev& d, cudaStream_t s);
 // *st = v on the stream (no host staging buffer to race with later calls)

@@ -16,6 +16,13 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
+// the first step of a sum: C = A B
+__device__ __forceinline__ void dmma_8x8x4_first(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};\n"
+               : "=d"(c[0]), "=d"(c[1])
+               : "d"(a), "d"(b), "d"(0.0));
+}
+
 constexpr int round_up(int x, int m) { return (x + m - 1) / m * m; }
 // leading dimension (in doubles) of a shared-memory tile read by fragments:
 // rows 4 apart must land 8 banks apart, i.e. ld = 4 (mod 16)

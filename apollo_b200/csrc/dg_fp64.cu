@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dg_chain64.cuh"
 #include "dg_device.cuh"
 #include "dg_dmma.cuh"
 #include "dg_flux64.cuh"
@@ -330,6 +331,7 @@ __global__ void k_init_speed(DgDev d, const double* u, int nnodes) {
 // to the end time (ApSolver::ComputeRHSforTS + MonitorVTK,
 // src/solvers/apsolver.cc:421-480).
 __global__ void k_finalize(DgDev d) {
+  wait_previous();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.ninst) return;
   DevState* st = d.st + i;
@@ -661,9 +663,8 @@ __global__ void k_reset_lambda(DevState* st, int n) {
   if (i < n) st[i].lam_bits = 0ull;
 }
 
-cudaError_t launch_finalize(const DgDev& d, cudaStream_t s) {
-  k_finalize<<<(d.ninst + 127) / 128, 128, 0, s>>>(d);
-  return cudaGetLastError();
+cudaError_t launch_finalize(const DgDev& d, cudaStream_t s, bool overlap) {
+  return launch_kernel(k_finalize, (d.ninst + 127) / 128, 128, 0, s, overlap, d);
 }
 
 cudaError_t launch_reset_lambda(const DgDev& d, cudaStream_t s) {

@@ -339,11 +339,12 @@ apollo_status enqueue_step(apollo_dg* h, apollo_precision prec) {
         CK(mixed_launch_traces(h->mixed, d, lim, (float*)a.tr_in, h->stream), "trace launch");
       }
     }
+    a.overlap = i > 0 && !h->lim_on;
     apollo_status r = enqueue_stage(h, a, prec);
     if (r != APOLLO_OK) return r;
   }
   DgDev d = make_dev(h);
-  cudaError_t e = launch_finalize(d, h->stream);
+  cudaError_t e = launch_finalize(d, h->stream, prec != APOLLO_PREC_MIXED);
   if (e != cudaSuccess) return cuda_fail(h, e, "finalize launch");
   return APOLLO_OK;
 }
@@ -1145,6 +1146,7 @@ apollo_status fixed_stage(apollo_dg* h, int s, const double* x, const double* u0
   a.t_arg = stage_time(s, tn, dt);
   a.dt_arg = dt;
   a.reset_lambda = 0;
+  a.overlap = s > 0;
   DgDev d = make_dev(h);
   cudaError_t e = launch_rhs_fp64(h->eq, d, a, h->stream);
   if (e != cudaSuccess) return cuda_fail(h, e, "stage launch");

@@ -59,7 +59,7 @@ template <int EQ, int N> struct Chain {
   // [24] int2 and where the face nodes come from [24] int2
   static constexpr int ES = elem_stride(NP * M, M), FS = face_stride(3 * (N + 1) * M, M);
   static constexpr int X = 8 * ES, G = 8 * kGeoStride, PN = 8 * FS, C = 48;
-  static constexpr int XB = M == 8 ? 1 : 2;
+  static constexpr int XB = LIN && M != 8 || !LIN && N >= 5 ? 2 : 1;
   // results leave by bulk copies where a row is long enough to pay for one:
   // K = 130,050: Euler N = 4 (480 bytes a row) 209 -> 204 us, Maxwell TM N = 5
   // (one copy of 4,032) 105 -> 95; Euler N = 2 (192 bytes) 89 -> 93
@@ -68,7 +68,7 @@ template <int EQ, int N> struct Chain {
   static constexpr size_t bytes(int warps) { return sizeof(double) * (size_t)(SHARED + warps * WARP); }
   // warps per block (one block per SM): what the registers allow
   static constexpr int fit(int w) { return bytes(w) <= 227 * 1024 ? w : fit(w - 1); }
-    static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : (N >= 5 ? 8 : 12));
+    static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : (N >= 5 ? 8 : 16));
 };
 
 // One SSPRK stage (or right-hand side).  Reads the neighbours of x: x and out
@@ -94,11 +94,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   for (int i = 2 * tid; i < T::OPS; i += 2 * blockDim.x) cp_async16(sOps + i, d.pack64 + T::OPS_OFF + i);
   for (int i = tid; i < NG; i += blockDim.x) sGz[i] = d.gz[i];
   for (int i = tid; i < NFN; i += blockDim.x) sFm[i] = PK::face_node(i / (N + 1), i % (N + 1));
-  // the last stage of a step (and a lone right-hand side) reduces the wave
-  // speeds; an earlier stage clears the word instead
-  const bool want_lam = a.mode != MODE_STAGE;
-  if (a.mode == MODE_STAGE && a.reset_lambda && blockIdx.x == 0)
-    for (int i = tid; i < d.ninst; i += blockDim.x) d.st[i].lam_bits = 0ull;
+  allow_next();
   int err = 0;
   LamAcc lam_acc;
   const int n = list ? nlist : d.K;
@@ -135,8 +131,14 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
   int2 conn_next = make_int2(0, -1);
   if (tile < ntiles) {
     conn_next = load_conn(tile);
-    if (T::XB == 2) load_tile(tile, sX0);
   }
+  wait_previous();
+  // the last stage of a step (and a lone right-hand side) reduces the wave
+  // speeds; an earlier stage clears the word instead
+  const bool want_lam = a.mode != MODE_STAGE;
+  if (a.mode == MODE_STAGE && a.reset_lambda && blockIdx.x == 0)
+    for (int i = tid; i < d.ninst; i += blockDim.x) d.st[i].lam_bits = 0ull;
+  if (T::XB == 2 && tile < ntiles) load_tile(tile, sX0);
   cp_async_wait_all();
   __syncthreads();
   for (int it = 0; tile < ntiles; tile += stride, ++it) {
@@ -201,27 +203,24 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
       }
     } else {
       const double *sV = sOps + PK::V_OFF, *sD = sOps + PK::D_OFF;
-      double q[KS][M];
-#pragma unroll
-      for (int k = 0; k < KS; ++k) {
-        const int node = min(PK::node(k, lc), NP - 1);  // past the last node the operator is zero
-#pragma unroll
-        for (int f = 0; f < M; ++f) q[k][f] = xe[node * M + f];
-      }
 #pragma unroll 1
       for (int pb = 0; pb < PB; ++pb) {
         // the eight cubature points of the block, two per lane
         double v[M][2];
 #pragma unroll
-        for (int f = 0; f < M; ++f) v[f][0] = v[f][1] = 0.0;
-#pragma unroll
         for (int k = 0; k < KS; k += 2) {
           const double2 w = reinterpret_cast<const double2*>(sV)[(pb * ((KS + 1) / 2) + k / 2) * 32 + lane];
+          double q[2][M];
 #pragma unroll
-          for (int f = 0; f < M; ++f) dmma_8x8x4(v[f], q[k][f], w.x);
+          for (int j = 0; j < 2; ++j) shared_run<M>(xe + min(PK::node(k + j, lc), NP - 1) * M, q[j]);
+#pragma unroll
+          for (int f = 0; f < M; ++f) {
+            if (k == 0) dmma_8x8x4_first(v[f], q[0][f], w.x);
+            else dmma_8x8x4(v[f], q[0][f], w.x);
+          }
           if (k + 1 < KS) {
 #pragma unroll
-            for (int f = 0; f < M; ++f) dmma_8x8x4(v[f], q[k + 1][f], w.y);
+            for (int f = 0; f < M; ++f) dmma_8x8x4(v[f], q[1][f], w.y);
           }
         }
         double qc[2][M], R[2][M], S[2][M];
@@ -442,8 +441,7 @@ cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nl
   const int tiles = (n + 7) / 8, grid = tiles < sms ? tiles : sms;
   int warps = (tiles + grid - 1) / grid;
   if (warps > T::WMAX) warps = T::WMAX;
-  k_stage64<EQ, N, GF><<<grid, 32 * warps, T::bytes(warps), s>>>(d, a, list, nlist);
-  return cudaGetLastError();
+  return launch_kernel(k_stage64<EQ, N, GF>, grid, 32 * warps, T::bytes(warps), s, a.overlap != 0, d, a, list, nlist);
 }
 
 template <int EQ, bool GF>
