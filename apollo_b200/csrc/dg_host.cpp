@@ -344,7 +344,7 @@ apollo_status enqueue_step(apollo_dg* h, apollo_precision prec) {
     if (r != APOLLO_OK) return r;
   }
   DgDev d = make_dev(h);
-  cudaError_t e = launch_finalize(d, h->stream, prec != APOLLO_PREC_MIXED);
+  cudaError_t e = launch_finalize(d, h->stream, true);
   if (e != cudaSuccess) return cuda_fail(h, e, "finalize launch");
   return APOLLO_OK;
 }

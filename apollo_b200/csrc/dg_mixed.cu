@@ -25,6 +25,7 @@
 // Apollo: the RHS of wxnodaldg2dmethod.cc:235-542 (volume :346-380, traces and
 // partner gather :389-440, numerical flux :442-469, surface integral and M^-1/J
 // :472-504) fused with the TSSSP RK_2 stage update.
+#include "dg_chain64.cuh"
 #include "dg_mixed.h"
 #include "dg_umma.cuh"
 
@@ -360,6 +361,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
   const uint32_t wlim = d.wait_limit ? d.wait_limit : (1u << 22);
   auto xs_buf = [&](int i) { return (double*)(sm + C::O_XS + (C::XS2 ? (i & 1) * C::SZ_XS : 0)); };
 
+  allow_next();
   // ---- once per CTA: operators split into tf32 halves (K-major)
   for (int i = tid; i < C::NC16 * K1; i += kMixThreads) {
     const int r = i / K1, k = i % K1;
@@ -416,6 +418,7 @@ __global__ void __launch_bounds__(kMixThreads, 1)
     }
     *abort_flag = 0;
   }
+  wait_previous();  // the stage before has ended: its results and its tensor memory
   if (warp == 0) umma::tmem_alloc(umma::smem_u32(tslot), C::TCOLS);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   umma::fence_proxy_async();
@@ -1136,7 +1139,9 @@ cudaError_t launch_mixed_sh(MixedPlan* p, const DgDev& d, const StageArgs& a0, c
     int grid = sms;
     if (grid > ntiles) grid = ntiles;
     StageArgs a = a0;
-    if (a.reset_lambda && a.mode != MODE_STAGE) {
+    // a step's last stage finds the word clear: the stages before reduce
+    // nothing, and the step's start and the end of the one before cleared it
+    if (a.reset_lambda && a.mode == MODE_RHS) {
       cudaError_t e = launch_reset_lambda(d, s);
       if (e != cudaSuccess) return e;
     }
@@ -1158,12 +1163,13 @@ cudaError_t launch_mixed_sh(MixedPlan* p, const DgDev& d, const StageArgs& a0, c
     // bit 0: the state is bulk-copied (16-byte aligned); bit 1: warm L2 with u0
     const int flags = (((uintptr_t)a.x & 15) == 0 ? 1 : 0) |
                       (a.mode == MODE_FINAL && ((uintptr_t)a.u0 & 15) == 0 ? 2 : 0);
-    k_mixed_stage<EQ, N, SH, GF><<<grid, kMixThreads, C::BYTES, s>>>(d, a, p->rowsum, flags);
+    const cudaError_t e = launch_kernel(k_mixed_stage<EQ, N, SH, GF>, grid, kMixThreads, C::BYTES, s, a.overlap != 0, d,
+                                        a, (const double*)p->rowsum, flags);
     if (ev) {
       cudaEventRecord(ev[2], s);
       cudaEventRecord(ev[3], s);
     }
-    return cudaGetLastError();
+    return e;
   }
 }
 
@@ -1189,7 +1195,9 @@ cudaError_t launch_fused(MixedPlan* p, const DgDev& d, const StageArgs& a0, cuda
     int grid = sms;
     if (grid > ntiles) grid = ntiles;
     StageArgs a = a0;
-    if (a.reset_lambda && a.mode != MODE_STAGE) {
+    // a step's last stage finds the word clear: the stages before reduce
+    // nothing, and the step's start and the end of the one before cleared it
+    if (a.reset_lambda && a.mode == MODE_RHS) {
       cudaError_t e = launch_reset_lambda(d, s);
       if (e != cudaSuccess) return e;
     }
@@ -1211,12 +1219,13 @@ cudaError_t launch_fused(MixedPlan* p, const DgDev& d, const StageArgs& a0, cuda
     if (ev) cudaEventRecord(ev[1], s);
     const int flags = (((uintptr_t)a.x & 15) == 0 ? 1 : 0) |
                       (a.mode == MODE_FINAL && ((uintptr_t)a.u0 & 15) == 0 ? 2 : 0);
-    k_mixed_fused<EQ, N><<<grid, kFusedThreads, C::BYTES, s>>>(d, a, p->rowsum, flags);
+    const cudaError_t e = launch_kernel(k_mixed_fused<EQ, N>, grid, kFusedThreads, C::BYTES, s, a.overlap != 0, d, a,
+                                        (const double*)p->rowsum, flags);
     if (ev) {
       cudaEventRecord(ev[2], s);
       cudaEventRecord(ev[3], s);
     }
-    return cudaGetLastError();
+    return e;
   }
 }
 

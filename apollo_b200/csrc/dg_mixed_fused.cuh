@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
   const uint32_t mbX = umma::smem_u32(mbar + 0), mbD1 = umma::smem_u32(mbar + 1), mbD2 = umma::smem_u32(mbar + 2),
                  mbD3 = umma::smem_u32(mbar + 3), mbDrain = umma::smem_u32(mbar + 4), mbG = umma::smem_u32(mbar + 5);
 
+  allow_next();
   // ---- once per CTA: operators split into tf32 halves (K-major), zeroed operands
   for (int i = tid; i < C::NC16 * K1; i += kFusedThreads) {
     const int r = i / K1, k = i % K1;
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     for (int b = 0; b < 6; ++b) umma::mbar_init(umma::smem_u32(mbar + b), 1);
     *abort_flag = 0;
   }
+  wait_previous();  // the stage before has ended: its results and its tensor memory
   if (warp == 0) umma::tmem_alloc(umma::smem_u32(tslot), C::TCOLS);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   umma::fence_proxy_async();
