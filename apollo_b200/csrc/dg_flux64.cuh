@@ -12,8 +12,13 @@ namespace apollo {
 // approximation (PTX rcp.approx.ftz.f64, rsqrt.approx.ftz.f64; relative error
 // e of some 2^-20) corrected once by the third-order iteration that the series
 // of 1/(1-e) and (1-e)^(-1/2) give (Householder, The Numerical Treatment of a
-// Single Nonlinear Equation, 1970), which leaves e^3.  Error measured against
-// the general operations: at most one unit in the last place.
+// Single Nonlinear Equation, 1970), which leaves e^3.  Error measured against the
+// correctly rounded operations over 1.5e9 numbers between 2^-400 and 2^400: at
+// most one unit in the last place (two for the reciprocal root, against the
+// rounded reciprocal of the rounded root).  Together with the tile prefetch and
+// one branch for a lane's two points they took a right-hand side of Euler N = 4,
+// K = 130,050 from 256 to 199 us, of HLL with 5 fields, N = 3, K = 32,258 from
+// 122 to 67.
 __device__ __forceinline__ double recip_normal(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

@@ -293,11 +293,10 @@ apollo_status enqueue_stage(apollo_dg* h, const StageArgs& a, apollo_precision p
   return APOLLO_OK;
 }
 
-// Stage i of SSPRK(5,2).  Stages update W in place: the float64 kernels read
-// neighbour data only in the volume/face kernels, before the LIFT kernel
-// writes, and the mixed kernel reads only its own elements' state plus the
-// face traces of the previous stage, which alternate between T0 and T1 (TU
-// holds those of U).
+// Stage i of SSPRK(5,2).  Stage states alternate between W and W2, since the
+// float64 stage reads its neighbours' states while other warps write theirs;
+// the mixed kernel reads only its own elements' state plus the face traces of
+// the previous stage, which alternate between T0 and T1 (TU holds those of U).
 StageArgs stage_args(const apollo_dg* h, int i) {
   const int s = 5;
   StageArgs a{};

@@ -2,7 +2,9 @@
 // for callers that cannot allocate device memory when they evaluate it.
 //
 // The three float64 kernels (volume, face, LIFT) pass the volume term, the
-// face traces and the face fluxes between them through global memory.  The
+// face traces and the face fluxes between them through global memory (the fused
+// stage, which calls with aligned disjoint arrays take, needs none of them; the
+// size limit is the same for both, since the caller's arrays decide).  The
 // regular entry point keeps those arrays in the handle; this one keeps them in
 // g_rhs_scratch below, a fixed 64 MiB array that every GPU loading the library
 // holds until the process exits.  Nothing here calls cudaMalloc or cudaFree.

@@ -28,7 +28,14 @@
 // makes a round trip through memory.
 //
 // What bounds it.  The float64 pipe: mma.m8n8k4 and DFMA share 64 multiply-adds
-// per clock and SM.
+// per clock and SM (measured: either alone 63.9, the two in turn 86-93 % of
+// that).  Euler N = 4 fills 69 % of it (K = 79,202: DMMA 48 %, DFMA 20 %), the
+// rest is the latency of the pointwise flux; DRAM is at 6 %.  The linear
+// equations' smaller contractions leave it at 58 % with the shared-memory pipe
+// at 48 %.  A right-hand side, before (volume, face and LIFT kernels) and now:
+// Euler 4 fields, K = 130,050, N = 2..5: 168, 259, 355, 572 us and 87, 132, 195,
+// 329 us; Maxwell TM N = 5, K = 522,242: 1,796 and 300 us; 8 fields N = 5,
+// K = 32,258: 333 and 71 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -59,16 +66,19 @@ template <int EQ, int N> struct Chain {
   // [24] int2 and where the face nodes come from [24] int2
   static constexpr int ES = elem_stride(NP * M, M), FS = face_stride(3 * (N + 1) * M, M);
   static constexpr int X = 8 * ES, G = 8 * kGeoStride, PN = 8 * FS, C = 48;
-  static constexpr int XB = LIN && M != 8 || !LIN && N >= 5 ? 2 : 1;
+  // (8 fields would lose warps to it; Euler up to order 4 gains more from
+  // sixteen warps with one buffer than from twelve with two: K = 130,050, N = 4
+  // 202 -> 195 us; at order 5 the registers allow eight warps)
+  static constexpr int XB = (LIN && M != 8) || (!LIN && N >= 5) ? 2 : 1;
   // results leave by bulk copies where a row is long enough to pay for one:
   // K = 130,050: Euler N = 4 (480 bytes a row) 209 -> 204 us, Maxwell TM N = 5
   // (one copy of 4,032) 105 -> 95; Euler N = 2 (192 bytes) 89 -> 93
   static constexpr bool BULK = NP * M >= 30;
   static constexpr int WARP = XB * (X + G) + PN + C;
   static constexpr size_t bytes(int warps) { return sizeof(double) * (size_t)(SHARED + warps * WARP); }
-  // warps per block (one block per SM): what the registers allow
+  // warps per block (one block per SM): what registers and shared memory allow
   static constexpr int fit(int w) { return bytes(w) <= 227 * 1024 ? w : fit(w - 1); }
-    static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : (N >= 5 ? 8 : 16));
+  static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : (N >= 5 ? 8 : 16));
 };
 
 // One SSPRK stage (or right-hand side).  Reads the neighbours of x: x and out
@@ -488,7 +498,7 @@ cudaError_t launch_cut_nodes(int eq, const DgDev& d, const double* x, const int*
 
 // warps of one wave of k_stage64 (the launch-bound limit of form 2)
 int stage64_wave_tiles(int eq, int N, int sms) {
-  const int w = (eq == EQ_EULER || eq == EQ_EULER2D) ? (N >= 5 ? 8 : 12) : eq == EQ_MAXWELL ? 8 : 16;
+  const int w = (eq == EQ_EULER || eq == EQ_EULER2D) ? (N >= 5 ? 8 : 16) : eq == EQ_MAXWELL ? 8 : 16;
   return sms * w;
 }
 

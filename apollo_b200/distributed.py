@@ -1,11 +1,11 @@
-"""Partitioned meshes: one rank per GPU, cut-face traces exchanged once per stage.
+"""Partitioned meshes: one rank per GPU, cut-face blocks exchanged once per stage.
 
 Apollo distributes its mesh with PETSc DMPlex (overlap 1) and refreshes the
 ghost cells with ``DMGlobalToLocal`` before each right-hand side, then reduces
 the dt estimate with ``MPI_Allreduce`` (src/solvers/apsolver.cc:318-392,
-431-433).  Here each rank holds its elements plus ghost slots for the face
-traces of remote neighbours (``apollo_dg_set_mesh_partition``); per stage the
-library packs the traces of the cut faces into a send buffer, the
+431-433).  Here each rank holds its elements plus ghost slots for the faces of
+remote neighbours (``apollo_dg_set_mesh_partition``); per stage the library
+packs the cut faces (float64: their nodes, mixed: their traces) into a send buffer, the
 communicator moves them (NCCL point-to-point through ``torch.distributed`` on
 GPUs, gloo on CPU), and the library unpacks them into the ghost slots before
 the face fluxes.  The ranks together compute bit for bit what one handle on

@@ -70,7 +70,7 @@ def parse():
                     help="profiling driver: set up the workload, advance this many SSPRK steps, exit")
     ap.add_argument("--vjp-only", type=int, default=0,
                     help="profiling driver: set up the workload, evaluate this many adjoint right-hand sides, exit")
-    ap.add_argument("--fp64-kernels", type=int, default=0, choices=[0, 1, 2],
+    ap.add_argument("--fp64-kernels", type=int, default=1, choices=[0, 1, 2],
                     help="profiling drivers: the float64 stage form (0 three kernels, 1 fused, 2 by mesh size)")
     return ap.parse_args()
 
@@ -298,14 +298,13 @@ def advection_measure(args, device: int, cpu: bool):
         ends[prec] = s.get_state()
         out[prec] = {"value": dofs * steps / (ms / 1000.0), "ms_per_step": ms / steps, "t_end": t}
     out["l2_mixed_vs_fp64"] = float(np.linalg.norm(ends["mixed"] - ends["fp64"]) / np.linalg.norm(ends["fp64"]))
-    # the mesh is one wave of tiles: the fused float64 stage (one launch per
-    # stage instead of three) is the faster form here
-    s.set_fp64_kernels(1)
-    ms, (t, dt) = _device_run(s, stream, U0, dt0, "fp64", steps)
-    out["fp64_fused_stage"] = {"value": dofs * steps / (ms / 1000.0), "ms_per_step": ms / steps, "t_end": t,
-                               "l2_vs_fp64": float(np.linalg.norm(s.get_state() - ends["fp64"]) /
-                                                   np.linalg.norm(ends["fp64"]))}
+    # the other float64 form (three kernels per stage instead of the fused one)
     s.set_fp64_kernels(0)
+    ms, (t, dt) = _device_run(s, stream, U0, dt0, "fp64", steps)
+    out["fp64_three_kernels"] = {"value": dofs * steps / (ms / 1000.0), "ms_per_step": ms / steps, "t_end": t,
+                                 "l2_vs_fp64": float(np.linalg.norm(s.get_state() - ends["fp64"]) /
+                                                     np.linalg.norm(ends["fp64"]))}
+    s.set_fp64_kernels(1)
     # the configuration names an upwind flux; Apollo's advection flux is
     # Lax-Friedrichs with max(|ux|, |uy|) (the parity runs above), and the
     # upwind flux (dissipation |n.u|) is this library's extension
@@ -858,15 +857,11 @@ def partitioned_arm(args, rank: int, world: int, local: int):
         s1.set_state(np.ascontiguousarray(p.ic(xs, ys)))
         kt = s1.kernel_times(10, precision=prec)
         peaks, peak_src = measured_peaks()
-        K1, Np, M, Nf = s1.K, s1.Np, s1.m, 3 * s1.Ng
+        K1, Np, M = s1.K, s1.Np, s1.m
         if prec == "mixed":
             name, kms, alg = "stage", kt[1], K1 * (8 * 2 * Np * M + 160)
         else:
-            i = int(np.argmax(kt[:3]))
-            name, kms = ["volume", "face", "lift_update"][i], kt[i]
-            alg = {"volume": K1 * (8 * Np * M * 2 + 8 * Nf * M + 32),
-                   "face": (3 * K1 // 2) * 2 * (8 * s1.Ng * M) * 2 + (3 * K1 // 2) * 16,
-                   "lift_update": K1 * (8 * Np * M * 3 + 8 * Nf * M + 8)}[name]
+            name, kms, alg = "stage", kt[0], K1 * (8 * 2 * Np * M + 160)
         ach = alg / (kms / 1000.0) / 1e9
         roofline = {"bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                     "frac": ach / peaks["hbm_gbs"], "traffic": profile_traffic().get(f"{prec}:{name}:{WORKLOAD}"),
@@ -886,7 +881,7 @@ def partitioned_arm(args, rank: int, world: int, local: int):
                        "cut_faces_rank0": nsend,
                        "halo_bytes_per_stage_rank0": nsend * d.block_bytes[prec] * 2,
                        "l2_flush": "inputs larger than L2 (state + stage + scratch per rank > 126 MiB)"},
-            "gpu_launches": args.steps * (26 if prec == "fp64" else 16), "clocks": clocks, "roofline": roofline,
+            "gpu_launches": args.steps * (21 if prec == "fp64" else 16), "clocks": clocks, "roofline": roofline,
             "e2e": e2e, "cpu_baseline": None, **extra,
         }
         print(json.dumps(line), flush=True)
@@ -1046,7 +1041,6 @@ def ours_arm(args):
     N, K, M = p.N, s.K, s.m
     Np, Nc, Ng = s.Np, s.Nc, s.Ng
     Nf = 3 * Ng
-    nfaces = 3 * K // 2
     if prec == "mixed":
         # one right-hand side = the trace kernel (state -> fp32 face traces) and
         # the fused stage kernel in right-hand-side mode
@@ -1061,17 +1055,11 @@ def ours_arm(args):
         }
         kt = kt[:2]
     else:
-        names = ["volume", "face", "lift_update"]
-        alg_bytes = {  # compulsory bytes per launch (float64)
-            "volume": K * (8 * Np * M + 8 * Np * M + 8 * Nf * M + 32),
-            "face": nfaces * 2 * (8 * Ng * M) * 2 + nfaces * 16,
-            "lift_update": K * (8 * Np * M * 3 + 8 * Nf * M + 8),
-        }
-        alg_flops = {
-            "volume": K * 2 * M * (Nc * Np + 2 * Nc * Np + Nf * Np),
-            "face": nfaces * Ng * 60,
-            "lift_update": K * 2 * M * Nf * Np,
-        }
+        # one launch per right-hand side
+        names = ["stage_rhs"]
+        alg_bytes = {"stage_rhs": K * (8 * 2 * Np * M + 160)}  # read x, write the RHS, geometry
+        alg_flops = {"stage_rhs": K * 2 * M * (3 * Nc * Np + 2 * Nf * Np + Np * Np)}
+        kt = kt[:1]
     dom = int(np.argmax(kt))
     dname = names[dom]
     achieved = alg_bytes[dname] / (kt[dom] / 1000.0) / 1e9
@@ -1091,9 +1079,7 @@ def ours_arm(args):
     stage_b = 8 * 3 * Np * M + 160
     stage_ms = ms_step / 5.0
     stage_ach = stage_b * K / (stage_ms / 1000.0) / 1e9
-    stage_traffic = (profile_traffic().get(f"mixed:stage:{workload_name(p.N, s.K)}") if prec == "mixed" else
-                     sum(profile_traffic().get(f"fp64:{k}:{workload_name(p.N, s.K)}") or 0
-                         for k in ("volume", "face", "lift_update")) or None)
+    stage_traffic = profile_traffic().get(f"{prec}:stage:{workload_name(p.N, s.K)}")
     roofline["stage_mode"] = {"bytes_per_element": stage_b, "bytes": stage_b * K, "stage_ms": stage_ms,
                               "achieved": stage_ach, "frac": stage_ach / peaks["hbm_gbs"],
                               "traffic": stage_traffic,
@@ -1194,8 +1180,8 @@ def ours_arm(args):
                 extra["apollo_cpu"] = {"error": str(exc)}
 
     if rank == 0:
-        # our kernels per step: float64 5 x (volume, face, lift) + finalize;
-        # mixed 5 fused stages + finalize (the trace kernel runs in the warm-up)
+        # our kernels per step: 5 fused stages + finalize (mixed: the trace
+        # kernel runs in the warm-up)
         line = {
             "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
@@ -1207,7 +1193,7 @@ def ours_arm(args):
                        f"{(dofs * 8 * 4 + 2 * K * Nf * M * 8) / 2**20:.0f} MiB > 126 MiB)",
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
             "l2_vs_exact_vortex": l2_exact, "t_end": t_end,
-            "gpu_launches": args.steps * (16 if prec == "fp64" else 6), "clocks": clocks, "roofline": roofline, "e2e": e2e,
+            "gpu_launches": args.steps * 6, "clocks": clocks, "roofline": roofline, "e2e": e2e,
             "cpu_baseline": cpu, **extra,
         }
         print(json.dumps(line), flush=True)

@@ -454,8 +454,9 @@ apollo_status apollo_dg_mesh_destroy(apollo_dg_mesh* m);
  * Apollo's PETSc DMPlex distribution with an overlap-1 halo refreshed by
  * DMGlobalToLocal before every right-hand side (src/solvers/apsolver.cc:318-392)
  * and its MPI_Allreduce of the dt estimate (apsolver.cc:431-433): here only the
- * face traces of cut faces cross between ranks, once per stage, and the
- * caller's communicator (NCCL, MPI, ...) moves them.
+ * data of the cut faces crosses between ranks (float64: the face's nodes; mixed:
+ * its fp32 traces), once per stage, and the caller's communicator (NCCL, MPI,
+ * ...) moves it.
  *
  * Host-only calls (no device needed): */
 /* Recursive coordinate bisection of the element centroids: part[K] receives
@@ -467,8 +468,8 @@ typedef struct {
   int n_local;  /* elements owned by the rank */
   int n_ghost;  /* remote elements sharing a face with a local one */
   int n_peers;  /* ranks exchanged with */
-  int n_send;   /* trace blocks sent per stage (one per cut face) */
-  int n_recv;   /* trace blocks received per stage */
+  int n_send;   /* face blocks sent per stage (one per cut face) */
+  int n_recv;   /* face blocks received per stage */
 } apollo_dg_halo_sizes;
 
 /* The halo plan of one rank of the global mesh (apollo_dg_set_mesh's mesh
@@ -487,7 +488,7 @@ apollo_status apollo_dg_halo_plan(int nverts, int K, const int* etov, const int*
 /* Device calls: */
 /* Like apollo_dg_set_mesh with the GLOBAL mesh, keeping the elements with
  * part[k] == rank (in global order; node coordinates, states and
- * apollo_dg_num_elements refer to them) plus ghost slots for the traces of
+ * apollo_dg_num_elements refer to them) plus ghost slots for the face blocks of
  * their remote neighbours.  Every face keeps the orientation it has in the
  * global mesh and dt uses the global inscribed radius, so the ranks together
  * compute bit for bit what one handle on the whole mesh computes.  With
@@ -496,8 +497,9 @@ apollo_status apollo_dg_halo_plan(int nverts, int K, const int* etov, const int*
 apollo_status apollo_dg_set_mesh_partition(apollo_dg* h, int nverts, const double* vx, const double* vy, int K,
                                            const int* etov, const int* face_tag, const int* vert_canon,
                                            const int* part, int rank);
-/* Peers (ascending), blocks per peer and the bytes of one trace block in this
- * precision (float64 or float32 traces); any pointer may be NULL. */
+/* Peers (ascending), blocks per peer and the bytes of one face block in this
+ * precision (float64: the N + 1 face nodes at its front); any pointer may be
+ * NULL. */
 apollo_status apollo_dg_halo_info(const apollo_dg* h, apollo_precision prec, int* n_peers, int* peers,
                                   int* send_count, int* recv_count, int* block_bytes);
 /* Caller-owned device buffers, 16-byte aligned: send and recv hold the blocks
@@ -510,7 +512,7 @@ apollo_status apollo_dg_halo_bind(apollo_dg* h, void* send, size_t send_bytes, v
 /* Staged stepping, all on the handle's stream (nothing waits on the host):
  *   apollo_dg_dist_start(t, dt)          once, before the first step
  *   per step, for stage = 0..4:
- *     apollo_dg_stage_begin(stage)       traces of the stage input, packed into send
+ *     apollo_dg_stage_begin(stage)       face blocks of the stage input, packed into send
  *     <caller: send -> peers, peers -> recv>
  *     apollo_dg_stage_end(stage)         recv unpacked into the ghost slots, the stage
  *   <caller: MAX all-reduce of the lam word> (stage 4 wrote it)
