@@ -24,7 +24,7 @@ apollo_status handle_set_instances(apollo_dg* h, int ninst, const int* einst);
 cudaStream_t handle_stream(const apollo_dg* h);
 DevState* handle_states_host(apollo_dg* h);
 apollo_status handle_push_states(apollo_dg* h);
-apollo_status handle_pull_states(apollo_dg* h);
+apollo_status handle_pull_states(apollo_dg* h, cudaStream_t s);
 apollo_status handle_init_speed(apollo_dg* h);
 double handle_rmin(const apollo_dg* h);
 double handle_cfl(const apollo_dg* h);
@@ -344,7 +344,7 @@ apollo_status apollo_dg_batch_init_dt(apollo_dg_batch* b, double* dt) {
   if (!b || !b->finalized || !dt) return APOLLO_ERR_ARG;
   for (auto& G : b->groups) {
     apollo_status r = from_handle(b, G.h, handle_init_speed(G.h));
-    if (!r) r = from_handle(b, G.h, handle_pull_states(G.h));
+    if (!r) r = from_handle(b, G.h, handle_pull_states(G.h, handle_stream(G.h)));
     if (r) return r;
   }
   for (auto& G : b->groups) {
@@ -376,16 +376,21 @@ apollo_status apollo_dg_batch_step(apollo_dg_batch* b, int nsteps, double* t, do
     if (!r) r = from_handle(b, G.h, handle_prepare_step(G.h, prec));
     if (r) return r;
   }
-  for (auto& G : b->groups) BCK(cudaStreamSynchronize(handle_stream(G.h)), "batch step");
+  // the graph follows every group's copies, and one wait ends the call
+  for (size_t i = 0; i < b->groups.size(); ++i) {
+    BCK(cudaEventRecord(b->join[i], handle_stream(b->groups[i].h)), "batch step");
+    BCK(cudaStreamWaitEvent(b->master, b->join[i], 0), "batch step");
+  }
   cudaGraphExec_t g = nullptr;
   apollo_status r = build_graph(b, prec, &g);
   if (r) return r;
   for (int i = 0; i < nsteps; ++i) BCK(cudaGraphLaunch(g, b->master), "batch graph launch");
+  for (auto& G : b->groups) {
+    r = from_handle(b, G.h, handle_pull_states(G.h, b->master));
+    if (r) return r;
+  }
   BCK(cudaStreamSynchronize(b->master), "batch step");
   for (auto& G : b->groups) {
-    r = from_handle(b, G.h, handle_pull_states(G.h));
-    if (r) return r;
-    BCK(cudaStreamSynchronize(handle_stream(G.h)), "batch step");
     const DevState* st = handle_states_host(G.h);
     for (int id : G.insts) {
       t[id] = st[b->inst[id].local].t;
@@ -418,7 +423,7 @@ apollo_status apollo_dg_batch_autotune(apollo_dg_batch* b, apollo_precision prec
   for (size_t gi = 0; gi < b->groups.size(); ++gi) {
     apollo_dg* h = b->groups[gi].h;
     const DevState* st = handle_states_host(h);
-    apollo_status r = from_handle(b, h, handle_pull_states(h));
+    apollo_status r = from_handle(b, h, handle_pull_states(h, handle_stream(h)));
     if (r) return r;
     BCK(cudaStreamSynchronize(handle_stream(h)), "autotune");
     for (int id : b->groups[gi].insts) {

@@ -1288,15 +1288,15 @@ apollo_status handle_set_instances(apollo_dg* h, int ninst, const int* einst) {
 cudaStream_t handle_stream(const apollo_dg* h) { return h->stream; }
 DevState* handle_states_host(apollo_dg* h) { return h->st_h; }
 
-// host states <-> device states (all instances), on the handle's stream
+// host states <-> device states (all instances): to the device on the handle's
+// stream, back on a stream that follows the work
 apollo_status handle_push_states(apollo_dg* h) {
   CK(cudaMemcpyAsync(h->st_d, h->st_h, (size_t)h->ninst * sizeof(DevState), cudaMemcpyHostToDevice, h->stream),
      "states");
   return APOLLO_OK;
 }
-apollo_status handle_pull_states(apollo_dg* h) {
-  CK(cudaMemcpyAsync(h->st_h, h->st_d, (size_t)h->ninst * sizeof(DevState), cudaMemcpyDeviceToHost, h->stream),
-     "states");
+apollo_status handle_pull_states(apollo_dg* h, cudaStream_t s) {
+  CK(cudaMemcpyAsync(h->st_h, h->st_d, (size_t)h->ninst * sizeof(DevState), cudaMemcpyDeviceToHost, s), "states");
   return APOLLO_OK;
 }
 

@@ -176,6 +176,16 @@ def _ptr(a, sync: bool = True):
     return C.c_void_p(a.data_ptr()), APOLLO_HOST_PTR
 
 
+def _ptrs(*arrays):
+    """``_ptr`` of each; torch's stream of a device is drained once."""
+    got, drained = [], []
+    for a in arrays:
+        dev = None if isinstance(a, np.ndarray) or not a.is_cuda else a.device
+        got.append(_ptr(a, sync=dev not in drained))
+        drained.append(dev)
+    return got
+
+
 class NodalDG2d:
     """One nodal-DG discretisation on the GPU (Apollo ``Kind = nodalDG2d``)."""
 
@@ -327,8 +337,7 @@ class NodalDG2d:
         """One RHS evaluation out = L(u) (WxNodalDG2dMethod::step); returns (out, suggested dt)."""
         if out is None:
             out = np.empty(self.shape) if isinstance(u, np.ndarray) else u.new_empty(u.shape)
-        pi, wi = _ptr(u)
-        po, wo = _ptr(out)
+        (pi, wi), (po, wo) = _ptrs(u, out)
         assert wi == wo
         s = C.c_double()
         self._check(self.lib.apollo_dg_rhs(self.h, t, dt, pi, po, C.byref(s), wi, PREC[precision]))
@@ -413,8 +422,7 @@ class NodalDG2d:
     def backward(self, ubar_T, out=None):
         """dJ/dU(0) of the last forward_fixed trajectory, given dJ/dU(T)."""
         out = self._like(ubar_T, out)
-        pi, wi = _ptr(ubar_T)
-        po, wo = _ptr(out)
+        (pi, wi), (po, wo) = _ptrs(ubar_T, out)
         assert wi == wo
         self._check(self.lib.apollo_dg_backward(self.h, pi, po, wi))
         return out
@@ -422,21 +430,20 @@ class NodalDG2d:
     def tangent(self, nsteps: int, t0: float, dt: float, du0, out=None):
         """Advance the resident state and return (dU(T)/dU(0)) du0."""
         out = self._like(du0, out)
-        pi, wi = _ptr(du0)
-        po, wo = _ptr(out)
+        (pi, wi), (po, wo) = _ptrs(du0, out)
         assert wi == wo
         self._check(self.lib.apollo_dg_tangent(self.h, nsteps, t0, dt, pi, po, wi))
         return out
 
     def rhs_jvp(self, t: float, x, v, out=None):
         out = self._like(x, out)
-        (px, wx), (pv, _), (po, _) = _ptr(x), _ptr(v), _ptr(out)
+        (px, wx), (pv, _), (po, _) = _ptrs(x, v, out)
         self._check(self.lib.apollo_dg_rhs_jvp(self.h, t, px, pv, po, wx))
         return out
 
     def rhs_vjp(self, t: float, x, w, out=None):
         out = self._like(x, out)
-        (px, wx), (pw, _), (po, _) = _ptr(x), _ptr(w), _ptr(out)
+        (px, wx), (pw, _), (po, _) = _ptrs(x, w, out)
         self._check(self.lib.apollo_dg_rhs_vjp(self.h, t, px, pw, po, wx))
         return out
 
