@@ -52,7 +52,12 @@ template <int EQ, int N> struct Deriv {
     return sizeof(double) * (size_t)(round_up(ops + TABS, 2) + warps * WARP);
   }
   static constexpr int fit(int ops, int w) { return bytes(ops, w) <= 227 * 1024 ? w : fit(ops, w - 1); }
-  static constexpr int WMAX = LIN ? (M == 8 ? 8 : 12) : (N >= 5 || M == 5 ? 8 : 12);
+  // Eight warps have 255 registers a lane.  Twelve have 168, and the Euler
+  // kernels then spill 40 to 470 bytes a lane: the gradient of ten steps, N = 3,
+  // K = 6,962 2,605 us with twelve and 2,192 with eight, N = 4, K = 32,258 9,495
+  // and 8,990, N = 3, K = 32,258 6,000 and 5,890.  The linear equations (but for
+  // eight fields) fit in 168.
+  static constexpr int WMAX = LIN && M != 8 ? 12 : 8;
   static constexpr int ADJ_WARPS = fit(ADJ_OPS, WMAX), TAN_WARPS = fit(TAN_OPS, WMAX);
 };
 
@@ -141,11 +146,17 @@ template <int EQ, int N> struct Warp {
     for (int i = tid; i < T::NG; i += blockDim.x) sGz[i] = d.gz[i];
     for (int i = tid; i < PK::NFN; i += blockDim.x) sFm[i] = PK::face_node(i / (N + 1), i % (N + 1));
   }
+  // lane's entry of a tile's connectivity
+  __device__ __forceinline__ int2 load_conn(const DgDev& d, int tile) const {
+    const int l = min(lane, 23);
+    return *reinterpret_cast<const int2*>(d.conn + (size_t)min(tile * 8 + l / 3, d.K - 1) * 6 + 2 * (l % 3));
+  }
+  // a tile's own arrays; the neighbours' nodes arrive during the volume term
+  // (faces_here), and the next tile's connectivity replaces conn
   __device__ __forceinline__ void load(const DgDev& d, int tile, const double* a, const double* b) {
     const int ke = min(tile * 8 + lr, d.K - 1);
     __syncwarp();  // the previous tile's reads are done
-    if (lane < 24)
-      sC[lane] = *reinterpret_cast<const int2*>(d.conn + (size_t)min(tile * 8 + lane / 3, d.K - 1) * 6 + 2 * (lane % 3));
+    if (lane < 24) sC[lane] = load_conn(d, tile);
     copy_tile<NP * M, T::ES>(sB, b, tile, d.K, lane);
     if (!T::LIN) copy_tile<NP * M, T::ES>(sA, a, tile, d.K, lane);
 #pragma unroll
@@ -153,10 +164,16 @@ template <int EQ, int N> struct Warp {
       const int i = lane + 32 * u, e = i >> 3, q = i & 7;
       cp_async16(sG + kGeoStride * e + 2 * q, reinterpret_cast<const double*>(d.geo + min(tile * 8 + e, d.K - 1)) + 2 * q);
     }
+    cp_async_commit();
     __syncwarp();
     copy_face_nodes<N, M, T::FS>(sPB, b, sC, sFm, ke, lr, lc);
     if (!T::LIN) copy_face_nodes<N, M, T::FS>(sPA, a, sC, sFm, ke, lr, lc);
-    cp_async_wait_all();
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncwarp();
+  }
+  __device__ __forceinline__ void faces_here() const {
+    cp_async_wait<0>();
     __syncwarp();
   }
   // boundary hook of face fc at face coordinate z
@@ -231,13 +248,14 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
   Warp<EQ, N> W;
   W.init(d, smem, T::ADJ_OPS);
   allow_next();
+  const int stride = gridDim.x * (blockDim.x >> 5), first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   cp_async_wait_all();
   __syncthreads();
   wait_previous();
   const int lane = W.lane, lr = W.lr, lc = W.lc;
   int err = 0;  // the float64 forward reports non-physical states
   const int ntiles = (d.K + 7) / 8;
-  for (int tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; tile < ntiles; tile += gridDim.x * (blockDim.x >> 5)) {
+  for (int tile = first; tile < ntiles; tile += stride) {
     const int ke = min(tile * 8 + lr, d.K - 1);
     double wv[PK::NBT][M][2];
 #pragma unroll
@@ -258,6 +276,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
         acc.add(sWT + k * PK::NS, lane, u, z);
       }
       // at the face nodes: sJ (y_own - y_partner) through the flux Jacobian
+      W.faces_here();
 #pragma unroll 1
       for (int qb = 0; qb < PK::QB; ++qb) {
         double A[2][M];
@@ -328,6 +347,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::ADJ_WARPS, 1) k_adjoint64(D
         }
         acc.add(sVT + (pb) * PK::NS, lane, g[0], g[1]);
       }
+      W.faces_here();
 #pragma unroll 1
       for (int fb = 0; fb < PK::FB; ++fb) {
         const int p0 = min(fb * 8 + 2 * lc, NF - 2), fc = p0 / NG, g0 = p0 - fc * NG;
@@ -421,13 +441,14 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
   Warp<EQ, N> W;
   W.init(d, smem, T::TAN_OPS);
   allow_next();
+  const int stride = gridDim.x * (blockDim.x >> 5), first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   cp_async_wait_all();
   __syncthreads();
   wait_previous();
   const int lane = W.lane, lr = W.lr, lc = W.lc;
   int err = 0;  // the float64 forward reports non-physical states
   const int ntiles = (d.K + 7) / 8;
-  for (int tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; tile < ntiles; tile += gridDim.x * (blockDim.x >> 5)) {
+  for (int tile = first; tile < ntiles; tile += stride) {
     const int ke = min(tile * 8 + lr, d.K - 1);
     W.load(d, tile, a.x, a.dx);
     const double *ge = W.sG + kGeoStride * lr, *xe = W.sA + lr * T::ES, *de = W.sB + lr * T::ES;
@@ -446,6 +467,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
         LinearFast64<EQ>::along(d.eqp, q, sx, sy, S);
         acc.add(sW + k * PK::NS, lane, R, S);
       }
+      W.faces_here();
 #pragma unroll 1
       for (int qb = 0; qb < PK::QB; ++qb) {
         double A[2][M];
@@ -500,6 +522,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
         acc.add(sD + (pb * 2) * PK::NS, lane, R[0], R[1]);
         acc.add(sD + (pb * 2 + 1) * PK::NS, lane, S[0], S[1]);
       }
+      W.faces_here();
 #pragma unroll 1
       for (int fb = 0; fb < PK::FB; ++fb) {
         const int p0 = min(fb * 8 + 2 * lc, NF - 2), fc = p0 / NG, g0 = p0 - fc * NG;
