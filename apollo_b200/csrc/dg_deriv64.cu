@@ -16,10 +16,10 @@
 // Tangent: the forward stage on the pair (x, v).
 //
 // What bounds them: the float64 pipe and the latency of the pointwise
-// derivatives, as the forward stage (Euler N = 3, K = 32,258: 51 % of the pipe
+// derivatives, as the forward stage (Euler N = 3, K = 32,258: 53 % of the pipe
 // busy).  Euler N = 3, K = 32,258, before (trace and face kernels of their own,
 // block-wide contractions) and now: adjoint right-hand side 22 + 120 and
-// 10 + 54 us, tangent 57 + 43 us and the LIFT kernel, and 58 us.
+// 10 + 51 us, tangent 57 + 43 us and the LIFT kernel, and 53 us.
 #include <cuda_runtime.h>
 
 #include "dg_adjoint.h"

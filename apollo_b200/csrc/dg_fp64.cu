@@ -590,10 +590,15 @@ int fp64_supported(int eq, int N) { return eq >= 0 && eq <= 4 && N >= 2 && N <= 
 
 // The fused stage where it applies: an output that does not overlap the input
 // (it reads the neighbours' states while other warps write theirs), and arrays
-// that start on a 16-byte boundary (its copies and vector accesses).  Where it
-// applies it is the faster one at every size measured (a right-hand side,
-// three kernels and fused: Euler N = 2, K = 130,050 168 and 87 us, N = 5 572 and
-// 329; 8 fields N = 3, K = 32,258 129 and 39).
+// that start on a 16-byte boundary (its copies and vector accesses).  The
+// rule knows no mesh size or flux, so that batches and partitions compute the
+// whole mesh's bits.  A right-hand side, three kernels and fused: Euler N = 2,
+// K = 130,050 168 and 87 us, N = 5 572 and 329; 8 fields N = 3, K = 32,258 129
+// and 39; HLL 5 fields N = 3, K = 50,562 260 and 84; Wave the same 304 and 181.
+// The three kernels stay faster for Roe and Wave below one wave of tiles (5
+// fields, N = 3, K = 2,048: Roe 41 and 46, Wave 48 and 52; N = 5 51 and 63), for
+// Roe with 4 fields at orders 2 and 5, and for HLL below a wave with 5 fields at
+// order 5 (57 and 65) and 4 at order 2 (37 and 39).
 static bool fused_applies(int eq, const DgDev& d, const StageArgs& a) {
   if (d.fp64_fused == 0) return false;
   if (d.fp64_fused == 2 && (d.K + 7) / 8 > stage64_wave_tiles(eq, d.N, num_sms())) return false;
