@@ -446,7 +446,9 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
   __syncthreads();
   wait_previous();
   const int lane = W.lane, lr = W.lr, lc = W.lc;
-  int err = 0;  // the float64 forward reports non-physical states
+  // reported: a non-physical state at a cubature point and a NaN in the result
+  // (at the face points the forward stage reports them)
+  int err = 0, face_err = 0;
   const int ntiles = (d.K + 7) / 8;
   for (int tile = first; tile < ntiles; tile += stride) {
     const int ke = min(tile * 8 + lr, d.K - 1);
@@ -571,7 +573,7 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
               pa[f].v = qP[j][f];
               pa[f].d[0] = dP[j][f];
             }
-            Eq<EQ>::lf(d.eqp, Dual<1>(nx), Dual<1>(ny), ma, pa, nf, &err);
+            Eq<EQ>::lf(d.eqp, Dual<1>(nx), Dual<1>(ny), ma, pa, nf, &face_err);
 #pragma unroll
             for (int f = 0; f < M; ++f) A[j][f] = 2.0 * w * nf[f].d[0];
           }
@@ -584,10 +586,16 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
     if (tile * 8 + lr < d.K) {
       const size_t off = (size_t)ke * NP * M;
       const double c_r = a.mode == MODE_STAGE ? a.dt / 4.0 : a.dt / 5.0;
+      int top = 0;  // as in k_stage64: above infinity's, a NaN
 #pragma unroll
       for (int b = 0; b < PK::NBT; ++b) {
         double o[M][2];
         acc.get(b, lc, o);
+#pragma unroll
+        for (int f = 0; f < M; ++f) {
+          top = max(top, __double2hiint(o[f][0]) & 0x7fffffff);
+          top = max(top, __double2hiint(o[f][1]) & 0x7fffffff);
+        }
         if (a.mode != MODE_RHS) {
           double x[M][2];
           load_block<M, PK>(de, b, lc, x);
@@ -607,9 +615,11 @@ __global__ void __launch_bounds__(32 * Deriv<EQ, N>::TAN_WARPS, 1) k_tangent64(D
         }
         store_block<M, PK>(a.dout + off, b, lc, o);
       }
+      if (top > 0x7ff00000) err |= ERRB_NAN;
     }
   }
-  (void)err;
+  (void)face_err;
+  if (err) atomicOr(&d.st->err, err);
 }
 
 template <class Kern>
