@@ -419,6 +419,9 @@ __global__ void __launch_bounds__(kMixThreads, 1)
     *abort_flag = 0;
   }
   wait_previous();  // the stage before has ended: its results and its tensor memory
+  // a stage that reduces no wave speeds clears the word for the one that does
+  if (a.mode == MODE_STAGE && a.reset_lambda && blockIdx.x == 0)
+    for (int i = tid; i < d.ninst; i += kMixThreads) d.st[i].lam_bits = 0ull;
   if (warp == 0) umma::tmem_alloc(umma::smem_u32(tslot), C::TCOLS);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   umma::fence_proxy_async();
@@ -1139,8 +1142,7 @@ cudaError_t launch_mixed_sh(MixedPlan* p, const DgDev& d, const StageArgs& a0, c
     int grid = sms;
     if (grid > ntiles) grid = ntiles;
     StageArgs a = a0;
-    // a step's last stage finds the word clear: the stages before reduce
-    // nothing, and the step's start and the end of the one before cleared it
+    // a step's last stage finds the word clear: the stages before clear it
     if (a.reset_lambda && a.mode == MODE_RHS) {
       cudaError_t e = launch_reset_lambda(d, s);
       if (e != cudaSuccess) return e;
@@ -1195,8 +1197,7 @@ cudaError_t launch_fused(MixedPlan* p, const DgDev& d, const StageArgs& a0, cuda
     int grid = sms;
     if (grid > ntiles) grid = ntiles;
     StageArgs a = a0;
-    // a step's last stage finds the word clear: the stages before reduce
-    // nothing, and the step's start and the end of the one before cleared it
+    // a step's last stage finds the word clear: the stages before clear it
     if (a.reset_lambda && a.mode == MODE_RHS) {
       cudaError_t e = launch_reset_lambda(d, s);
       if (e != cudaSuccess) return e;

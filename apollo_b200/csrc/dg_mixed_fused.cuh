@@ -191,6 +191,9 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     *abort_flag = 0;
   }
   wait_previous();  // the stage before has ended: its results and its tensor memory
+  // a stage that reduces no wave speeds clears the word for the one that does
+  if (a.mode == MODE_STAGE && a.reset_lambda && blockIdx.x == 0)
+    for (int i = tid; i < d.ninst; i += kFusedThreads) d.st[i].lam_bits = 0ull;
   if (warp == 0) umma::tmem_alloc(umma::smem_u32(tslot), C::TCOLS);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   umma::fence_proxy_async();
