@@ -98,9 +98,10 @@ struct apollo_dg {
   size_t hsend_bytes = 0, hrecv_bytes = 0;
   // elements without a cut face first (nel_int of them), then the others: a
   // float64 stage runs the first group on side_stream while the caller's
-  // exchange is in flight
+  // exchange is in flight; until the handle's stream has joined it, side_busy
   int* elist_d = nullptr;
   int nel_int = 0;
+  bool side_busy = false;
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_packed = nullptr, ev_interior = nullptr;
   // Euler limiter (apollo_dg_set_limiter): applied to every stage input
@@ -162,6 +163,8 @@ void dfree(T*& p) {
 }
 
 void free_mesh(apollo_dg* h) {
+  if (h->side_busy) cudaStreamSynchronize(h->side_stream);
+  h->side_busy = false;
   for (auto& g : h->graph)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   dfree(h->geo_d); dfree(h->faces_d); dfree(h->conn_d); dfree(h->einst_d);
@@ -238,13 +241,22 @@ DgDev make_dev(const apollo_dg* h) {
   return d;
 }
 
-apollo_status check_ready(apollo_dg* h) {
-  if (!h) return APOLLO_ERR_ARG;
-  if (h->eq < 0) return fail(h, APOLLO_ERR_STATE, "no equation set");
-  if (h->K == 0) return fail(h, APOLLO_ERR_STATE, "no mesh set");
+// The handle's stream waits for the side stream's part of a partitioned stage
+// that apollo_dg_stage_begin started (and whose exchange may have failed).
+apollo_status join_side(apollo_dg* h) {
+  if (!h->side_busy) return APOLLO_OK;
+  CK(cudaStreamWaitEvent(h->stream, h->ev_interior, 0), "stage event");
+  h->side_busy = false;
   return APOLLO_OK;
 }
 
+// every call but apollo_dg_stage_end, which joins the side stream later
+apollo_status check_ready(apollo_dg* h, bool join = true) {
+  if (!h) return APOLLO_ERR_ARG;
+  if (h->eq < 0) return fail(h, APOLLO_ERR_STATE, "no equation set");
+  if (h->K == 0) return fail(h, APOLLO_ERR_STATE, "no mesh set");
+  return join ? join_side(h) : APOLLO_OK;
+}
 
 // the derivatives do not differentiate the limiter
 apollo_status check_adjoint_flux(apollo_dg* h) {
@@ -991,12 +1003,14 @@ apollo_status apollo_dg_step_async(apollo_dg* h, int nsteps, double t, double dt
 
 apollo_status apollo_dg_synchronize(apollo_dg* h) {
   if (!h) return APOLLO_ERR_ARG;
+  if (apollo_status r = join_side(h)) return r;
   CK(cudaStreamSynchronize(h->stream), "synchronize");
   return APOLLO_OK;
 }
 
 apollo_status apollo_dg_get_time(apollo_dg* h, double* t, double* dt) {
   if (!h || !t || !dt) return APOLLO_ERR_ARG;
+  if (apollo_status r = join_side(h)) return r;
   CK(cudaMemcpyAsync(h->st_h, h->st_d, sizeof(DevState), cudaMemcpyDeviceToHost, h->stream), "get time");
   CK(cudaStreamSynchronize(h->stream), "get time");
   *t = h->st_h->t;
@@ -1874,19 +1888,22 @@ apollo_status apollo_dg_stage_begin(apollo_dg* h, int stage, apollo_precision pr
   } else if (!h->peers.empty()) {
     // the cut faces' nodes, then the stage of the elements without a cut face
     // on the side stream while the caller's exchange is in flight (enqueued on
-    // the handle's stream after this call); apollo_dg_stage_end joins it
+    // the handle's stream after this call); apollo_dg_stage_end joins it.  Not
+    // the last stage, which writes over the step's start state: where its
+    // exchange fails, that state is still whole and the stage can be begun again.
     CK(launch_cut_nodes(h->eq, d, a.x, h->halo_src_d, h->n_send, (double*)h->hsend, h->stream), "halo pack");
-    if (h->nel_int > 0) {
+    if (h->nel_int > 0 && a.mode == MODE_STAGE) {
       CK(fork_side(h), "stage event");
       CK(launch_stage64(h->eq, d, a, h->elist_d, h->nel_int, h->side_stream), "interior stage launch");
       CK(cudaEventRecord(h->ev_interior, h->side_stream), "stage event");
+      h->side_busy = true;
     }
   }
   return APOLLO_OK;
 }
 
 apollo_status apollo_dg_stage_end(apollo_dg* h, int stage, apollo_precision prec) {
-  apollo_status r = check_ready(h);
+  apollo_status r = check_ready(h, false);
   if (r) return r;
   if (h->lim_on) return fail(h, APOLLO_ERR_CONFIG, "partitioned meshes do not support the limiter");
   if (stage < 0 || stage > 4) return APOLLO_ERR_ARG;
@@ -1900,12 +1917,13 @@ apollo_status apollo_dg_stage_end(apollo_dg* h, int stage, apollo_precision prec
   } else {
     const int blk = h->ops.Ng * h->M * (int)sizeof(double);
     CK(launch_halo_blocks(h->hrecv, h->trace_d, h->halo_dst_d, h->n_recv, blk, true, h->stream), "halo unpack");
-    if (h->peers.empty()) {
+    if (!h->side_busy) {
       CK(launch_stage64(h->eq, d, a, nullptr, 0, h->stream), "stage launch");
     } else {
       // the elements with a cut face; they share no output with the others
       CK(launch_stage64(h->eq, d, a, h->elist_d + h->nel_int, h->K - h->nel_int, h->stream), "cut stage launch");
-      if (h->nel_int > 0) CK(cudaStreamWaitEvent(h->stream, h->ev_interior, 0), "stage event");
+      r = join_side(h);
+      if (r) return r;
     }
   }
   if (stage == 4 && h->hlam)
