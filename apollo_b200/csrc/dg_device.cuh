@@ -170,8 +170,9 @@ cudaError_t launch_rhs_fp64(int eq, const DgDev& d, const StageArgs& a, cudaStre
 // the fused float64 stage (dg_stage64.cu) on the elements of `list` (nullptr:
 // all); x and out must not overlap; the caller clears the wave-speed word
 // before a MODE_RHS launch (a MODE_STAGE launch with reset_lambda clears it for
-// the MODE_FINAL one that follows)
-cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s);
+// the MODE_FINAL one that follows).  spare: SMs left to other work
+cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s,
+                           int spare = 0);
 // the nodes on the cut faces (3 k + f) of x into blocks dst [n][NG M]
 cudaError_t launch_cut_nodes(int eq, const DgDev& d, const double* x, const int* blocks, int n, double* dst,
                              cudaStream_t s);

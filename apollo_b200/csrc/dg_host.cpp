@@ -1858,6 +1858,16 @@ apollo_status apollo_dg_dist_start(apollo_dg* h, double t, double dt, apollo_pre
 }
 
 namespace {
+// SMs that the elements without a cut face leave to the exchange and to the
+// elements with one.  A block of the float64 stage holds its SM's registers
+// until it has done all its tiles, so a kernel queued behind a launch on every
+// SM waits for the end of that launch.  Euler N = 4, a rank of 65,025 elements, a
+// copy queued 30 us behind the launch: done after 128 us with none, 60, 56, 54 us
+// with 4, 8, 16.  A staged step (exchange replaced by a local copy) with 0, 4, 8,
+// 16, 24: 608, 557, 565, 587, 631 us; 16,129 elements 258, 224, 201, 204, 238; HLL
+// 5 fields, N = 3, 16,129 elements 269, 207, 204, 208, 249.
+constexpr int kExchangeSms = 8;
+
 // the side stream, waiting for what the handle's stream holds now
 cudaError_t fork_side(apollo_dg* h) {
   cudaError_t e = cudaSuccess;
@@ -1894,7 +1904,7 @@ apollo_status apollo_dg_stage_begin(apollo_dg* h, int stage, apollo_precision pr
     CK(launch_cut_nodes(h->eq, d, a.x, h->halo_src_d, h->n_send, (double*)h->hsend, h->stream), "halo pack");
     if (h->nel_int > 0 && a.mode == MODE_STAGE) {
       CK(fork_side(h), "stage event");
-      CK(launch_stage64(h->eq, d, a, h->elist_d, h->nel_int, h->side_stream), "interior stage launch");
+      CK(launch_stage64(h->eq, d, a, h->elist_d, h->nel_int, h->side_stream, kExchangeSms), "interior stage launch");
       CK(cudaEventRecord(h->ev_interior, h->side_stream), "stage event");
       h->side_busy = true;
     }

@@ -430,7 +430,7 @@ cudaError_t cut_nodes_n(const DgDev& d, const double* x, const int* blocks, int 
 }
 
 template <int EQ, int N, bool GF>
-cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s) {
+cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s, int spare) {
   using T = Chain<EQ, N>;
   static unsigned configured = 0;  // bit per device
   int dev = 0;
@@ -445,6 +445,7 @@ cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nl
   if (n <= 0) return cudaSuccess;
   int sms = device_sms();
   if (d.grid_div > 1) sms = (sms + d.grid_div - 1) / d.grid_div;
+  if (sms > spare) sms -= spare;
   // one block per SM with as many warps as its share of the tiles needs (a
   // warp without a tile would only hold registers): the smallest meshes run
   // one tile per warp on as many SMs as there are tiles
@@ -455,30 +456,31 @@ cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nl
 }
 
 template <int EQ, bool GF>
-cudaError_t dispatch_n(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s) {
+cudaError_t dispatch_n(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s, int spare) {
   switch (d.N) {
-    case 2: return launch_t<EQ, 2, GF>(d, a, list, nlist, s);
-    case 3: return launch_t<EQ, 3, GF>(d, a, list, nlist, s);
-    case 4: return launch_t<EQ, 4, GF>(d, a, list, nlist, s);
-    case 5: return launch_t<EQ, 5, GF>(d, a, list, nlist, s);
+    case 2: return launch_t<EQ, 2, GF>(d, a, list, nlist, s, spare);
+    case 3: return launch_t<EQ, 3, GF>(d, a, list, nlist, s, spare);
+    case 4: return launch_t<EQ, 4, GF>(d, a, list, nlist, s, spare);
+    case 5: return launch_t<EQ, 5, GF>(d, a, list, nlist, s, spare);
     default: return cudaErrorInvalidValue;
   }
 }
 
 }  // namespace
 
-cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s) {
+cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s,
+                           int spare) {
   const int kind = (int)d.eqp.p[3];
   const bool gf = kind == NF_HLL || kind == NF_ROE || kind == NF_WAVE;  // Euler kinds only
   switch (eq) {
-    case EQ_ADVECTION: return dispatch_n<EQ_ADVECTION, false>(d, a, list, nlist, s);
+    case EQ_ADVECTION: return dispatch_n<EQ_ADVECTION, false>(d, a, list, nlist, s, spare);
     case EQ_EULER:
-      return gf ? dispatch_n<EQ_EULER, true>(d, a, list, nlist, s) : dispatch_n<EQ_EULER, false>(d, a, list, nlist, s);
-    case EQ_MAXWELL: return dispatch_n<EQ_MAXWELL, false>(d, a, list, nlist, s);
+      return gf ? dispatch_n<EQ_EULER, true>(d, a, list, nlist, s, spare) : dispatch_n<EQ_EULER, false>(d, a, list, nlist, s, spare);
+    case EQ_MAXWELL: return dispatch_n<EQ_MAXWELL, false>(d, a, list, nlist, s, spare);
     case EQ_EULER2D:
-      return gf ? dispatch_n<EQ_EULER2D, true>(d, a, list, nlist, s)
-                : dispatch_n<EQ_EULER2D, false>(d, a, list, nlist, s);
-    case EQ_MAXWELL_TM: return dispatch_n<EQ_MAXWELL_TM, false>(d, a, list, nlist, s);
+      return gf ? dispatch_n<EQ_EULER2D, true>(d, a, list, nlist, s, spare)
+                : dispatch_n<EQ_EULER2D, false>(d, a, list, nlist, s, spare);
+    case EQ_MAXWELL_TM: return dispatch_n<EQ_MAXWELL_TM, false>(d, a, list, nlist, s, spare);
     default: return cudaErrorInvalidValue;
   }
 }
