@@ -46,10 +46,13 @@ __device__ __forceinline__ double rsqrt_normal(double x) {
 // of the reference's clamps and whose density and pressure lie between 2^-500
 // and 2^500 (checked on the high words, so that the float64 pipe does not
 // compare); any other state takes the equation's own code, which applies the
-// clamps and raises its error flags.
+// clamps and raises its error flags.  The density's bound comes from the host:
+// formed here from the floor's high word, two of the kernels (HLL with 4 fields
+// at order 2, with 5 at order 5) found sound states below it and ran at half
+// their rate.
 template <int MF> struct EulerFast64 {
   static constexpr int IE = MF - 1;
-  static constexpr int LO = 0x20b00000, HI = 0x5f300000;  // high words of 2^-500 and 2^500
+  static constexpr int LO = kWordLo, HI = kWordHi;
   struct Side {
     double rho, ir, vx, vy, vz, v2, p;
     bool clean;
@@ -59,8 +62,6 @@ template <int MF> struct EulerFast64 {
   }
   __device__ __forceinline__ static Side side(const EqParams& P, const double* q) {
     const double g1 = P.p[0] - 1.0;
-    // a density whose high word is above the floor's is above the floor
-    const int lo = min(max(__double2hiint(P.p[2]) + 1, LO), HI);
     Side s;
     s.rho = q[0];
     s.ir = recip_normal(s.rho);
@@ -70,7 +71,7 @@ template <int MF> struct EulerFast64 {
     // 1e-300 keeps the speed's square root off zero and changes no other sum
     s.v2 = fma(s.vx, s.vx, fma(s.vy, s.vy, MF == 5 ? fma(s.vz, s.vz, 1e-300) : 1e-300));
     s.p = g1 * fma(-0.5 * s.rho, s.v2, q[IE]);
-    s.clean = within(s.rho, lo) && within(s.p, LO);
+    s.clean = within(s.rho, P.rho_lo) && within(s.p, LO);
     return s;
   }
   // the flux along (ax, ay): ax F + ay G

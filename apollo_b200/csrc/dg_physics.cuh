@@ -6,6 +6,7 @@
 #pragma once
 
 #include <math.h>
+#include <string.h>
 
 #if defined(__CUDACC__)
 #define APOLLO_HD __host__ __device__ __forceinline__
@@ -45,7 +46,19 @@ constexpr int kMaxBc = 8;
 
 struct EqParams {
   double p[4];  // advection: ux uy uz; Euler: gamma minP minD; Maxwell: c0 gamma chi
+  int rho_lo;   // the Euler fast fluxes' least high word of a density (density_word, set for the device)
 };
+
+// Densities and pressures that the float64 Euler kernels' own flux code takes
+// (dg_flux64.cuh) have high words in [kWordLo, kWordHi): 2^-500 to 2^500.  A
+// density's must also lie above the floor's high word.
+constexpr int kWordLo = 0x20b00000, kWordHi = 0x5f300000;
+inline int density_word(double min_density) {
+  long long bits;
+  memcpy(&bits, &min_density, sizeof bits);
+  const int above = (int)(bits >> 32) + 1;
+  return above < kWordLo ? kWordLo : above > kWordHi ? kWordHi : above;
+}
 
 struct BcTable {
   int n;
