@@ -131,6 +131,64 @@ template <int MF> struct EulerFast64 {
     *lam = la > lb ? la : lb;
     return true;
   }
+  // twice Apollo's Roe flux of two clean states times w (wxeulereqn.cc:1206-1275:
+  // the first momentum component assigned twice, no second and no z one); false
+  // as for hll2
+  __device__ __forceinline__ static bool roe2(const EqParams& P, const Side& a, const Side& b, const double* qM,
+                                              const double* qP, double nx, double ny, double w, double* nf,
+                                              double* lam) {
+    const double gamma = P.p[0];
+    const double ua = nx * a.vx + ny * a.vy, ub = nx * b.vx + ny * b.vy;
+    const double ta = nx * a.vy - ny * a.vx, tb = nx * b.vy - ny * b.vx;
+    const double ra = sqrt_normal(a.rho), rb = sqrt_normal(b.rho), ri = recip_normal(ra + rb);
+    const double ea = qM[IE] + a.p, eb = qP[IE] + b.p;
+    const double u = (ra * ua + rb * ub) * ri, t = (ra * ta + rb * tb) * ri;
+    const double z = MF == 5 ? (ra * a.vz + rb * b.vz) * ri : 0.0;
+    const double H = (ra * (ea * a.ir) + rb * (eb * b.ir)) * ri;
+    const double c2 = (gamma - 1.0) * (H - 0.5 * (u * u + t * t + z * z));
+    if (!within(c2, LO)) return false;
+    const double ic = rsqrt_normal(c2), c = c2 * ic, rho = ra * rb;
+    const double du = 0.5 * rho * (ub - ua) * ic, dp = 0.5 * (b.p - a.p) * (ic * ic);
+    const double w1 = fabs(u - c) * (dp - du), w2 = fabs(u) * ((b.rho - a.rho) - 2.0 * dp);
+    const double w3 = fabs(u) * (rho * (tb - ta)), w4 = fabs(u + c) * (dp + du), ws = w1 + w2 + w4;
+    const double na = nx * qM[1] + ny * qM[2], nb = nx * qP[1] + ny * qP[2];
+    const double sa = nx * qM[2] - ny * qM[1], sb = nx * qP[2] - ny * qP[1];
+    const double f1 = (fma(na, ua, a.p) + fma(nb, ub, b.p)) - (w1 * (u - c) + w2 * u + w4 * (u + c));
+    const double f2 = (sa * ua + sb * ub) - (ws * t + w3);
+    nf[0] = w * ((na + nb) - ws);
+    nf[1] = w * (ny * f1 + nx * f2);
+    nf[2] = 0.0;
+    if (MF == 5) nf[3] = 0.0;
+    nf[IE] = w * ((ea * ua + eb * ub) -
+                  (w1 * (H - u * c) + w2 * (0.5 * (u * u + t * t)) + w3 * t + w4 * (H + u * c)));
+    const double la = speed(P, a), lb = speed(P, b);
+    *lam = la > lb ? la : lb;
+    return true;
+  }
+  // twice what remains of Apollo's Wave flux (wxeulereqn.cc:888-892, :1279-1322)
+  // of two clean states times w: Lax-Friedrichs of the rotated traces with the
+  // unrotated normal; its checks and its pressure floor do not touch states that
+  // pass wave_ok
+  __device__ __forceinline__ static bool wave_ok(const EqParams& P, const Side& s, const double* q) {
+    // a pressure 2^40 below the energy is rounding, and so are the checks on it
+    return s.p >= P.p[1] && __double2hiint(q[IE]) - __double2hiint(s.p) < (40 << 20);
+  }
+  __device__ __forceinline__ static double wave2(const EqParams& P, Side a, Side b, const double* qM, const double* qP,
+                                                 double nx, double ny, double w, double* nf) {
+    double rM[MF], rP[MF];
+    rotate(a, qM, nx, ny, rM);
+    rotate(b, qP, nx, ny, rP);
+    return lf2(P, a, b, rM, rP, w * nx, w * ny, w, nf);
+  }
+  __device__ __forceinline__ static void rotate(Side& s, const double* q, double nx, double ny, double* r) {
+#pragma unroll
+    for (int f = 0; f < MF; ++f) r[f] = q[f];
+    r[1] = nx * q[1] + ny * q[2];
+    r[2] = nx * q[2] - ny * q[1];
+    const double u = nx * s.vx + ny * s.vy;
+    s.vy = nx * s.vy - ny * s.vx;
+    s.vx = u;
+  }
   // qb = (d (aR . R + aS . S) / d q)^T of the fluxes R along (rx, ry), S along
   // (sx, sy): with cF = rx aR + sx aS, cG = ry aR + sy aS the reverse sweep of
   // cF . F + cG . G, F = (m1, m1 vx + p, m1 vy, (E + p) vx) and so on
@@ -413,18 +471,29 @@ __device__ __forceinline__ void volume_flux_pair(const EqParams& P, const double
 }
 
 // Twice the numerical flux of one face point (qM, qP may be modified as the
-// reference modifies them) times w.  GF: any numerical flux; otherwise the
-// Euler flux is Lax-Friedrichs.
-template <int EQ, bool GF>
+// reference modifies them) times w, by the equation's own code but for
+// Lax-Friedrichs.  KIND: the numerical flux, or kAnyFlux.
+constexpr int kAnyFlux = -1;
+template <int EQ, int KIND>
 __device__ __forceinline__ double face_flux2(const EqParams& P, double nx, double ny, double w, double* qM, double* qP,
                                              double* nf, int* err) {
   constexpr int M = Eq<EQ>::M;
   double lam;
-  if constexpr (kEulerEq<EQ> && !GF) {
-    using X = EulerFast64<M>;
-    const typename X::Side a = X::side(P, qM), b = X::side(P, qP);
-    if (a.clean && b.clean) return X::lf2(P, a, b, qM, qP, w * nx, w * ny, w, nf);
-    lam = Eq<EQ>::lf(P, nx, ny, qM, qP, nf, err);
+  if constexpr (kEulerEq<EQ> && KIND != kAnyFlux) {
+    if constexpr (KIND == NF_HLL) {
+      lam = Eq<EQ>::hll(P, nx, ny, qM, qP, nf, err);
+    } else if constexpr (KIND == NF_ROE) {
+      lam = Eq<EQ>::roe(P, nx, ny, qM, qP, nf, err);
+    } else {
+      if constexpr (KIND == NF_WAVE) {
+        Eq<EQ>::wave_prelude(P, nx, ny, qM, qP, err);
+      } else {
+        using X = EulerFast64<M>;
+        const typename X::Side a = X::side(P, qM), b = X::side(P, qP);
+        if (a.clean && b.clean) return X::lf2(P, a, b, qM, qP, w * nx, w * ny, w, nf);
+      }
+      lam = Eq<EQ>::lf(P, nx, ny, qM, qP, nf, err);
+    }
   } else {
     lam = Eq<EQ>::numflux(P, nx, ny, qM, qP, nf, err);
   }
@@ -434,7 +503,7 @@ __device__ __forceinline__ double face_flux2(const EqParams& P, double nx, doubl
 }
 
 // The same for two points of one face: one branch for both
-template <int EQ, bool GF>
+template <int EQ, int KIND>
 __device__ __forceinline__ void face_flux2_pair(const EqParams& P, double nx, double ny, double w,
                                                 double (*qM)[Eq<EQ>::M], double (*qP)[Eq<EQ>::M],
                                                 double (*nf)[Eq<EQ>::M], double* lam, int* err) {
@@ -443,22 +512,32 @@ __device__ __forceinline__ void face_flux2_pair(const EqParams& P, double nx, do
     const typename X::Side a0 = X::side(P, qM[0]), b0 = X::side(P, qP[0]);
     const typename X::Side a1 = X::side(P, qM[1]), b1 = X::side(P, qP[1]);
     const bool clean = a0.clean && b0.clean && a1.clean && b1.clean;
-    if constexpr (!GF) {
+    if constexpr (KIND == NF_HLL) {
+      if (clean && (X::hll2(P, a0, b0, qM[0], qP[0], nx, ny, w, nf[0], &lam[0]) &
+                    X::hll2(P, a1, b1, qM[1], qP[1], nx, ny, w, nf[1], &lam[1])))
+        return;
+    } else if constexpr (KIND == NF_ROE) {
+      if (clean && (X::roe2(P, a0, b0, qM[0], qP[0], nx, ny, w, nf[0], &lam[0]) &
+                    X::roe2(P, a1, b1, qM[1], qP[1], nx, ny, w, nf[1], &lam[1])))
+        return;
+    } else if constexpr (KIND == NF_WAVE) {
+      if (clean && X::wave_ok(P, a0, qM[0]) && X::wave_ok(P, b0, qP[0]) && X::wave_ok(P, a1, qM[1]) &&
+          X::wave_ok(P, b1, qP[1])) {
+        lam[0] = X::wave2(P, a0, b0, qM[0], qP[0], nx, ny, w, nf[0]);
+        lam[1] = X::wave2(P, a1, b1, qM[1], qP[1], nx, ny, w, nf[1]);
+        return;
+      }
+    } else {
       if (clean) {
         const double nxw = w * nx, nyw = w * ny;
         lam[0] = X::lf2(P, a0, b0, qM[0], qP[0], nxw, nyw, w, nf[0]);
         lam[1] = X::lf2(P, a1, b1, qM[1], qP[1], nxw, nyw, w, nf[1]);
         return;
       }
-    } else {
-      if (clean && (int)P.p[3] == NF_HLL &&
-          (X::hll2(P, a0, b0, qM[0], qP[0], nx, ny, w, nf[0], &lam[0]) &
-           X::hll2(P, a1, b1, qM[1], qP[1], nx, ny, w, nf[1], &lam[1])))
-        return;
     }
   }
 #pragma unroll
-  for (int j = 0; j < 2; ++j) lam[j] = face_flux2<EQ, GF>(P, nx, ny, w, qM[j], qP[j], nf[j], err);
+  for (int j = 0; j < 2; ++j) lam[j] = face_flux2<EQ, KIND>(P, nx, ny, w, qM[j], qP[j], nf[j], err);
 }
 
 // The source plugins at one point (Apollo adds each into its output field,

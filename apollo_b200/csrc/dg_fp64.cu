@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(kThreads) k_face(DgDev d, StageArgs a) {
     }
     const int kind = (int)d.eqp.p[3];
     const double lam = kind == NF_HLL || kind == NF_ROE || kind == NF_WAVE
-                           ? face_flux2<EQ, true>(d.eqp, nx, ny, 0.5, qM, qP, nf, &err)
-                           : face_flux2<EQ, false>(d.eqp, nx, ny, 0.5, qM, qP, nf, &err);
+                           ? face_flux2<EQ, kAnyFlux>(d.eqp, nx, ny, 0.5, qM, qP, nf, &err)
+                           : face_flux2<EQ, NF_LF>(d.eqp, nx, ny, 0.5, qM, qP, nf, &err);
     lam_acc.add(d.st, inst, fabs(lam));
     const double w = d.gw[gq] * sJ;
     store_point<M>(d.flux + ((size_t)fr.k1 * NF + fr.f1 * NG + gq) * M, nf, w);
@@ -594,11 +594,9 @@ int fp64_supported(int eq, int N) { return eq >= 0 && eq <= 4 && N >= 2 && N <= 
 // rule knows no mesh size or flux, so that batches and partitions compute the
 // whole mesh's bits.  A right-hand side, three kernels and fused: Euler N = 2,
 // K = 130,050 168 and 87 us, N = 5 572 and 329; 8 fields N = 3, K = 32,258 129
-// and 39; HLL 5 fields N = 3, K = 50,562 260 and 84; Wave the same 304 and 181.
-// The three kernels stay faster for Roe and Wave below one wave of tiles (5
-// fields, N = 3, K = 2,048: Roe 41 and 46, Wave 48 and 52; N = 5 51 and 63), for
-// Roe with 4 fields at orders 2 and 5, and for HLL below a wave with 5 fields at
-// order 5 (57 and 65) and 4 at order 2 (37 and 39).
+// and 39; K = 2,048, 16,200 and 50,562 with 5 fields, N = 3: HLL 43, 94, 260 and
+// 24, 40, 84; Roe 38, 84, 213 and 24, 40, 83; Wave 47, 106, 306 and 25, 38, 77.  Over
+// fluxes, orders and field counts it takes 0.84 of the three kernels' time at most.
 static bool fused_applies(int eq, const DgDev& d, const StageArgs& a) {
   if (d.fp64_fused == 0) return false;
   if (d.fp64_fused == 2 && (d.K + 7) / 8 > stage64_wave_tiles(eq, d.N, num_sms())) return false;

@@ -50,7 +50,7 @@ namespace apollo {
 namespace {
 
 // Sizes of the chain for one equation and order (doubles unless said).
-template <int EQ, int N> struct Chain {
+template <int EQ, int N, int KIND> struct Chain {
   static constexpr int M = Eq<EQ>::M;
   static constexpr int NP = Sizes<N>::NP, NC = Sizes<N>::NC, NG = Sizes<N>::NG, NF = Sizes<N>::NF;
   static constexpr bool LIN = kLinearEq<EQ>;
@@ -76,19 +76,27 @@ template <int EQ, int N> struct Chain {
   static constexpr bool BULK = NP * M >= 30;
   static constexpr int WARP = XB * (X + G) + PN + C;
   static constexpr size_t bytes(int warps) { return sizeof(double) * (size_t)(SHARED + warps * WARP); }
-  // warps per block (one block per SM): what registers and shared memory allow
+  // Warps per block (one block per SM): what registers and shared memory allow.
+  // Sixteen have 128 registers a lane, and the Euler kernels then spill 110 to
+  // 720 bytes; eight spill nothing.  The spills cost less than the missing warps
+  // on large meshes, more on small ones, and the longest bodies (HLL and Roe, 5
+  // fields, orders 3 and 4) gain from eight at every size.  A right-hand side, K =
+  // 2,048, 16,200, 50,562, with eight and with sixteen: Lax-Friedrichs N = 4, 4
+  // fields 25, 44, 93 and 26, 42, 88 us, 5 fields 27, 52, 116 and 29, 50, 112; HLL
+  // N = 3, 4 fields 26, 39, 76 and 27, 39, 74, 5 fields 24, 40, 84 and 29, 41, 87.
   static constexpr int fit(int w) { return bytes(w) <= 227 * 1024 ? w : fit(w - 1); }
-  static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : (N >= 5 ? 8 : 16));
+  static constexpr bool LONG = M == 5 && N >= 3 && (KIND == NF_HLL || KIND == NF_ROE);
+  static constexpr int WMAX = fit(LIN ? (M == 8 ? 8 : 16) : (N >= 5 || LONG ? 8 : 16));
 };
 
 // One SSPRK stage (or right-hand side).  Reads the neighbours of x: x and out
 // must not overlap.  `list` (nlist entries) names the elements of this launch;
-// nullptr: all of them.  GF: the Euler flux is HLL, Roe or Wave (a kernel of its
-// own, so that their code does not take registers from the others).
-template <int EQ, int N, bool GF>
-__global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
+// nullptr: all of them.  KIND: the Euler numerical flux (a kernel of its own, so
+// that the others' code takes no registers from it).
+template <int EQ, int N, int KIND>
+__global__ void __launch_bounds__(32 * Chain<EQ, N, KIND>::WMAX, 1)
     k_stage64(DgDev d, StageArgs a, const int* __restrict__ list, int nlist) {
-  using T = Chain<EQ, N>;
+  using T = Chain<EQ, N, KIND>;
   using PK = Pack64<N>;
   using P = Eq<EQ>;
   constexpr int M = T::M, NP = T::NP, NG = T::NG, NF = T::NF;
@@ -340,7 +348,7 @@ __global__ void __launch_bounds__(32 * Chain<EQ, N>::WMAX, 1)
 #pragma unroll
           for (int j = 0; j < 2; ++j) ghost_state(-cn.x, fc, sGz[g0 + j], qM[j], qP[j]);
         }
-        face_flux2_pair<EQ, GF>(d.eqp, ge[6 + fc], ge[9 + fc], miJ * ge[12 + fc], qM, qP, A, lam, &err);
+        face_flux2_pair<EQ, KIND>(d.eqp, ge[6 + fc], ge[9 + fc], miJ * ge[12 + fc], qM, qP, A, lam, &err);
         if (want_lam) {
           lam_acc.add(d.st, inst, fabs(lam[0]));
           lam_acc.add(d.st, inst, fabs(lam[1]));
@@ -429,14 +437,14 @@ cudaError_t cut_nodes_n(const DgDev& d, const double* x, const int* blocks, int 
   return cudaGetLastError();
 }
 
-template <int EQ, int N, bool GF>
+template <int EQ, int N, int KIND>
 cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s, int spare) {
-  using T = Chain<EQ, N>;
+  using T = Chain<EQ, N, KIND>;
   static unsigned configured = 0;  // bit per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(configured & (1u << (dev & 31)))) {
-    cudaError_t e = cudaFuncSetAttribute(k_stage64<EQ, N, GF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_stage64<EQ, N, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)T::bytes(T::WMAX));
     if (e != cudaSuccess) return e;
     configured |= 1u << (dev & 31);
@@ -452,17 +460,27 @@ cudaError_t launch_t(const DgDev& d, const StageArgs& a, const int* list, int nl
   const int tiles = (n + 7) / 8, grid = tiles < sms ? tiles : sms;
   int warps = (tiles + grid - 1) / grid;
   if (warps > T::WMAX) warps = T::WMAX;
-  return launch_kernel(k_stage64<EQ, N, GF>, grid, 32 * warps, T::bytes(warps), s, a.overlap != 0, d, a, list, nlist);
+  return launch_kernel(k_stage64<EQ, N, KIND>, grid, 32 * warps, T::bytes(warps), s, a.overlap != 0, d, a, list, nlist);
 }
 
-template <int EQ, bool GF>
+template <int EQ, int KIND>
 cudaError_t dispatch_n(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s, int spare) {
   switch (d.N) {
-    case 2: return launch_t<EQ, 2, GF>(d, a, list, nlist, s, spare);
-    case 3: return launch_t<EQ, 3, GF>(d, a, list, nlist, s, spare);
-    case 4: return launch_t<EQ, 4, GF>(d, a, list, nlist, s, spare);
-    case 5: return launch_t<EQ, 5, GF>(d, a, list, nlist, s, spare);
+    case 2: return launch_t<EQ, 2, KIND>(d, a, list, nlist, s, spare);
+    case 3: return launch_t<EQ, 3, KIND>(d, a, list, nlist, s, spare);
+    case 4: return launch_t<EQ, 4, KIND>(d, a, list, nlist, s, spare);
+    case 5: return launch_t<EQ, 5, KIND>(d, a, list, nlist, s, spare);
     default: return cudaErrorInvalidValue;
+  }
+}
+
+template <int EQ>
+cudaError_t dispatch_kind(const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s, int spare) {
+  switch ((int)d.eqp.p[3]) {
+    case NF_HLL: return dispatch_n<EQ, NF_HLL>(d, a, list, nlist, s, spare);
+    case NF_ROE: return dispatch_n<EQ, NF_ROE>(d, a, list, nlist, s, spare);
+    case NF_WAVE: return dispatch_n<EQ, NF_WAVE>(d, a, list, nlist, s, spare);
+    default: return dispatch_n<EQ, NF_LF>(d, a, list, nlist, s, spare);
   }
 }
 
@@ -470,17 +488,12 @@ cudaError_t dispatch_n(const DgDev& d, const StageArgs& a, const int* list, int 
 
 cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int* list, int nlist, cudaStream_t s,
                            int spare) {
-  const int kind = (int)d.eqp.p[3];
-  const bool gf = kind == NF_HLL || kind == NF_ROE || kind == NF_WAVE;  // Euler kinds only
   switch (eq) {
-    case EQ_ADVECTION: return dispatch_n<EQ_ADVECTION, false>(d, a, list, nlist, s, spare);
-    case EQ_EULER:
-      return gf ? dispatch_n<EQ_EULER, true>(d, a, list, nlist, s, spare) : dispatch_n<EQ_EULER, false>(d, a, list, nlist, s, spare);
-    case EQ_MAXWELL: return dispatch_n<EQ_MAXWELL, false>(d, a, list, nlist, s, spare);
-    case EQ_EULER2D:
-      return gf ? dispatch_n<EQ_EULER2D, true>(d, a, list, nlist, s, spare)
-                : dispatch_n<EQ_EULER2D, false>(d, a, list, nlist, s, spare);
-    case EQ_MAXWELL_TM: return dispatch_n<EQ_MAXWELL_TM, false>(d, a, list, nlist, s, spare);
+    case EQ_ADVECTION: return dispatch_n<EQ_ADVECTION, NF_LF>(d, a, list, nlist, s, spare);
+    case EQ_EULER: return dispatch_kind<EQ_EULER>(d, a, list, nlist, s, spare);
+    case EQ_MAXWELL: return dispatch_n<EQ_MAXWELL, NF_LF>(d, a, list, nlist, s, spare);
+    case EQ_EULER2D: return dispatch_kind<EQ_EULER2D>(d, a, list, nlist, s, spare);
+    case EQ_MAXWELL_TM: return dispatch_n<EQ_MAXWELL_TM, NF_LF>(d, a, list, nlist, s, spare);
     default: return cudaErrorInvalidValue;
   }
 }
