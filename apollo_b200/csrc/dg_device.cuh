@@ -176,8 +176,8 @@ cudaError_t launch_stage64(int eq, const DgDev& d, const StageArgs& a, const int
 // the nodes on the cut faces (3 k + f) of x into blocks dst [n][NG M]
 cudaError_t launch_cut_nodes(int eq, const DgDev& d, const double* x, const int* blocks, int n, double* dst,
                              cudaStream_t s);
-int stage64_wave_tiles(int eq, int N, int sms);  // tiles (of 8 elements) of one resident wave
-int device_sms();                                // SMs of the current device
+int stage64_wave_tiles(int eq, const DgDev& d, int sms);  // tiles (of 8 elements) of one resident wave
+int device_sms();                                         // SMs of the current device
 // k_lift alone on d.vol / d.flux (used by the tangent of a stage)
 cudaError_t launch_lift_fp64(int eq, const DgDev& d, const StageArgs& a, cudaStream_t s);
 cudaError_t launch_init_speed(int eq, const DgDev& d, const double* u, cudaStream_t s);

@@ -599,7 +599,7 @@ int fp64_supported(int eq, int N) { return eq >= 0 && eq <= 4 && N >= 2 && N <= 
 // fluxes, orders and field counts it takes 0.84 of the three kernels' time at most.
 static bool fused_applies(int eq, const DgDev& d, const StageArgs& a) {
   if (d.fp64_fused == 0) return false;
-  if (d.fp64_fused == 2 && (d.K + 7) / 8 > stage64_wave_tiles(eq, d.N, num_sms())) return false;
+  if (d.fp64_fused == 2 && (d.K + 7) / 8 > stage64_wave_tiles(eq, d, num_sms())) return false;
   if (((uintptr_t)a.x | (uintptr_t)a.out | (uintptr_t)a.u0) % 16) return false;
   const size_t nbytes = (size_t)d.K * ((d.N + 1) * (d.N + 2) / 2) * eq_fields(eq) * sizeof(double);
   const char *xb = (const char*)a.x, *ob = (const char*)a.out;

@@ -511,10 +511,35 @@ cudaError_t launch_cut_nodes(int eq, const DgDev& d, const double* x, const int*
   }
 }
 
-// warps of one wave of k_stage64 (the launch-bound limit of form 2)
-int stage64_wave_tiles(int eq, int N, int sms) {
-  const int w = (eq == EQ_EULER || eq == EQ_EULER2D) ? (N >= 5 ? 8 : 16) : eq == EQ_MAXWELL ? 8 : 16;
-  return sms * w;
+namespace {
+template <int EQ, int KIND> int warps_n(int N) {
+  switch (N) {
+    case 2: return Chain<EQ, 2, KIND>::WMAX;
+    case 3: return Chain<EQ, 3, KIND>::WMAX;
+    case 4: return Chain<EQ, 4, KIND>::WMAX;
+    case 5: return Chain<EQ, 5, KIND>::WMAX;
+    default: return 0;
+  }
+}
+template <int EQ> int warps_kind(int N, int kind) {
+  return kind == NF_HLL    ? warps_n<EQ, NF_HLL>(N)
+         : kind == NF_ROE  ? warps_n<EQ, NF_ROE>(N)
+         : kind == NF_WAVE ? warps_n<EQ, NF_WAVE>(N)
+                           : warps_n<EQ, NF_LF>(N);
+}
+}  // namespace
+
+// tiles of one wave of k_stage64 (the limit of form 2)
+int stage64_wave_tiles(int eq, const DgDev& d, int sms) {
+  const int kind = (int)d.eqp.p[3];
+  switch (eq) {
+    case EQ_ADVECTION: return sms * warps_n<EQ_ADVECTION, NF_LF>(d.N);
+    case EQ_EULER: return sms * warps_kind<EQ_EULER>(d.N, kind);
+    case EQ_MAXWELL: return sms * warps_n<EQ_MAXWELL, NF_LF>(d.N);
+    case EQ_EULER2D: return sms * warps_kind<EQ_EULER2D>(d.N, kind);
+    case EQ_MAXWELL_TM: return sms * warps_n<EQ_MAXWELL_TM, NF_LF>(d.N);
+    default: return 0;
+  }
 }
 
 }  // namespace apollo
