@@ -609,8 +609,9 @@ static bool fused_applies(int eq, const DgDev& d, const StageArgs& a) {
 cudaError_t launch_rhs_fp64(int eq, const DgDev& d, const StageArgs& a, cudaStream_t s, cudaEvent_t* ev) {
   if (fused_applies(eq, d, a)) {
     if (ev) cudaEventRecord(ev[0], s);
-    if (a.reset_lambda && a.mode == MODE_RHS) launch_reset_lambda(d, s);
-    const cudaError_t e = launch_stage64(eq, d, a, nullptr, 0, s);
+    cudaError_t e = cudaSuccess;
+    if (a.reset_lambda && a.mode == MODE_RHS) e = launch_reset_lambda(d, s);
+    if (e == cudaSuccess) e = launch_stage64(eq, d, a, nullptr, 0, s);
     if (ev)
       for (int i = 1; i < 4; ++i) cudaEventRecord(ev[i], s);
     return e;

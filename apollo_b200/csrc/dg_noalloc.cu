@@ -100,8 +100,9 @@ extern "C" apollo_status apollo_dg_rhs_noalloc(apollo_dg* h, double t, double dt
     }
   }
   unsigned char* p = (unsigned char*)base;
-  // per-call state starts at zero (wave-speed maximum, error word); the three
-  // arrays are written in full by the kernels before they are read
+  // per-call state starts at zero (wave-speed maximum, error word: no kernel
+  // clears them again); the three arrays are written in full by the kernels
+  // before they are read
   d.st = (DevState*)p;
   d.einst = nullptr;  // one DevState in the array's header: a single instance
   d.ninst = 1;
@@ -116,7 +117,6 @@ extern "C" apollo_status apollo_dg_rhs_noalloc(apollo_dg* h, double t, double dt
   a.time_from_state = 0;
   a.t_arg = t;
   a.dt_arg = dt;
-  a.reset_lambda = 1;
   if (launch_rhs_fp64(eq, d, a, s) != cudaSuccess) {
     handle_set_error(h, "apollo_dg_rhs_noalloc: kernel launch failed");
     return APOLLO_ERR_CUDA;
