@@ -15,7 +15,8 @@ namespace apollo {
 // Single Nonlinear Equation, 1970), which leaves e^3.  Error measured against the
 // correctly rounded operations over 1.5e9 numbers between 2^-400 and 2^400: at
 // most one unit in the last place (two for the reciprocal root, against the
-// rounded reciprocal of the rounded root).  Together with the tile prefetch and
+// rounded reciprocal of the rounded root); the test suite holds these bounds from
+// 2^-1000 to 2^1000.  Together with the tile prefetch and
 // one branch for a lane's two points they took a right-hand side of Euler N = 4,
 // K = 130,050 from 256 to 199 us, of HLL with 5 fields, N = 3, K = 32,258 from
 // 122 to 67.
@@ -43,9 +44,10 @@ __device__ __forceinline__ double rsqrt_normal(double x) {
 // the flux formed along a direction directly (a n.F + b n.G in one pass): the
 // same quantities as WxEulerEqn's flux and Lax-Friedrichs flux
 // (wxeulereqn.cc:809-871, :1097-1117) to round-off, for states that need none
-// of the reference's clamps and whose density and pressure lie between 2^-500
-// and 2^500 (checked on the high words, so that the float64 pipe does not
-// compare); any other state takes the equation's own code, which applies the
+// of the reference's clamps and whose density and pressure lie between 2^-400
+// and 2^400 (checked on the high words, so that the float64 pipe does not
+// compare; their quotient, the square of the sound speed up to gamma, then lies
+// far above the 1e-300 that keeps the flow speed's root off zero); any other state takes the equation's own code, which applies the
 // clamps and raises its error flags.  The density's bound comes from the host:
 // formed here from the floor's high word, two of the kernels (HLL with 4 fields
 // at order 2, with 5 at order 5) found sound states below it and ran at half
@@ -68,7 +70,8 @@ template <int MF> struct EulerFast64 {
     s.vx = q[1] * s.ir;
     s.vy = q[2] * s.ir;
     s.vz = MF == 5 ? q[3] * s.ir : 0.0;
-    // 1e-300 keeps the speed's square root off zero and changes no other sum
+    // 1e-300 keeps the speed's square root off zero and, with p / rho above
+    // 2^-800, changes no other sum
     s.v2 = fma(s.vx, s.vx, fma(s.vy, s.vy, MF == 5 ? fma(s.vz, s.vz, 1e-300) : 1e-300));
     s.p = g1 * fma(-0.5 * s.rho, s.v2, q[IE]);
     s.clean = within(s.rho, P.rho_lo) && within(s.p, LO);

@@ -50,9 +50,9 @@ struct EqParams {
 };
 
 // Densities and pressures that the float64 Euler kernels' own flux code takes
-// (dg_flux64.cuh) have high words in [kWordLo, kWordHi): 2^-500 to 2^500.  A
+// (dg_flux64.cuh) have high words in [kWordLo, kWordHi): 2^-400 to 2^400.  A
 // density's must also lie above the floor's high word.
-constexpr int kWordLo = 0x20b00000, kWordHi = 0x5f300000;
+constexpr int kWordLo = 0x26f00000, kWordHi = 0x58f00000;
 inline int density_word(double min_density) {
   long long bits;
   memcpy(&bits, &min_density, sizeof bits);
