@@ -683,6 +683,17 @@ def fp64_gemm_peak(device: int) -> float:
     return 2.0 * n ** 3 / best / 1e12
 
 
+def contraction_flops(prec: str, N: int, Np: int, Nc: int, Ng: int, m: int) -> int:
+    """FLOPs of the contractions that a stage of a Lax-Friedrichs Euler element runs (2 per
+    multiply-add, the pointwise fluxes not counted).  Both forms interpolate to the Nc
+    cubature points, take two derivatives there and lift from the 3 Ng face points; the
+    mixed form also contracts its own traces with all Np nodes, the float64 form sums both
+    sides' traces over the N + 1 nodes of the face."""
+    Nf = 3 * Ng
+    traces = Nf * Np if prec == "mixed" else 2 * Nf * (N + 1)
+    return 2 * m * (3 * Nc * Np + Nf * Np + traces)
+
+
 def profile_traffic():
     """DRAM bytes per launch of the dominant kernels from the committed ncu summary."""
     try:
@@ -1012,10 +1023,8 @@ def ours_arm(args):
         ms64 = timed("fp64", args.steps, args.warmup)
         extra["fp64"] = {"value": dofs * world * args.steps / (ms64 / 1000.0), "ms_per_step": ms64 / args.steps}
         try:
-            # the float64 stepper against the float64 pipe: Survey-8d contraction
-            # FLOPs, 2 m (3 Nc Np + 2 Nf Np + Np^2) per element per stage
-            Nc, Nf = s.Nc, 3 * s.Ng
-            flops = 5 * s.K * 2 * s.m * (3 * Nc * s.Np + 2 * Nf * s.Np + s.Np * s.Np)
+            # the float64 stepper's contractions against the float64 pipe
+            flops = 5 * s.K * contraction_flops("fp64", p.N, s.Np, s.Nc, s.Ng, s.m)
             ach = flops / (ms64 / args.steps / 1000.0) / 1e12
             pk = fp64_gemm_peak(local)
             extra["fp64"]["roofline"] = {"bound": "fp64", "achieved": ach, "peak": pk, "unit": "TFLOP/s",
@@ -1051,14 +1060,14 @@ def ours_arm(args):
         }
         alg_flops = {  # contraction flops (multiply-adds x2), pointwise flux excluded
             "traces": K * 2 * M * Nf * Np,
-            "stage": K * 2 * M * (3 * Nc * Np + 2 * Nf * Np + Np * Np),
+            "stage": K * contraction_flops("mixed", N, Np, Nc, Ng, M),
         }
         kt = kt[:2]
     else:
         # one launch per right-hand side
         names = ["stage_rhs"]
         alg_bytes = {"stage_rhs": K * (8 * 2 * Np * M + 160)}  # read x, write the RHS, geometry
-        alg_flops = {"stage_rhs": K * 2 * M * (3 * Nc * Np + 2 * Nf * Np + Np * Np)}
+        alg_flops = {"stage_rhs": K * contraction_flops("fp64", N, Np, Nc, Ng, M)}
         kt = kt[:1]
     dom = int(np.argmax(kt))
     dname = names[dom]
