@@ -49,9 +49,9 @@ __device__ __forceinline__ double rsqrt_normal(double x) {
 // compare; their quotient, the square of the sound speed up to gamma, then lies
 // far above the 1e-300 that keeps the flow speed's root off zero); any other state takes the equation's own code, which applies the
 // clamps and raises its error flags.  The density's bound comes from the host:
-// formed here from the floor's high word, two of the kernels (HLL with 4 fields
-// at order 2, with 5 at order 5) found sound states below it and ran at half
-// their rate.
+// formed here from the floor's high word, four of the kernels (HLL with 4 fields
+// at order 2 and with 5 at order 5, the tangent with 5 fields at orders 4 and 5)
+// found sound states below it and ran at half their rate.
 template <int MF> struct EulerFast64 {
   static constexpr int IE = MF - 1;
   static constexpr int LO = kWordLo, HI = kWordHi;

@@ -4,6 +4,8 @@ LIFT kernels give, for every flux, order and field count, and sound states stay
 on the fast fluxes (a right-hand side with the HLL flux then costs at most half
 as much again as with Lax-Friedrichs; with sound states on the general code it
 cost 1.9 times as much)."""
+import time
+
 import numpy as np
 import pytest
 
@@ -57,3 +59,25 @@ def _us(p, flux):
 def test_sound_states_take_the_fast_flux(fields, N):
     p = problems.euler_vortex(n=91, N=N, fields=fields)
     assert _us(p, "HLL") <= 1.5 * _us(p, "LF")
+
+
+@pytest.mark.parametrize("N", [4, 5])
+def test_sound_states_take_the_fast_tangent(N):
+    """The tangent of 5 fields against that of 4 (1.3 and 1.6 times as long; with
+    sound states differentiated through the equation's own code 2.6 and 3.2)."""
+    torch = pytest.importorskip("torch")
+    us = {}
+    for fields in (4, 5):
+        p = problems.euler_vortex(n=181, N=N, fields=fields)
+        s = NodalDG2d(p.N, p.cfl, p.equation, p.eq_params, p.mesh)
+        x, y = s.node_coords()
+        U = torch.from_numpy(np.ascontiguousarray(p.ic(x, y))).cuda()
+        v, out = torch.ones_like(U), torch.empty_like(U)
+        times = []
+        for _ in range(25):
+            t = time.perf_counter()
+            s.rhs_jvp(0.0, U, v, out)
+            times.append(time.perf_counter() - t)
+        us[fields] = np.median(times[5:])
+        s.close()
+    assert us[5] <= 2.0 * us[4]
