@@ -136,7 +136,9 @@ cudaError_t dev_malloc(void** p, size_t bytes) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
-  return cudaMalloc(p, bytes);
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by a later launch
+  return e;
 }
 
 #define CK(call, where)                          \
@@ -475,15 +477,15 @@ apollo_status apollo_dg_add_source(apollo_dg* h, const char* kind, const int* ou
     case EQ_MAXWELL_TM: f = a == 2 ? 0 : a == 3 ? 1 : a == 4 ? 2 : -1; break;
   }
   if (f < 0) return fail(h, APOLLO_ERR_CONFIG, "source output field " + std::to_string(a) + " is not a field of this equation");
+  if (h->K > 0 && h->mixed && !h->srcv_d) {
+    const size_t nU = (size_t)h->K * h->ops.Np * h->M;
+    CK(dev_malloc((void**)&h->srcv_d, nU * sizeof(double)), "source alloc");
+  }
   const int i = h->src.n;
   h->src.kind[i] = kd;
   h->src.out[i] = f;
   for (int j = 0; j < 9; ++j) h->src.p[i][j] = j < nparams ? params[j] : 0.0;
   h->src.n = i + 1;
-  if (h->K > 0 && h->mixed && !h->srcv_d) {
-    const size_t nU = (size_t)h->K * h->ops.Np * h->M;
-    CK(dev_malloc((void**)&h->srcv_d, nU * sizeof(double)), "source alloc");
-  }
   for (auto& g : h->graph)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   return APOLLO_OK;
@@ -620,11 +622,10 @@ apollo_status apollo_dg_set_limiter(apollo_dg* h, const char* kind, const double
   L.gamma = ta ? h->eqp.p[0] : params[0];
   L.minP = ta ? h->eqp.p[1] : params[1];
   L.minD = ta ? h->eqp.p[2] : params[2];
-  if (!h->lim_work_d) {
+  if (!h->lim_work_d)
     CK(dev_malloc((void**)&h->lim_work_d, limiter_work_doubles(h->K) * sizeof(double)), "limiter alloc");
-    CK(upload(&h->xn_d, h->xn.data(), h->xn.size()), "limiter coordinates");
-    CK(upload(&h->yn_d, h->yn.data(), h->yn.size()), "limiter coordinates");
-  }
+  if (!h->xn_d) CK(upload(&h->xn_d, h->xn.data(), h->xn.size()), "limiter coordinates");
+  if (!h->yn_d) CK(upload(&h->yn_d, h->yn.data(), h->yn.size()), "limiter coordinates");
   h->lim = L;
   h->lim_on = true;
   return APOLLO_OK;
@@ -1131,15 +1132,16 @@ apollo_status apollo_dg_kernel_times(apollo_dg* h, apollo_precision prec, int it
 namespace {
 
 apollo_status ensure_deriv_buffers(apollo_dg* h) {
-  if (h->dvol_d) return APOLLO_OK;
   const size_t nU = (size_t)h->K * h->ops.Np * h->M, nT = (size_t)h->K * h->ops.Nf * h->M;
-  CK(dev_malloc((void**)&h->dvol_d, nU * sizeof(double)), "derivative scratch");
-  CK(dev_malloc((void**)&h->dtrace_d, nT * sizeof(double)), "derivative scratch");
-  CK(dev_malloc((void**)&h->dflux_d, nT * sizeof(double)), "derivative scratch");
-  CK(dev_malloc((void**)&h->sbar_d, nT * sizeof(double)), "derivative scratch");
-  CK(dev_malloc((void**)&h->tU_d, nU * sizeof(double)), "derivative state");
-  CK(dev_malloc((void**)&h->tW_d, nU * sizeof(double)), "derivative state");
-  for (auto& p : h->A_d) CK(dev_malloc((void**)&p, nU * sizeof(double)), "adjoint state");
+  // each on its own: a call after one that ran out of memory allocates the rest
+  auto need = [](double*& p, size_t n) { return p ? cudaSuccess : dev_malloc((void**)&p, n * sizeof(double)); };
+  CK(need(h->dvol_d, nU), "derivative scratch");
+  CK(need(h->dtrace_d, nT), "derivative scratch");
+  CK(need(h->dflux_d, nT), "derivative scratch");
+  CK(need(h->sbar_d, nT), "derivative scratch");
+  CK(need(h->tU_d, nU), "derivative state");
+  CK(need(h->tW_d, nU), "derivative state");
+  for (auto& p : h->A_d) CK(need(p, nU), "adjoint state");
   return APOLLO_OK;
 }
 
@@ -1514,12 +1516,12 @@ apollo_status apollo_dg_forward_revolve(apollo_dg* h, int nsteps, double t0, dou
   if (!h->have_state) return fail(h, APOLLO_ERR_STATE, "no state set");
   // a slot per step already stores every state the sweep needs
   if (snapshots > nsteps) snapshots = nsteps;
+  h->tr_valid = false;  // the stored trajectory's buffers are resized
   r = ensure_deriv_buffers(h);
   if (!r) r = size_checkpoints(h, snapshots);
   if (!r) r = size_segment(h, 1);
   if (r) return r;
   const size_t nU = state_doubles(h);
-  h->tr_valid = false;
   h->tu_valid = false;
   r = clear_errors(h);
   if (r) return r;
@@ -1553,6 +1555,7 @@ apollo_status apollo_dg_forward_fixed(apollo_dg* h, int nsteps, double t0, doubl
   if (h->lim_on) return fail(h, APOLLO_ERR_CONFIG, "the derivatives do not support the limiter");
   if (nsteps < 1 || checkpoint_every < 1 || !(dt > 0.0)) return fail(h, APOLLO_ERR_ARG, "nsteps, checkpoint_every >= 1, dt > 0");
   if (!h->have_state) return fail(h, APOLLO_ERR_STATE, "no state set");
+  h->tr_valid = false;  // the stored trajectory's buffers are resized
   r = ensure_deriv_buffers(h);
   if (r) return r;
   const size_t nU = state_doubles(h);
@@ -1560,7 +1563,6 @@ apollo_status apollo_dg_forward_fixed(apollo_dg* h, int nsteps, double t0, doubl
   r = size_checkpoints(h, nck);
   if (!r) r = size_segment(h, checkpoint_every);
   if (r) return r;
-  h->tr_valid = false;
   h->tu_valid = false;
   r = clear_errors(h);
   if (r) return r;
