@@ -1844,14 +1844,21 @@ apollo_status apollo_dg_halo_bind(apollo_dg* h, void* send, size_t send_bytes, v
   return APOLLO_OK;
 }
 
+namespace {
+apollo_status check_halo(apollo_dg* h) {
+  if (!h->peers.empty() && (!h->hsend || !h->hrecv || !h->hlam))
+    return fail(h, APOLLO_ERR_STATE, "bind the halo buffers first (apollo_dg_halo_bind)");
+  return APOLLO_OK;
+}
+}  // namespace
+
 apollo_status apollo_dg_dist_start(apollo_dg* h, double t, double dt, apollo_precision prec) {
   apollo_status r = check_ready(h);
   if (r) return r;
   if (!h->have_state) return fail(h, APOLLO_ERR_STATE, "no state set");
   if (prec == APOLLO_PREC_MIXED && !h->mixed)
     return fail(h, APOLLO_ERR_CONFIG, "mixed precision is not available for this equation/order");
-  if (!h->peers.empty() && (!h->hsend || !h->hrecv || !h->hlam))
-    return fail(h, APOLLO_ERR_STATE, "bind the halo buffers first (apollo_dg_halo_bind)");
+  if ((r = check_halo(h))) return r;
   DevState s{};
   s.t = t;
   s.dt = dt;
@@ -1891,6 +1898,7 @@ apollo_status apollo_dg_stage_begin(apollo_dg* h, int stage, apollo_precision pr
   if (h->lim_on) return fail(h, APOLLO_ERR_CONFIG, "partitioned meshes do not support the limiter");
   if (stage < 0 || stage > 4) return APOLLO_ERR_ARG;
   if (prec == APOLLO_PREC_MIXED && !h->mixed) return fail(h, APOLLO_ERR_CONFIG, "mixed precision not available");
+  if ((r = check_halo(h))) return r;
   StageArgs a = stage_args(h, stage);
   DgDev d = make_dev(h);
   if (prec == APOLLO_PREC_MIXED) {
@@ -1921,6 +1929,7 @@ apollo_status apollo_dg_stage_end(apollo_dg* h, int stage, apollo_precision prec
   if (h->lim_on) return fail(h, APOLLO_ERR_CONFIG, "partitioned meshes do not support the limiter");
   if (stage < 0 || stage > 4) return APOLLO_ERR_ARG;
   if (prec == APOLLO_PREC_MIXED && !h->mixed) return fail(h, APOLLO_ERR_CONFIG, "mixed precision not available");
+  if ((r = check_halo(h))) return r;
   StageArgs a = stage_args(h, stage);
   DgDev d = make_dev(h);
   if (prec == APOLLO_PREC_MIXED) {
