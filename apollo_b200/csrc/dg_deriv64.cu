@@ -52,8 +52,10 @@ template <int EQ, int N> struct Deriv {
     return sizeof(double) * (size_t)(round_up(ops + TABS, 2) + warps * WARP);
   }
   static constexpr int fit(int ops, int w) { return bytes(ops, w) <= 227 * 1024 ? w : fit(ops, w - 1); }
-  // Eight warps have 255 registers a lane.  Twelve have 168, and the Euler
-  // kernels then spill 40 to 470 bytes a lane: the gradient of ten steps, N = 3,
+  // Eight warps have 255 registers a lane; the Euler tangent still spills 16 to 52
+  // bytes (4 fields, orders 3-5) and 72 to 168 (5 fields), the adjoint of 5 and of 8
+  // fields at order 5 some 155.  Twelve have 168, and the Euler kernels then
+  // spill 40 to 470 bytes a lane: the gradient of ten steps, N = 3,
   // K = 6,962 2,605 us with twelve and 2,192 with eight, N = 4, K = 32,258 9,495
   // and 8,990, N = 3, K = 32,258 6,000 and 5,890.  The linear equations (but for
   // eight fields) fit in 168.

@@ -145,7 +145,10 @@ struct StageArgs {
   double frac;
   double t_arg;
   double dt_arg;        // dt used when time_from_state == 0
-  int reset_lambda;     // volume kernel zeroes st->lam_bits first
+  // the wave-speed words: a stage that reduces none (MODE_STAGE) clears them for the
+  // one that does; a MODE_RHS launch clears them first.  A step's end (k_finalize)
+  // leaves them clear; a caller that clears them itself passes 0
+  int reset_lambda;
   int overlap;          // fused float64 stage: the kernel before in the stream is one of the same step, and this
                         // one may start while it runs (it waits for it before it reads any of its results)
   // mixed precision only: fp32 face traces [K][3][NG M, padded] of x (tr_in) and of

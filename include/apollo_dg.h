@@ -306,8 +306,9 @@ apollo_status apollo_dg_energy(apollo_dg* h, const double* U, int where, double*
 
 /* Diagnostics: average device time in milliseconds of each kernel of one
  * right-hand side, over `iters` evaluations of the resident state (CUDA events
- * on the handle's stream).  ms[0..2] = volume, face, LIFT + update.  *nk
- * receives the number of kernels timed. */
+ * on the handle's stream).  ms[0..2] = volume, face, LIFT + update of the
+ * three-kernel float64 form; the fused stage, and the mixed form's traces and
+ * stage, fill ms from the front.  *nk receives the number of entries. */
 apollo_status apollo_dg_kernel_times(apollo_dg* h, apollo_precision prec, int iters, double* ms, int* nk);
 
 /* The float64 right-hand side for callers that cannot allocate device memory
@@ -519,7 +520,9 @@ apollo_status apollo_dg_halo_bind(apollo_dg* h, void* send, size_t send_bytes, v
  *   apollo_dg_step_end()                 the dt policy of apollo_dg_step
  * then apollo_dg_get_time as after apollo_dg_step_async.  The caller orders
  * its transfers after the begin call's work and before the end call's on the
- * handle's stream (or synchronises it). */
+ * handle's stream (or synchronises it).  Until apollo_dg_stage_end of stage 4 the
+ * resident state is the one the step started from: after a failed transfer it can
+ * be read, or the step taken again from apollo_dg_dist_start. */
 apollo_status apollo_dg_dist_start(apollo_dg* h, double t, double dt, apollo_precision prec);
 apollo_status apollo_dg_stage_begin(apollo_dg* h, int stage, apollo_precision prec);
 apollo_status apollo_dg_stage_end(apollo_dg* h, int stage, apollo_precision prec);
