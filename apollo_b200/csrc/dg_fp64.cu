@@ -596,10 +596,8 @@ int fp64_supported(int eq, int N) { return eq >= 0 && eq <= 4 && N >= 2 && N <= 
 // K = 130,050 168 and 87 us, N = 5 572 and 329; 8 fields N = 3, K = 32,258 129
 // and 39; K = 2,048, 16,200 and 50,562 with 5 fields, N = 3: HLL 43, 94, 260 and
 // 24, 40, 84; Roe 38, 84, 213 and 24, 40, 83; Wave 47, 106, 306 and 25, 38, 77.  Over
-// fluxes, orders and field counts it takes 0.84 of the three kernels' time at most,
-// for states that need no clamp; with 2 % of the elements below the density floor
-// the three kernels are faster below a wave of tiles (5 fields, N = 3, K = 2,048,
-// Lax-Friedrichs 36 and 46 us) and slower above (K = 16,200 75 and 58).
+// fluxes, orders and field counts it takes 0.84 of the three kernels' time at most;
+// with floored states on meshes below a wave of tiles about their time.
 static bool fused_applies(int eq, const DgDev& d, const StageArgs& a) {
   if (d.fp64_fused == 0) return false;
   if (d.fp64_fused == 2 && (d.K + 7) / 8 > stage64_wave_tiles(eq, d, num_sms())) return false;

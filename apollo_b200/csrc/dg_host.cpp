@@ -238,6 +238,7 @@ DgDev make_dev(const apollo_dg* h) {
   d.srcv = h->src.n > 0 ? h->srcv_d : nullptr;
   d.eqp = h->eqp;
   d.eqp.rho_lo = density_word(h->eqp.p[2]);
+  d.eqp.quick = quick_floors(h->eqp);
   d.bcs = h->bcs;
   d.dtfac = 2. / 3. * h->cfg.cfl * h->dtscale;
   d.rmin = h->ops.rmin;

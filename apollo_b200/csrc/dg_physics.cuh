@@ -46,7 +46,9 @@ constexpr int kMaxBc = 8;
 
 struct EqParams {
   double p[4];  // advection: ux uy uz; Euler: gamma minP minD; Maxwell: c0 gamma chi
-  int rho_lo;   // the Euler fast fluxes' least high word of a density (density_word, set for the device)
+  // set for the device: the Euler fast fluxes' least high word of a density
+  // (density_word), and whether gamma and the floors suit Quick (quick_floors)
+  int rho_lo, quick;
 };
 
 // Densities and pressures that the float64 Euler kernels' own flux code takes
@@ -58,6 +60,9 @@ inline int density_word(double min_density) {
   memcpy(&bits, &min_density, sizeof bits);
   const int above = (int)(bits >> 32) + 1;
   return above < kWordLo ? kWordLo : above > kWordHi ? kWordHi : above;
+}
+inline int quick_floors(const EqParams& P) {
+  return P.p[0] - 1.0 > 1e-9 && P.p[0] < 1e9 && P.p[1] >= 0.0 && P.p[1] < 1e75 && P.p[2] >= 0.0 && P.p[2] < 1e60;
 }
 
 struct BcTable {

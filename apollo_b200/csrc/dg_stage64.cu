@@ -77,8 +77,8 @@ template <int EQ, int N, int KIND> struct Chain {
   static constexpr int WARP = XB * (X + G) + PN + C;
   static constexpr size_t bytes(int warps) { return sizeof(double) * (size_t)(SHARED + warps * WARP); }
   // Warps per block (one block per SM): what registers and shared memory allow.
-  // Sixteen have 128 registers a lane, and the Euler kernels then spill 110 to
-  // 720 bytes; eight spill nothing.  The spills cost less than the missing warps
+  // Sixteen have 128 registers a lane, and the Euler kernels then spill 130 to
+  // 670 bytes; eight spill nothing.  The spills cost less than the missing warps
   // on large meshes, more on small ones, and the longest bodies (HLL and Roe, 5
   // fields, orders 3 and 4) gain from eight at every size.  A right-hand side, K =
   // 2,048, 16,200, 50,562, with eight and with sixteen: Lax-Friedrichs N = 4, 4

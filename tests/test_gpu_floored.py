@@ -1,0 +1,73 @@
+"""States that need the density or pressure floors (B200), against the CPU
+oracle, which clamps as Apollo does: every flux, order and field count, in the
+fused and in the three-kernel form; and what they cost on a mesh of one wave."""
+import numpy as np
+import pytest
+
+from apollo_b200 import NodalDG2d, problems
+from apollo_b200.mesh import jittered_square
+from golden_cases import rel_l2
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+CODE = {"LF": 0, "HLL": 1, "Roe": 2, "Wave": 4}
+
+
+@pytest.mark.parametrize("N", [2, 3, 4, 5])
+@pytest.mark.parametrize("fields", [4, 5])
+@pytest.mark.parametrize("flux", list(CODE))
+def test_floored_states_against_the_oracle(flux, fields, N):
+    """Elements below the density floor, with a negative density, with pressures
+    below and above the floor, at rest and not, beside sound ones.  1e-12 as for
+    the parity tests; speeds off the integers of the truncated HLL bound."""
+    m = jittered_square(6, seed=4)  # K = 50
+    minP, minD = 0.3, 0.2
+    s = NodalDG2d(N, 0.5, {4: "eulerEqn2d", 5: "eulerEqn"}[fields], (1.4, minP, minD), m, numerical_flux=flux)
+    rng = np.random.default_rng(100 * N + fields)
+    U = rng.uniform(-0.02, 0.02, s.shape[:2] + (5,))
+    U[..., 0] += 1.0
+    U[..., 1] += 0.31
+    U[..., 2] -= 0.17
+    if fields == 4:
+        U[..., 3] = 0.0
+    U[4, :, 0] = 0.15                        # below the floor
+    U[5, :, 0] = rng.uniform(0.15, 0.25, s.Np)  # across it
+    U[16, :, 1:4] = 0.0                      # at rest
+    U[17, :, :4] *= 0.1                      # below the floor, the velocity of the others
+    U[..., 4] = 0.5 * (U[..., 1:4] ** 2).sum(-1) / U[..., 0] + 2.37
+    U[23, :, 4] -= 2.0                       # pressure below its floor
+    U[30, 2, 4] -= 2.3                       # at one node
+    U[41, :, 4] = 0.02                       # negative pressure
+    if flux != "Wave":                       # its Riemann solver refuses a negative density
+        U[48, :, 0] = -0.1
+    o = orc.Oracle(m, N, orc.EQ_EULER, (1.4, minP, minD, CODE[flux]), cfl=0.5)
+    ref, sugg = o.rhs(np.ascontiguousarray(U))
+    keep = [0, 1, 2, 4] if fields == 4 else slice(None)
+    for form in (1, 0):
+        s.set_fp64_kernels(form)
+        got, gs = s.step(0.0, 0.0, np.ascontiguousarray(U[..., keep]))
+        assert rel_l2(got, ref[..., keep]) <= 1e-12, form
+        assert gs == pytest.approx(sugg, rel=1e-12), form
+
+
+@pytest.mark.parametrize("n", [17, 33])
+@pytest.mark.parametrize("flux", list(CODE))
+def test_floored_states_on_a_small_mesh(flux, n):
+    """2 % of the elements below the density floor, order 5, below one wave of
+    tiles: 0.98 of the three kernels' time at most (1.3 to 1.7 with the equation's
+    code on doubles)."""
+    p = problems.euler_vortex(n=n, N=5, fields=4)
+    s = NodalDG2d(p.N, p.cfl, p.equation, (1.4, 1e-3, 0.3), p.mesh, bcs=p.bcs, numerical_flux=flux)
+    x, y = s.node_coords()
+    U = np.ascontiguousarray(p.ic(x, y))
+    cx = x.mean(1)
+    U[cx <= np.quantile(cx, 0.02)] *= 0.2
+    s.set_state(U)
+    us = {}
+    for form in (0, 1):
+        s.set_fp64_kernels(form)
+        s.kernel_times(5)
+        us[form] = min(sum(s.kernel_times(10)) for _ in range(5)) * 1e3
+    s.close()
+    assert us[1] <= 1.15 * us[0]
