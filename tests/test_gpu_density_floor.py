@@ -44,21 +44,20 @@ def test_densities_at_the_floor(flux, fields, N, floor):
     assert got[1][1] == pytest.approx(got[0][1], rel=1e-13)
 
 
-def _us(p, flux):
-    s = NodalDG2d(p.N, p.cfl, p.equation, p.eq_params, p.mesh, bcs=p.bcs, numerical_flux=flux)
-    x, y = s.node_coords()
-    s.set_state(np.ascontiguousarray(p.ic(x, y)))
-    s.kernel_times(5)
-    us = min(sum(s.kernel_times(10)) for _ in range(5)) * 1e3
-    s.close()
-    return us
-
-
 @pytest.mark.parametrize("N", [2, 3, 4, 5])
 @pytest.mark.parametrize("fields", [4, 5])
 def test_sound_states_take_the_fast_flux(fields, N):
     p = problems.euler_vortex(n=91, N=N, fields=fields)
-    assert _us(p, "HLL") <= 1.5 * _us(p, "LF")
+    s = {f: NodalDG2d(p.N, p.cfl, p.equation, p.eq_params, p.mesh, bcs=p.bcs, numerical_flux=f) for f in ("LF", "HLL")}
+    us = {"LF": [], "HLL": []}
+    for h in s.values():
+        x, y = h.node_coords()
+        h.set_state(np.ascontiguousarray(p.ic(x, y)))
+    for _ in range(8):  # in turn, so that a slow spell meets both
+        for f, h in s.items():
+            h.kernel_times(3)
+            us[f].append(sum(h.kernel_times(10)) * 1e3)
+    assert min(us["HLL"]) <= 1.5 * min(us["LF"])
 
 
 @pytest.mark.parametrize("N", [4, 5])

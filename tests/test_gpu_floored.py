@@ -64,10 +64,11 @@ def test_floored_states_on_a_small_mesh(flux, n):
     cx = x.mean(1)
     U[cx <= np.quantile(cx, 0.02)] *= 0.2
     s.set_state(U)
-    us = {}
-    for form in (0, 1):
-        s.set_fp64_kernels(form)
-        s.kernel_times(5)
-        us[form] = min(sum(s.kernel_times(10)) for _ in range(5)) * 1e3
+    us = {0: [], 1: []}
+    for _ in range(8):  # in turn, so that a slow spell meets both
+        for form in (0, 1):
+            s.set_fp64_kernels(form)
+            s.kernel_times(3)
+            us[form].append(sum(s.kernel_times(10)) * 1e3)
     s.close()
-    assert us[1] <= 1.15 * us[0]
+    assert min(us[1]) <= 1.15 * min(us[0])

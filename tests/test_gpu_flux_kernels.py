@@ -77,10 +77,11 @@ def test_not_slower_than_the_three_kernels(flux, fields, N, n):
     s = NodalDG2d(p.N, p.cfl, p.equation, p.eq_params, p.mesh, bcs=p.bcs, numerical_flux=flux)
     x, y = s.node_coords()
     s.set_state(np.ascontiguousarray(p.ic(x, y)))
-    us = {}
-    for form in (0, 1):
-        s.set_fp64_kernels(form)
-        s.kernel_times(5)
-        us[form] = min(sum(s.kernel_times(10)) for _ in range(5)) * 1e3
+    us = {0: [], 1: []}
+    for _ in range(8):  # in turn, so that a slow spell meets both
+        for form in (0, 1):
+            s.set_fp64_kernels(form)
+            s.kernel_times(3)
+            us[form].append(sum(s.kernel_times(10)) * 1e3)
     s.close()
-    assert us[1] <= us[0]
+    assert min(us[1]) <= min(us[0])
